@@ -22,6 +22,10 @@ namespace des {
 
 constexpr int TPB_A = 128;
 
+// DES_LAUNCH for kernels of at most TPB_A threads a block
+#define DES_LAUNCH_A(KERNEL, n, s, ...) \
+    KERNEL<<<grid_blocks(n, TPB_A), block_threads(n, TPB_A), 0, (s)>>>(__VA_ARGS__)
+
 static inline int nblk(long long n, int tpb = TPB_A)
 {
     long long b = (n + tpb - 1) / tpb;
@@ -232,7 +236,7 @@ __global__ void __launch_bounds__(TPB_A) k_adj_end_geometry(KP p, AdjBufs a, Tap
 int launch_adj_end_geometry(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
                             cudaStream_t s)
 {
-    k_adj_end_geometry<<<nblk(p.ne), TPB_A, 0, s>>>(p, a, t, t1, dt);
+    DES_LAUNCH_A(k_adj_end_geometry, p.ne, s, p, a, t, t1, dt);
     return 1;
 }
 
@@ -531,16 +535,16 @@ int launch_adj_force(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStrea
 {
     int n = 0;
     if (p.nbf > 0) {
-        k_adj_facets<<<nblk(p.nbf), TPB_A, 0, s>>>(p, a, t);
+        DES_LAUNCH_A(k_adj_facets, p.nbf, s, p, a, t);
         ++n;
     }
-    k_adj_force<<<nblk(p.ne), TPB_A, 0, s>>>(p, a, t);
+    DES_LAUNCH_A(k_adj_force, p.ne, s, p, a, t);
     return n + 1;
 }
 
 int launch_adj_nmd_nodes(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStream_t s)
 {
-    k_adj_nmd_nodes<<<nblk(p.nn), TPB_A, 0, s>>>(p, a, t);
+    DES_LAUNCH_A(k_adj_nmd_nodes, p.nn, s, p, a, t);
     return 1;
 }
 
@@ -1196,38 +1200,38 @@ __global__ void __launch_bounds__(TPB_A) k_adj_gather_xT(KP p, AdjBufs a)
 int launch_adj_stress(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
                       cudaStream_t s)
 {
-    k_adj_stress<<<nblk(p.ne), TPB_A, 0, s>>>(p, a, t, t1, dt);
+    DES_LAUNCH_A(k_adj_stress, p.ne, s, p, a, t, t1, dt);
     return 1;
 }
 
 int launch_adj_nodes_heat(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
                           cudaStream_t s)
 {
-    k_adj_nodes_heat<<<nblk(p.nn), TPB_A, 0, s>>>(p, a, t, t1, dt);
+    DES_LAUNCH_A(k_adj_nodes_heat, p.nn, s, p, a, t, t1, dt);
     return 1;
 }
 
 int launch_adj_kinematics(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStream_t s)
 {
-    k_adj_kinematics<<<nblk(p.ne), TPB_A, 0, s>>>(p, a, t);
+    DES_LAUNCH_A(k_adj_kinematics, p.ne, s, p, a, t);
     return 1;
 }
 
 int launch_adj_gather_vT(const KP &p, const AdjBufs &a, cudaStream_t s)
 {
-    k_adj_gather_vT<<<nblk(p.nn), TPB_A, 0, s>>>(p, a);
+    DES_LAUNCH_A(k_adj_gather_vT, p.nn, s, p, a);
     return 1;
 }
 
 int launch_adj_start_geometry(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStream_t s)
 {
-    k_adj_start_geometry<<<nblk(p.ne), TPB_A, 0, s>>>(p, a, t);
+    DES_LAUNCH_A(k_adj_start_geometry, p.ne, s, p, a, t);
     return 1;
 }
 
 int launch_adj_gather_xT(const KP &p, const AdjBufs &a, cudaStream_t s)
 {
-    k_adj_gather_xT<<<nblk(p.nn), TPB_A, 0, s>>>(p, a);
+    DES_LAUNCH_A(k_adj_gather_xT, p.nn, s, p, a);
     return 1;
 }
 

@@ -1357,7 +1357,7 @@ int launch_elem_props(const KP &p, cudaStream_t s, double *out)
 {
     KP q = p;
     q.eprop = nullptr;
-    k_elem_props<<<nblocks(p.ne), TPB, 0, s>>>(q, out);
+    DES_LAUNCH(k_elem_props, p.ne, s, q, out);
     return 1;
 }
 
@@ -1404,72 +1404,72 @@ __global__ void __launch_bounds__(TPB) k_rows(const __grid_constant__ RowTable t
 // ==================================================================
 // launchers
 // ==================================================================
-#define DISPATCH(KERNEL, GRID, ...)                                       \
+#define DISPATCH(KERNEL, N, ...)                                          \
     do {                                                                  \
-        if (p.nd == 3) KERNEL<3><<<(GRID), TPB, 0, s>>>(__VA_ARGS__);     \
-        else KERNEL<2><<<(GRID), TPB, 0, s>>>(__VA_ARGS__);               \
+        if (p.nd == 3) DES_LAUNCH(KERNEL<3>, (N), s, __VA_ARGS__);        \
+        else DES_LAUNCH(KERNEL<2>, (N), s, __VA_ARGS__);                  \
     } while (0)
 
 int launch_strain_rate(const KP &p, cudaStream_t s, bool begin_step)
 {
-    DISPATCH(k_strain_rate, nblocks(p.ne), p, (int)begin_step);
+    DISPATCH(k_strain_rate, p.ne, p, (int)begin_step);
     return 1;
 }
 
 int launch_heat_gather(const KP &p, cudaStream_t s)
 {
-    if (p.nd == 3) k_node_gather1<3, true, false><<<nblocks(p.nn), TPB, 0, s>>>(p);
-    else k_node_gather1<2, true, false><<<nblocks(p.nn), TPB, 0, s>>>(p);
+    if (p.nd == 3) DES_LAUNCH((k_node_gather1<3, true, false>), p.nn, s, p);
+    else DES_LAUNCH((k_node_gather1<2, true, false>), p.nn, s, p);
     return 1;
 }
 
 int launch_dvoldt(const KP &p, cudaStream_t s)
 {
-    if (p.nd == 3) k_node_gather1<3, false, true><<<nblocks(p.nn), TPB, 0, s>>>(p);
-    else k_node_gather1<2, false, true><<<nblocks(p.nn), TPB, 0, s>>>(p);
+    if (p.nd == 3) DES_LAUNCH((k_node_gather1<3, false, true>), p.nn, s, p);
+    else DES_LAUNCH((k_node_gather1<2, false, true>), p.nn, s, p);
     return 1;
 }
 
 int launch_elem_pass(const KP &p, cudaStream_t s, bool heat)
 {
-    DISPATCH(k_elem_pass, nblocks(p.e_hi - p.e_lo), p, (int)heat);
+    DISPATCH(k_elem_pass, p.e_hi - p.e_lo, p, (int)heat);
     return 1;
 }
 
 int launch_node_pass(const KP &p, cudaStream_t s, bool heat)
 {
-    DISPATCH(k_node_pass, nblocks(p.n_hi - p.n_lo), p, (int)heat);
+    DISPATCH(k_node_pass, p.n_hi - p.n_lo, p, (int)heat);
     return 1;
 }
 
 int launch_heat_and_dvoldt(const KP &p, cudaStream_t s)
 {
-    if (p.nd == 3) k_node_gather1<3, true, true><<<nblocks(p.nn), TPB, 0, s>>>(p);
-    else k_node_gather1<2, true, true><<<nblocks(p.nn), TPB, 0, s>>>(p);
+    if (p.nd == 3) DES_LAUNCH((k_node_gather1<3, true, true>), p.nn, s, p);
+    else DES_LAUNCH((k_node_gather1<2, true, true>), p.nn, s, p);
     return 1;
 }
 
 int launch_temperature_update(const KP &p, cudaStream_t s)
 {
-    k_temperature_update<<<nblocks(p.nn), TPB, 0, s>>>(p);
+    DES_LAUNCH(k_temperature_update, p.nn, s, p);
     return 1;
 }
 
 int launch_edvoldt(const KP &p, cudaStream_t s)
 {
-    DISPATCH(k_edvoldt, nblocks(p.ne), p);
+    DISPATCH(k_edvoldt, p.ne, p);
     return 1;
 }
 
 int launch_update_stress(const KP &p, cudaStream_t s, bool fused)
 {
-    DISPATCH(k_update_stress, nblocks(p.e_hi - p.e_lo), p, (int)fused);
+    DISPATCH(k_update_stress, p.e_hi - p.e_lo, p, (int)fused);
     return 1;
 }
 
 int launch_nmd_gather(const KP &p, cudaStream_t s, bool stored)
 {
-    DISPATCH(k_nmd_gather, nblocks(p.n_hi - p.n_lo), p, (int)(stored && p.pv));
+    DISPATCH(k_nmd_gather, p.n_hi - p.n_lo, p, (int)(stored && p.pv));
     return 1;
 }
 
@@ -1477,48 +1477,48 @@ int launch_nmd_correct(const KP &p, cudaStream_t s, bool with_facets)
 {
     long long n = (long long)(p.e_hi - p.e_lo) + (with_facets ? p.f_hi - p.f_lo : 0);
     if (uses_force_terms(p)) {
-        k_nmd_correct_ft3<<<nblocks(n), TPB, 0, s>>>(p, (int)with_facets);
+        DES_LAUNCH(k_nmd_correct_ft3, n, s, p, (int)with_facets);
         return 1;
     }
-    DISPATCH(k_nmd_correct, nblocks(n), p, (int)with_facets);
+    DISPATCH(k_nmd_correct, n, p, (int)with_facets);
     return 1;
 }
 
 int launch_force_terms(const KP &p, cudaStream_t s)
 {
     if (!uses_force_terms(p)) return 0;
-    k_force_terms3<<<nblocks(p.e_hi - p.e_lo), TPB, 0, s>>>(p);
+    DES_LAUNCH(k_force_terms3, p.e_hi - p.e_lo, s, p);
     return 1;
 }
 
 int launch_facet_forces(const KP &p, cudaStream_t s)
 {
     if (p.nbf == 0) return 0;
-    DISPATCH(k_facet_forces, nblocks(p.nbf), p);
+    DISPATCH(k_facet_forces, p.nbf, p);
     return 1;
 }
 
 int launch_force(const KP &p, cudaStream_t s, bool fused_motion, bool contract)
 {
     if (contract && uses_force_terms(p)) {
-        k_force_dw3<<<nblocks(p.n_hi - p.n_lo), TPB, 0, s>>>(p, (int)fused_motion);
+        DES_LAUNCH(k_force_dw3, p.n_hi - p.n_lo, s, p, (int)fused_motion);
         return 1;
     }
     if (contract) {
-        if (p.nd == 3) k_force<3, true><<<nblocks(p.n_hi - p.n_lo), TPB, 0, s>>>(p, (int)fused_motion);
-        else k_force<2, true><<<nblocks(p.n_hi - p.n_lo), TPB, 0, s>>>(p, (int)fused_motion);
+        if (p.nd == 3) DES_LAUNCH((k_force<3, true>), p.n_hi - p.n_lo, s, p, (int)fused_motion);
+        else DES_LAUNCH((k_force<2, true>), p.n_hi - p.n_lo, s, p, (int)fused_motion);
         return 1;
     }
-    DISPATCH(k_force, nblocks(p.n_hi - p.n_lo), p, (int)fused_motion);
+    DISPATCH(k_force, p.n_hi - p.n_lo, p, (int)fused_motion);
     return 1;
 }
 
 int launch_velocity(const KP &p, cudaStream_t s, bool contract)
 {
-    const int g = nblocks((long long)p.nn * p.nd);
+    const long long g = (long long)p.nn * p.nd;
     if (contract) {
-        if (p.nd == 3) k_velocity<3, true><<<g, TPB, 0, s>>>(p);
-        else k_velocity<2, true><<<g, TPB, 0, s>>>(p);
+        if (p.nd == 3) DES_LAUNCH((k_velocity<3, true>), g, s, p);
+        else DES_LAUNCH((k_velocity<2, true>), g, s, p);
         return 1;
     }
     DISPATCH(k_velocity, g, p);
@@ -1527,16 +1527,16 @@ int launch_velocity(const KP &p, cudaStream_t s, bool contract)
 
 int launch_vbcs(const KP &p, cudaStream_t s)
 {
-    DISPATCH(k_vbcs, nblocks(p.nn), p);
+    DISPATCH(k_vbcs, p.nn, p);
     return 1;
 }
 
 int launch_coordinate(const KP &p, cudaStream_t s, bool contract)
 {
-    const int g = nblocks((long long)p.nn * p.nd);
+    const long long g = (long long)p.nn * p.nd;
     if (contract) {
-        if (p.nd == 3) k_coordinate<3, true><<<g, TPB, 0, s>>>(p);
-        else k_coordinate<2, true><<<g, TPB, 0, s>>>(p);
+        if (p.nd == 3) DES_LAUNCH((k_coordinate<3, true>), g, s, p);
+        else DES_LAUNCH((k_coordinate<2, true>), g, s, p);
         return 1;
     }
     DISPATCH(k_coordinate, g, p);
@@ -1545,25 +1545,25 @@ int launch_coordinate(const KP &p, cudaStream_t s, bool contract)
 
 int launch_geometry(const KP &p, cudaStream_t s, int flags)
 {
-    DISPATCH(k_geometry, nblocks(p.e_hi - p.e_lo), p, flags);
+    DISPATCH(k_geometry, p.e_hi - p.e_lo, p, flags);
     return 1;
 }
 
 int launch_geometry_ahead(const KP &p, cudaStream_t s, int flags)
 {
-    k_geometry_ahead3<<<nblocks(p.e_hi - p.e_lo), TPB, 0, s>>>(p, flags);
+    DES_LAUNCH(k_geometry_ahead3, p.e_hi - p.e_lo, s, p, flags);
     return 1;
 }
 
 int launch_mass(const KP &p, cudaStream_t s)
 {
-    DISPATCH(k_mass, nblocks(p.nn), p);
+    DISPATCH(k_mass, p.nn, p);
     return 1;
 }
 
 int launch_mass_sum(const KP &p, cudaStream_t s)
 {
-    DISPATCH(k_mass_sum, nblocks(p.n_hi - p.n_lo), p);
+    DISPATCH(k_mass_sum, p.n_hi - p.n_lo, p);
     return 1;
 }
 
@@ -1582,21 +1582,21 @@ int launch_dt_reset(const KP &p, cudaStream_t s)
 
 int launch_output_elem(const KP &p, double *out, cudaStream_t s)
 {
-    DISPATCH(k_output_elem, nblocks(p.ne), p, out);
+    DISPATCH(k_output_elem, p.ne, p, out);
     return 1;
 }
 
 int launch_quality(const KP &p, cudaStream_t s, unsigned long long *red)
 {
-    DISPATCH(k_quality_min, nblocks(p.ne), p, red);
-    DISPATCH(k_quality_arg, nblocks(p.ne), p, red);
+    DISPATCH(k_quality_min, p.ne, p, red);
+    DISPATCH(k_quality_arg, p.ne, p, red);
     return 2;
 }
 
 int launch_quality_scans(const KP &p, cudaStream_t s, double smallest_vol, double bottom, double dist,
                          int check_bottom, unsigned long long *red)
 {
-    DISPATCH(k_quality_scans, nblocks(std::max(p.ne, p.nn)), p, smallest_vol, bottom, dist, check_bottom, red);
+    DISPATCH(k_quality_scans, std::max(p.ne, p.nn), p, smallest_vol, bottom, dist, check_bottom, red);
     return 1;
 }
 
@@ -1608,7 +1608,7 @@ __global__ void k_f64_to_f32(const double *__restrict__ a, float *__restrict__ b
 
 int launch_f64_to_f32(const double *a, float *b, long long n, cudaStream_t s)
 {
-    k_f64_to_f32<<<nblocks(n), TPB, 0, s>>>(a, b, n);
+    DES_LAUNCH(k_f64_to_f32, n, s, a, b, n);
     return 1;
 }
 
@@ -1623,19 +1623,19 @@ int launch_shp_join(const KP &p, cudaStream_t s)
 {
     if (!p.shpdw) return 0;
     const long long n = (long long)p.ne * p.npe * p.nd;
-    k_shp_join<<<nblocks(n), TPB, 0, s>>>(p.shpdw, p.shp, n);
+    DES_LAUNCH(k_shp_join, n, s, p.shpdw, p.shp, n);
     return 1;
 }
 
 int launch_aos_to_soa(const double *aos, double *soa, int n, int ncomp, cudaStream_t s)
 {
-    k_aos_to_soa<<<nblocks((long long)n * ncomp), TPB, 0, s>>>(aos, soa, n, ncomp);
+    DES_LAUNCH(k_aos_to_soa, (long long)n * ncomp, s, aos, soa, n, ncomp);
     return 1;
 }
 
 int launch_soa_to_aos(const double *soa, double *aos, int n, int ncomp, cudaStream_t s)
 {
-    k_soa_to_aos<<<nblocks((long long)n * ncomp), TPB, 0, s>>>(soa, aos, n, ncomp);
+    DES_LAUNCH(k_soa_to_aos, (long long)n * ncomp, s, soa, aos, n, ncomp);
     return 1;
 }
 

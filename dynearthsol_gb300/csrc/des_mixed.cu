@@ -652,19 +652,19 @@ __global__ void __launch_bounds__(TPB_M) k_node_pass_mixed3(KP p, int heat, int 
 
 int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused)
 {
-    k_update_stress_mixed3<<<nblocks_m(p.e_hi - p.e_lo), TPB_M, 0, s>>>(p, (int)fused);
+    DES_LAUNCH(k_update_stress_mixed3, p.e_hi - p.e_lo, s, p, (int)fused);
     return 1;
 }
 
 int launch_strain_rate_mixed(const KP &p, cudaStream_t s, bool begin_step)
 {
-    k_strain_rate_mixed3<<<nblocks_m(p.ne), TPB_M, 0, s>>>(p, (int)begin_step);
+    DES_LAUNCH(k_strain_rate_mixed3, p.ne, s, p, (int)begin_step);
     return 1;
 }
 
 int launch_heat_and_dvoldt_mixed(const KP &p, cudaStream_t s, bool heat, bool dvoldt)
 {
-    k_heat_dvoldt_mixed3<<<nblocks_m(p.nn), TPB_M, 0, s>>>(p, (int)heat, (int)dvoldt);
+    DES_LAUNCH(k_heat_dvoldt_mixed3, p.nn, s, p, (int)heat, (int)dvoldt);
     return 1;
 }
 
@@ -672,13 +672,13 @@ int launch_heat_and_dvoldt_mixed(const KP &p, cudaStream_t s, bool heat, bool dv
 
 int launch_elem_pass_mixed(const KP &p, cudaStream_t s, bool heat)
 {
-    k_elem_pass_mixed3<<<nblocks_m(p.e_hi - p.e_lo), TPB_M, 0, s>>>(p, (int)heat);
+    DES_LAUNCH(k_elem_pass_mixed3, p.e_hi - p.e_lo, s, p, (int)heat);
     return 1;
 }
 
 int launch_node_pass_mixed(const KP &p, cudaStream_t s, bool heat, bool mass_sums, bool begin_step)
 {
-    k_node_pass_mixed3<<<nblocks_m(p.n_hi - p.n_lo), TPB_M, 0, s>>>(p, (int)heat, (int)mass_sums, (int)begin_step);
+    DES_LAUNCH(k_node_pass_mixed3, p.n_hi - p.n_lo, s, p, (int)heat, (int)mass_sums, (int)begin_step);
     return 1;
 }
 
