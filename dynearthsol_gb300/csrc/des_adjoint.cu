@@ -64,60 +64,32 @@ __device__ __forceinline__ void tload3(const double *a, size_t nn, int n, double
 // ------------------------------------------------------------------
 // geometry: volume (geometry.cxx:29-49) and shape functions
 // (geometry.cxx:368-455) of one tet, reversed.  Given the adjoints gvol of
-// the volume and gs[k][i] of dN_i/dx_k, adds the coordinate adjoints to gc.
-// dN_i/dx_k = (P_a Q_b - P_b Q_a) / (6V), with (P, Q) = (y, z), (z, x),
-// (x, y) for k = 0, 1, 2 and the differences P_ij = P_i - P_j over the
-// pairs a, b listed below -- the forward's expressions, regrouped.
+// the volume and gs[k][i] of g_i,k = dN_i/dx_k, writes the coordinate
+// adjoints gc.  Moving the nodes by d_j changes the volume by
+// V sum_j g_j . d_j and the gradients of the linear functions by
+// dg_i = -sum_j (d_j . g_i) g_j (the first-order change of the inverse of
+// the element's deformation), so with M_ab = sum_i g_i,a gs_b,i
+//   gc_j,a = sum_b (gvol V delta_ab - M_ab) g_j,b:
+// 75 multiply-adds on the shape functions alone, in place of the reversed
+// cofactor expressions of the coordinates (about 250 FP64 operations).
 // ------------------------------------------------------------------
-__device__ void geom_reverse(const double (*c)[3], double vol, const double (*gs)[4], double gvol,
-                             double (*gc)[3])
+__device__ __forceinline__ void geom_reverse(const double (*g)[4], double vol, const double (*gs)[4], double gvol,
+                                             double (*gc)[3])
 {
-    const int PA[4][2] = {{1, 3}, {0, 2}, {1, 3}, {0, 1}};
-    const int PB[4][2] = {{1, 2}, {2, 3}, {0, 3}, {0, 2}};
-    const double iv = recip_newton(6 * vol);
-    double giv = 0;
+    double m[3][3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int P = (k + 1) % 3, Q = (k + 2) % 3;
+    for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int a0 = PA[i][0], a1 = PA[i][1], b0 = PB[i][0], b1 = PB[i][1];
-            const double Pa = c[a0][P] - c[a1][P], Qa = c[a0][Q] - c[a1][Q];
-            const double Pb = c[b0][P] - c[b1][P], Qb = c[b0][Q] - c[b1][Q];
-            const double g = gs[k][i];
-            giv += g * (Pa * Qb - Pb * Qa);
-            const double gt = g * iv;
-            // d/dPa = Qb, d/dQb = Pa, d/dPb = -Qa, d/dQa = -Pb
-            gc[a0][P] += gt * Qb;
-            gc[a1][P] -= gt * Qb;
-            gc[b0][Q] += gt * Pa;
-            gc[b1][Q] -= gt * Pa;
-            gc[b0][P] -= gt * Qa;
-            gc[b1][P] += gt * Qa;
-            gc[a0][Q] -= gt * Pb;
-            gc[a1][Q] += gt * Pb;
+        for (int b = 0; b < 3; ++b) {
+            double acc = a == b ? gvol * vol : 0.0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc -= g[a][i] * gs[b][i];
+            m[a][b] = acc;
         }
-    }
-    gvol += giv * (-6 * iv * iv);   // d/dvol 1/(6 vol) = -6 iv^2
-    // V = [x01 (y23 z12 - y12 z23) + x12 (y01 z23 - y23 z01) + x23 (y12 z01 - y01 z12)] / 6
-    const double g6 = div6(gvol);
-    const double x01 = c[0][0] - c[1][0], x12 = c[1][0] - c[2][0], x23 = c[2][0] - c[3][0];
-    const double y01 = c[0][1] - c[1][1], y12 = c[1][1] - c[2][1], y23 = c[2][1] - c[3][1];
-    const double z01 = c[0][2] - c[1][2], z12 = c[1][2] - c[2][2], z23 = c[2][2] - c[3][2];
-    const double gx01 = g6 * (y23 * z12 - y12 * z23), gx12 = g6 * (y01 * z23 - y23 * z01),
-                 gx23 = g6 * (y12 * z01 - y01 * z12);
-    const double gy01 = g6 * (x12 * z23 - x23 * z12), gy12 = g6 * (x23 * z01 - x01 * z23),
-                 gy23 = g6 * (x01 * z12 - x12 * z01);
-    const double gz01 = g6 * (x23 * y12 - x12 * y23), gz12 = g6 * (x01 * y23 - x23 * y01),
-                 gz23 = g6 * (x12 * y01 - x01 * y12);
-    const double gd[3][3] = {{gx01, gx12, gx23}, {gy01, gy12, gy23}, {gz01, gz12, gz23}};
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        gc[0][d] += gd[d][0];
-        gc[1][d] += gd[d][1] - gd[d][0];
-        gc[2][d] += gd[d][2] - gd[d][1];
-        gc[3][d] -= gd[d][2];
-    }
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) gc[j][a] = m[a][0] * g[0][j] + m[a][1] * g[1][j] + m[a][2] * g[2][j];
 }
 
 // mass, tmass and volume_n of the element's four nodes (geometry.cxx:313-365),
@@ -128,15 +100,13 @@ __device__ __forceinline__ double mass_reverse(const KP &p, int e, const double 
     const bool quasi = p.prm.is_quasi_static, thermal = p.prm.has_thermal_diffusion;
     const double rho = quasi ? p.mat.rho_pseudo : rho_e;
     const double cp = m_cp(p, e);
-    double grho = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        gvol += rho / 4 * gm[i] + gvn[i];
-        if (!quasi) grho += vol / 4 * gm[i];
-        if (thermal) {
-            gvol += rho_e * cp / 4 * gtm[i];
-            grho += cp * vol / 4 * gtm[i];
-        }
+    const double sm = (gm[0] + gm[1]) + (gm[2] + gm[3]);
+    gvol += rho / 4 * sm + ((gvn[0] + gvn[1]) + (gvn[2] + gvn[3]));
+    double grho = quasi ? 0.0 : vol / 4 * sm;
+    if (thermal) {
+        const double st = cp / 4 * ((gtm[0] + gtm[1]) + (gtm[2] + gtm[3]));
+        gvol += rho_e * st;
+        grho += vol * st;
     }
     return grho;
 }
@@ -157,11 +127,10 @@ __global__ void __launch_bounds__(TPB_A) k_adj_end_geometry(KP p, AdjBufs a, Tap
     if (e >= p.ne) return;
     const size_t ne = p.ne, nn = p.nn;
     int nodes[4];
-    double c[4][3], v[4][3];
+    double v[4][3], sh[3][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         nodes[i] = conn_at(p, i, e);
-        tload3(t1.x, nn, nodes[i], c[i]);
         tload3(t1.v, nn, nodes[i], v[i]);
     }
     const double vol = t1.vol[e];
@@ -170,7 +139,10 @@ __global__ void __launch_bounds__(TPB_A) k_adj_end_geometry(KP p, AdjBufs a, Tap
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) gs[k][i] = a.ashp[((size_t)k * 4 + i) * ne + e];
+        for (int i = 0; i < 4; ++i) {
+            sh[k][i] = tshp(t1, ne, k, i, e);
+            gs[k][i] = a.ashp[((size_t)k * 4 + i) * ne + e];
+        }
     {
         double gm[4], gtm[4], gvn[4];
 #pragma unroll
@@ -181,56 +153,48 @@ __global__ void __launch_bounds__(TPB_A) k_adj_end_geometry(KP p, AdjBufs a, Tap
         }
         a.arho[e] = mass_reverse(p, e, gm, gtm, gvn, vol, t.rho[e], gvol);
     }
-    double gv[4][3] = {};
+    double h3 = 0, h4 = 0, h5 = 0;   // half the spin's adjoints
     if (p.mat.rheol_type & DES_RH_ELASTIC) {
         double s[6], g[6];
         tape_sss(p, t, e, s);
 #pragma unroll
         for (int cc = 0; cc < 6; ++cc) g[cc] = a.as[cc * ne + e];
-        double sh[3][4];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) sh[k][i] = tshp(t1, ne, k, i, e);
-        double w3 = 0, w4 = 0, w5 = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) w3 += 0.5 * (v[i][0] * sh[1][i] - v[i][1] * sh[0][i]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) w4 += 0.5 * (v[i][0] * sh[2][i] - v[i][2] * sh[0][i]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) w5 += 0.5 * (v[i][1] * sh[2][i] - v[i][2] * sh[1][i]);
-        // s_out = s + dt * si(s, w) (jaumann3), bilinear in s and w
-        double gsin[6];
-        gsin[0] = g[0] + dt * (g[3] * w3 + g[4] * w4);
-        gsin[1] = g[1] + dt * (-g[3] * w3 + g[5] * w5);
-        gsin[2] = g[2] + dt * (-g[4] * w4 - g[5] * w5);
-        gsin[3] = g[3] + dt * (-2 * g[0] * w3 + 2 * g[1] * w3 + g[4] * w5 + g[5] * w4);
-        gsin[4] = g[4] + dt * (-2 * g[0] * w4 + 2 * g[2] * w4 - g[3] * w5 + g[5] * w3);
-        gsin[5] = g[5] + dt * (-2 * g[1] * w5 + 2 * g[2] * w5 - g[3] * w4 - g[4] * w3);
-        const double gw3 = dt * (-2 * s[3] * g[0] + 2 * s[3] * g[1] + (s[0] - s[1]) * g[3] - s[5] * g[4] + s[4] * g[5]);
-        const double gw4 = dt * (-2 * s[4] * g[0] + 2 * s[4] * g[2] - s[5] * g[3] + (s[0] - s[2]) * g[4] + s[3] * g[5]);
-        const double gw5 = dt * (-2 * s[5] * g[1] + 2 * s[5] * g[2] - s[4] * g[3] + s[3] * g[4] + (s[1] - s[2]) * g[5]);
-#pragma unroll
-        for (int cc = 0; cc < 6; ++cc) a.as[cc * ne + e] = gsin[cc];
+        double w3 = 0, w4 = 0, w5 = 0;   // dt times the spin
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            gv[i][0] += 0.5 * (gw3 * sh[1][i] + gw4 * sh[2][i]);
-            gv[i][1] += 0.5 * (-gw3 * sh[0][i] + gw5 * sh[2][i]);
-            gv[i][2] += 0.5 * (-gw4 * sh[0][i] - gw5 * sh[1][i]);
-            gs[0][i] += 0.5 * (-gw3 * v[i][1] - gw4 * v[i][2]);
-            gs[1][i] += 0.5 * (gw3 * v[i][0] - gw5 * v[i][2]);
-            gs[2][i] += 0.5 * (gw4 * v[i][0] + gw5 * v[i][1]);
+            w3 += v[i][0] * sh[1][i] - v[i][1] * sh[0][i];
+            w4 += v[i][0] * sh[2][i] - v[i][2] * sh[0][i];
+            w5 += v[i][1] * sh[2][i] - v[i][2] * sh[1][i];
         }
+        const double hdt = 0.5 * dt;
+        w3 *= hdt, w4 *= hdt, w5 *= hdt;
+        // s_out = s + dt * si(s, w) (jaumann3), bilinear in s and w
+        const double d01 = g[1] - g[0], d02 = g[2] - g[0], d12 = g[2] - g[1];
+        h3 = hdt * (2 * s[3] * d01 + (s[0] - s[1]) * g[3] - s[5] * g[4] + s[4] * g[5]);
+        h4 = hdt * (2 * s[4] * d02 - s[5] * g[3] + (s[0] - s[2]) * g[4] + s[3] * g[5]);
+        h5 = hdt * (2 * s[5] * d12 - s[4] * g[3] + s[3] * g[4] + (s[1] - s[2]) * g[5]);
+        a.as[0 * ne + e] = g[0] + g[3] * w3 + g[4] * w4;
+        a.as[1 * ne + e] = g[1] - g[3] * w3 + g[5] * w5;
+        a.as[2 * ne + e] = g[2] - g[4] * w4 - g[5] * w5;
+        a.as[3 * ne + e] = g[3] + 2 * w3 * d01 + g[4] * w5 + g[5] * w4;
+        a.as[4 * ne + e] = g[4] + 2 * w4 * d02 - g[3] * w5 + g[5] * w3;
+        a.as[5 * ne + e] = g[5] + 2 * w5 * d12 - g[3] * w4 - g[4] * w3;
     }
-    double gc[4][3] = {};
-    geom_reverse(c, vol, gs, gvol, gc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        a.slot3[((size_t)0 * 4 + i) * ne + e] = h3 * sh[1][i] + h4 * sh[2][i];
+        a.slot3[((size_t)1 * 4 + i) * ne + e] = h5 * sh[2][i] - h3 * sh[0][i];
+        a.slot3[((size_t)2 * 4 + i) * ne + e] = -h4 * sh[0][i] - h5 * sh[1][i];
+        gs[0][i] -= h3 * v[i][1] + h4 * v[i][2];
+        gs[1][i] += h3 * v[i][0] - h5 * v[i][2];
+        gs[2][i] += h4 * v[i][0] + h5 * v[i][1];
+    }
+    double gc[4][3];
+    geom_reverse(sh, vol, gs, gvol, gc);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            a.slot3[((size_t)d * 4 + i) * ne + e] = gv[i][d];
-            a.slotx[((size_t)d * 4 + i) * ne + e] = gc[i][d];
-        }
+        for (int d = 0; d < 3; ++d) a.slotx[((size_t)d * 4 + i) * ne + e] = gc[i][d];
 }
 
 int launch_adj_end_geometry(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
@@ -467,31 +431,37 @@ __global__ void __launch_bounds__(TPB_A) k_adj_force(KP p, AdjBufs a, TapeStep t
     const double buoy = (gravity != 0) ? t.rho[e] * gravity / 4 : 0.0;
     double gvol = a.avolo[e];
     a.avolo[e] = 0;
-    double grho = a.arho[e], gbuoy = 0;
+    double grho = a.arho[e];
     for (int q = a.e2f_off[e]; q < a.e2f_off[e + 1]; ++q) grho += a.frho[a.e2f_ent[q]];
+    // with F_lk = sum_i gf_i,l dN_i/dx_k over the nodes' force adjoints: the
+    // volume's adjoint is -(sigma : F + buoy sum gf_z), the stress's -vol sym(F)
+    // and dN_i/dx_k's -vol sum_l gf_i,l sigma_lk
+    double F[3][3] = {}, sv[6], fz = 0;
+#pragma unroll
+    for (int cc = 0; cc < 6; ++cc) sv[cc] = -vol * s[cc];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int n = conn_at(p, i, e);
         double gf[3];
-        tload3(a.af, nn, n, gf);
-        const double sx = tshp(t, ne, 0, i, e), sy = tshp(t, ne, 1, i, e), sz = tshp(t, ne, 2, i, e);
-        const double t0 = s[0] * sx + s[3] * sy + s[4] * sz;
-        const double t1 = s[3] * sx + s[1] * sy + s[5] * sz;
-        const double t2 = s[4] * sx + s[5] * sy + s[2] * sz + buoy;
-        gvol -= gf[0] * t0 + gf[1] * t1 + gf[2] * t2;
-        const double g0 = -gf[0] * vol, g1 = -gf[1] * vol, g2 = -gf[2] * vol;
-        gsig[0] += g0 * sx;
-        gsig[1] += g1 * sy;
-        gsig[2] += g2 * sz;
-        gsig[3] += g0 * sy + g1 * sx;
-        gsig[4] += g0 * sz + g2 * sx;
-        gsig[5] += g1 * sz + g2 * sy;
-        a.ashp[((size_t)0 * 4 + i) * ne + e] = g0 * s[0] + g1 * s[3] + g2 * s[4];
-        a.ashp[((size_t)1 * 4 + i) * ne + e] = g0 * s[3] + g1 * s[1] + g2 * s[5];
-        a.ashp[((size_t)2 * 4 + i) * ne + e] = g0 * s[4] + g1 * s[5] + g2 * s[2];
-        gbuoy += g2;
+        tload3(a.af, nn, conn_at(p, i, e), gf);
+        const double sh[3] = {tshp(t, ne, 0, i, e), tshp(t, ne, 1, i, e), tshp(t, ne, 2, i, e)};
+#pragma unroll
+        for (int l = 0; l < 3; ++l)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) F[l][k] += gf[l] * sh[k];
+        a.ashp[((size_t)0 * 4 + i) * ne + e] = gf[0] * sv[0] + gf[1] * sv[3] + gf[2] * sv[4];
+        a.ashp[((size_t)1 * 4 + i) * ne + e] = gf[0] * sv[3] + gf[1] * sv[1] + gf[2] * sv[5];
+        a.ashp[((size_t)2 * 4 + i) * ne + e] = gf[0] * sv[4] + gf[1] * sv[5] + gf[2] * sv[2];
+        fz += gf[2];
     }
-    if (gravity != 0) grho += gbuoy * gravity / 4;
+    const double f3 = F[0][1] + F[1][0], f4 = F[0][2] + F[2][0], f5 = F[1][2] + F[2][1];
+    gvol -= s[0] * F[0][0] + s[1] * F[1][1] + s[2] * F[2][2] + s[3] * f3 + s[4] * f4 + s[5] * f5 + buoy * fz;
+    gsig[0] -= vol * F[0][0];
+    gsig[1] -= vol * F[1][1];
+    gsig[2] -= vol * F[2][2];
+    gsig[3] -= vol * f3;
+    gsig[4] -= vol * f4;
+    gsig[5] -= vol * f5;
+    if (gravity != 0) grho -= vol * fz * gravity / 4;
 #pragma unroll
     for (int cc = 0; cc < 6; ++cc) a.as[cc * ne + e] = gsig[cc];
     a.avol[e] = gvol;
@@ -580,41 +550,37 @@ __device__ __forceinline__ void maxwell_reverse(double K, double G, double visc,
                                                 const double *s, const double *go, double *gs, double *gde,
                                                 double &gG, double &gvisc, double &gdv)
 {
+    // with the deviators x = s - s0, y = de - dev: out = (x f1 + 2G y) f2 (+ s0 + K dv)
     const double ivisc = recip_newton(visc);
     const double tmp = 0.5 * dt * G * ivisc;
     const double f1 = 1 - tmp, f2 = recip_newton(1 + tmp);
     const double dev = div3(de[0] + de[1] + de[2]), s0 = div3(s[0] + s[1] + s[2]);
-    double gf1 = 0, gf2 = 0, gs0 = 0, gdev = 0;
+    const double c = f1 * f2, d = 2 * G * f2;
+    double A = 0, B = 0;   // <go, x>, <go, y>
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const double u = (s[i] - s0) * f1 + 2 * G * (de[i] - dev);
-        gf2 += go[i] * u;
-        const double gu = go[i] * f2;
-        gs0 += go[i] - gu * f1;
-        gdv += K * go[i];
-        gs[i] += gu * f1;
-        gf1 += gu * (s[i] - s0);
-        gG += gu * 2 * (de[i] - dev);
-        gde[i] += 2 * G * gu;
-        gdev -= 2 * G * gu;
+        A += go[i] * (s[i] - s0);
+        B += go[i] * (de[i] - dev);
     }
 #pragma unroll
-    for (int c = 3; c < 6; ++c) {
-        const double u = s[c] * f1 + 2 * G * de[c];
-        gf2 += go[c] * u;
-        const double gu = go[c] * f2;
-        gs[c] += gu * f1;
-        gf1 += gu * s[c];
-        gG += 2 * gu * de[c];
-        gde[c] += 2 * G * gu;
+    for (int k = 3; k < 6; ++k) {
+        A += go[k] * s[k];
+        B += go[k] * de[k];
     }
+    const double tg = go[0] + go[1] + go[2], tg3 = div3(tg);
+    gdv += K * tg;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        gs[i] += div3(gs0);
-        gde[i] += div3(gdev);
+        gs[i] += c * go[i] + (tg3 - c * tg3);
+        gde[i] += d * (go[i] - tg3);
     }
-    const double gtmp = -gf1 - gf2 * f2 * f2;
-    gG += gtmp * 0.5 * dt * ivisc;
+#pragma unroll
+    for (int k = 3; k < 6; ++k) {
+        gs[k] += c * go[k];
+        gde[k] += d * go[k];
+    }
+    const double gtmp = -f2 * A - (f1 * A + 2 * G * B) * f2 * f2;
+    gG += 2 * f2 * B + gtmp * 0.5 * dt * ivisc;
     gvisc -= gtmp * tmp * ivisc;
 }
 
@@ -914,12 +880,12 @@ __global__ void __launch_bounds__(TPB_A) k_adj_stress(KP p, AdjBufs a, TapeStep 
         maxwell_reverse(K, G, visc, dt, de, s0, go, gs, gde, gG, gvisc, gdv);
     } else {   // EP or EVP
         double amc, anphi, anpsi, hardn, tmax;
-        m_plastic_props(p, e, pls, amc, anphi, anpsi, hardn, tmax);
         bool plastic = true;
         if (rt == DES_RH_EVP) {
             if (t.evp) {
                 plastic = t.evp[e] != 0;
             } else {
+                m_plastic_props(p, e, pls, amc, anphi, anpsi, hardn, tmax);
                 const double dv = vol / volo - 1;
                 double sv[6], sp[6];
 #pragma unroll
@@ -933,6 +899,7 @@ __global__ void __launch_bounds__(TPB_A) k_adj_stress(KP p, AdjBufs a, TapeStep 
             }
         }
         if (plastic) {
+            m_plastic_props(p, e, pls, amc, anphi, anpsi, hardn, tmax);
             double S[6];   // the elastic trial stress
 #pragma unroll
             for (int cc = 0; cc < 6; ++cc) S[cc] = s0[cc];
@@ -1048,67 +1015,48 @@ __global__ void __launch_bounds__(TPB_A) k_adj_kinematics(KP p, AdjBufs a, TapeS
     }
     double gTn[4] = {0, 0, 0, 0};
     if (p.prm.has_thermal_diffusion) {
-        double Tn[4], gtd[4];
+        // tdot_i = kv g_i . G - rh with the temperature gradient G = sum_j g_j
+        // (T_j - T_0) (the gradients sum to zero): with U = sum_i gtd_i g_i,
+        // the adjoints are U . G of kv, kv g_j . U of T_j and kv (gtd_m G +
+        // (T_m - T_0) U) of g_m (a common change of the g_m does not occur)
+        double Td[4], gtd[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            Tn[i] = t.T[nodes[i]];
+            Td[i] = t.T[nodes[i]];
             gtd[i] = a.atdot[nodes[i]];
         }
+        const double T0 = Td[0];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) Td[i] -= T0;
         const double k = m_k(p, e), kv = k * vol, hrcp = p.mat.hr_over_cp;
-        double gkv = 0, grh = 0;
-        // tdot_i = kv sum_j D_ij T_j - rh with the symmetric D_ij = dN_i . dN_j:
-        // D is formed once (10 entries), and the adjoints of D_ij and D_ji,
-        // kg_i T_j and kg_j T_i (kg = kv gtd), are folded into one symmetric
-        // H_mk, so that d/d dN_m = sum_k H_mk dN_k
-        double D[4][4], kg[4];
+        double gkv = 0;
+        const double grh = -((gtd[0] + gtd[1]) + (gtd[2] + gtd[3]));
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            kg[i] = kv * gtd[i];
+        for (int c = 0; c < 3; ++c) {
+            const double G = sh[c][1] * Td[1] + sh[c][2] * Td[2] + sh[c][3] * Td[3];
+            const double U = sh[c][0] * gtd[0] + sh[c][1] * gtd[1] + sh[c][2] * gtd[2] + sh[c][3] * gtd[3];
+            gkv += U * G;
+            const double kG = kv * G, kU = kv * U;
+            gsh[c][0] += gtd[0] * kG;
 #pragma unroll
-            for (int j = i; j < 4; ++j) {
-                D[i][j] = sh[0][i] * sh[0][j] + sh[1][i] * sh[1][j] + sh[2][i] * sh[2][j];
-                D[j][i] = D[i][j];
-            }
+            for (int m = 1; m < 4; ++m) gsh[c][m] += gtd[m] * kG + Td[m] * kU;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) gTn[m] += sh[c][m] * kU;
         }
-        double H[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            double diffusion = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                diffusion += D[i][j] * Tn[j];
-                gTn[i] += D[i][j] * kg[j];
-            }
-            gkv += gtd[i] * diffusion;
-            grh -= gtd[i];
-#pragma unroll
-            for (int j = i; j < 4; ++j) {
-                H[i][j] = kg[i] * Tn[j] + kg[j] * Tn[i];
-                H[j][i] = H[i][j];
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                double acc = 0;
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk) acc += H[m][kk] * sh[c][kk];
-                gsh[c][m] += acc;
-            }
         a.g[(size_t)DES_EF_THERM_COND * ne + e] += gkv * vol;
         gvol += gkv * k + grh * hrcp;
     }
     // strain rate
+    const double h3 = 0.5 * g[3], h4 = 0.5 * g[4], h5 = 0.5 * g[5];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const double sx = sh[0][i], sy = sh[1][i], sz = sh[2][i];
-        const double gv0 = g[0] * sx + 0.5 * g[3] * sy + 0.5 * g[4] * sz;
-        const double gv1 = g[1] * sy + 0.5 * g[3] * sx + 0.5 * g[5] * sz;
-        const double gv2 = g[2] * sz + 0.5 * g[4] * sx + 0.5 * g[5] * sy;
-        gsh[0][i] += g[0] * v[i][0] + 0.5 * g[3] * v[i][1] + 0.5 * g[4] * v[i][2];
-        gsh[1][i] += g[1] * v[i][1] + 0.5 * g[3] * v[i][0] + 0.5 * g[5] * v[i][2];
-        gsh[2][i] += g[2] * v[i][2] + 0.5 * g[4] * v[i][0] + 0.5 * g[5] * v[i][1];
+        const double gv0 = g[0] * sx + h3 * sy + h4 * sz;
+        const double gv1 = g[1] * sy + h3 * sx + h5 * sz;
+        const double gv2 = g[2] * sz + h4 * sx + h5 * sy;
+        gsh[0][i] += g[0] * v[i][0] + h3 * v[i][1] + h4 * v[i][2];
+        gsh[1][i] += g[1] * v[i][1] + h3 * v[i][0] + h5 * v[i][2];
+        gsh[2][i] += g[2] * v[i][2] + h4 * v[i][0] + h5 * v[i][1];
         a.slot3[((size_t)0 * 4 + i) * ne + e] = gv0;
         a.slot3[((size_t)1 * 4 + i) * ne + e] = gv1;
         a.slot3[((size_t)2 * 4 + i) * ne + e] = gv2;
@@ -1147,13 +1095,12 @@ __global__ void __launch_bounds__(TPB_A) k_adj_start_geometry(KP p, AdjBufs a, T
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= p.ne) return;
-    const size_t ne = p.ne, nn = p.nn;
+    const size_t ne = p.ne;
     int nodes[4];
-    double c[4][3], Tsum = 0;
+    double sh[3][4], Tsum = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         nodes[i] = conn_at(p, i, e);
-        tload3(t.x, nn, nodes[i], c[i]);
         Tsum += t.T[nodes[i]];
     }
     const double rho_e = m_rho_T(p, e, Tsum / 4);
@@ -1165,12 +1112,15 @@ __global__ void __launch_bounds__(TPB_A) k_adj_start_geometry(KP p, AdjBufs a, T
         gtm[i] = a.atm[nodes[i]];
         gvn[i] = a.avn[nodes[i]];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) gs[k][i] = a.ashp[((size_t)k * 4 + i) * ne + e];
+        for (int k = 0; k < 3; ++k) {
+            sh[k][i] = tshp(t, ne, k, i, e);
+            gs[k][i] = a.ashp[((size_t)k * 4 + i) * ne + e];
+        }
     }
     const double grho = mass_reverse(p, e, gm, gtm, gvn, t.vol[e], rho_e, gvol);
     const double gT = grho * (-p.mat.rho0[0] * p.mat.alpha[0]);
-    double gc[4][3] = {};
-    geom_reverse(c, t.vol[e], gs, gvol, gc);
+    double gc[4][3];
+    geom_reverse(sh, t.vol[e], gs, gvol, gc);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
 #pragma unroll
