@@ -549,7 +549,11 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
                              c->stream);
         if (e1 == cudaSuccess) e1 = cudaStreamSynchronize(c->stream);
         if (e1 == cudaSuccess) {
-            for (int m = 0; m < nm; ++m) p.mat.visc_coef[m] = tab[m];
+            for (int m = 0; m < nm; ++m) {
+                p.mat.visc_coef[m] = tab[m];
+                p.mat.visc_coef4[m] = 0.25 * tab[m];
+                p.mat.visc_nr[m] = p.mat.visc_exponent[m] * 8.3144;   // IEEE: the bits of the per-element product
+            }
             p.mat.visc_skip_empty = 1;
             for (int m = 0; m < nm; ++m) {
                 p.mat.visc_lnc[m] = std::log(0.25e6 * tab[m]);

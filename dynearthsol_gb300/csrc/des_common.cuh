@@ -62,6 +62,8 @@ struct MatC {
     double visc_pw[DES_MAXMAT];      // 1 / n - 1               (matprops.cxx:298)
     double visc_pw1[DES_MAXMAT];     // -1 / n                  (matprops.cxx:299)
     double visc_coef[DES_MAXMAT];    // pow(0.75 * A, -1 / n)   (matprops.cxx:300)
+    double visc_coef4[DES_MAXMAT];   // 0.25 * visc_coef (an exact scaling, matprops.cxx:300-301)
+    double visc_nr[DES_MAXMAT];      // n * R                   (matprops.cxx:301)
     double rho_pseudo;               // bulkm / (v_max * inertial_scaling)^2 (geometry.cxx:348-349), nmat == 1
     double visc_lnc[DES_MAXMAT];     // ln(0.25e6 * visc_coef[m])   (mixed step)
     double visc_lnmin, visc_lnmax;   // ln(visc_min), ln(visc_max)  (mixed step)
@@ -339,9 +341,9 @@ __device__ __forceinline__ double m_hr_over_cp(const KP &p, int e)
 template <int NPE>
 __device__ __forceinline__ double elem_avg_T(const KP &p, int e)
 {
-    double t = 0;
+    double t = p.T[p.conn[e]];
 #pragma unroll
-    for (int i = 0; i < NPE; ++i) t += p.T[p.conn[(size_t)i * p.ne + e]];
+    for (int i = 1; i < NPE; ++i) t += p.T[p.conn[(size_t)i * p.ne + e]];
     return t / NPE;
 }
 
@@ -380,7 +382,6 @@ __device__ double m_visc(const KP &p, int e, const double *edot)
     if (p.ef[DES_EF_LOG10_VISC]) {
         v = pow(10.0, p.ef[DES_EF_LOG10_VISC][e]);
     } else {
-        const double gas_constant = 8.3144;
         const double min_strain_rate = 1e-30;
         double T = elem_avg_T<ND + 1>(p, e);
         double ed = second_invariant_<ND>(edot);
@@ -392,8 +393,8 @@ __device__ double m_visc(const KP &p, int e, const double *edot)
             int k = mcount(p, e, m);
             if (k == 0 && skip_empty) continue;   // k / visc0 = +0 exactly
             const double pw = p.mat.visc_pw[m];
-            const double visc0 = 0.25 * pow(ed, pw) * p.mat.visc_coef[m]
-                * exp(p.mat.visc_activation_energy[m] / (p.mat.visc_exponent[m] * gas_constant * T)) * 1e6;
+            const double visc0 = pow(ed, pw) * p.mat.visc_coef4[m]
+                * exp(p.mat.visc_activation_energy[m] / (p.mat.visc_nr[m] * T)) * 1e6;
             result += k / visc0;
             n += k;
         }

@@ -43,35 +43,32 @@ __device__ __forceinline__ void strain_rate_elem(const KP &p, int e, double *s)
         if (ND == 3) sy[i] = shp_at(p, 1, i, e);
         sz[i] = shp_at(p, ND - 1, i, e);
     }
+    // The sums start from their first term, and the halves of the shear
+    // components are taken once per sum (a scaling by two commutes with every
+    // rounding above the subnormal range): the reference's bits with 15 of
+    // the 84 FP64 operations left out.
+    const auto normal = [&](int d, const double *sd) {
+        double t = v[0][d] * sd[0];
+#pragma unroll
+        for (int i = 1; i < NPE; ++i) t += v[i][d] * sd[i];
+        return t;
+    };
+    const auto shear = [&](int d, const double *sk, int k, const double *sd) {   // 0.5 (dv_d/dx_k + dv_k/dx_d)
+        double t = v[0][d] * sk[0] + v[0][k] * sd[0];
+#pragma unroll
+        for (int i = 1; i < NPE; ++i) t += v[i][d] * sk[i] + v[i][k] * sd[i];
+        return 0.5 * t;
+    };
+    s[0] = normal(0, sx);
     if (ND == 3) {
-        s[0] = 0;
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) s[0] += v[i][0] * sx[i];
-        s[1] = 0;
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) s[1] += v[i][1] * sy[i];
-        s[2] = 0;
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) s[2] += v[i][ND - 1] * sz[i];
-        s[3] = 0;
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) s[3] += 0.5 * (v[i][0] * sy[i] + v[i][1] * sx[i]);
-        s[4] = 0;
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) s[4] += 0.5 * (v[i][0] * sz[i] + v[i][ND - 1] * sx[i]);
-        s[5] = 0;
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) s[5] += 0.5 * (v[i][1] * sz[i] + v[i][ND - 1] * sy[i]);
+        s[1] = normal(1, sy);
+        s[2] = normal(ND - 1, sz);
+        s[3] = shear(0, sy, 1, sx);
+        s[4] = shear(0, sz, ND - 1, sx);
+        s[5] = shear(1, sz, ND - 1, sy);
     } else {
-        s[0] = 0;
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) s[0] += v[i][0] * sx[i];
-        s[1] = 0;
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) s[1] += v[i][ND - 1] * sz[i];
-        s[2] = 0;
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) s[2] += 0.5 * (v[i][0] * sz[i] + v[i][ND - 1] * sx[i]);
+        s[1] = normal(ND - 1, sz);
+        s[2] = shear(0, sz, ND - 1, sx);
     }
 }
 
@@ -195,9 +192,9 @@ __global__ void __launch_bounds__(TPB) k_elem_pass(KP p, int heat)
         }
 #pragma unroll
     for (int i = 0; i < NPE; ++i) {
-        double diffusion = 0;
+        double diffusion = D[i][0] * T[0];
 #pragma unroll
-        for (int j = 0; j < NPE; ++j) diffusion += D[i][j] * T[j];
+        for (int j = 1; j < NPE; ++j) diffusion += D[i][j] * T[j];
         p.hc64[(size_t)i * ne + e] = diffusion * kv - rh;
     }
 }
@@ -794,18 +791,21 @@ __device__ __forceinline__ void rel_shape_fn_dw(const RelEdges &r, const double 
     }
 }
 
-// jaumann_rate_3d / _2d (fields.cxx:375-404)
-__device__ __forceinline__ void jaumann3(double *s, double dt, double w3, double w4, double w5)
+// jaumann_rate_3d / _2d (fields.cxx:375-404).  The normal components' factors
+// of two are taken into the time step (dt2 = 2 dt) and their three products
+// shared: the reference's bits, as a scaling by two commutes with rounding.
+__device__ __forceinline__ void jaumann3(double *s, double dt, double dt2, double w3, double w4, double w5)
 {
-    double si[6];
-    si[0] = -2.0 * s[3] * w3 - 2.0 * s[4] * w4;
-    si[1] = 2.0 * s[3] * w3 - 2.0 * s[5] * w5;
-    si[2] = 2.0 * s[4] * w4 + 2.0 * s[5] * w5;
-    si[3] = s[0] * w3 - s[1] * w3 - s[4] * w5 - s[5] * w4;
-    si[4] = s[0] * w4 - s[2] * w4 + s[3] * w5 - s[5] * w3;
-    si[5] = s[1] * w5 - s[2] * w5 + s[3] * w4 + s[4] * w3;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) s[i] += dt * si[i];
+    const double a = s[3] * w3, b = s[4] * w4, c = s[5] * w5;
+    const double s3 = s[0] * w3 - s[1] * w3 - s[4] * w5 - s[5] * w4;
+    const double s4 = s[0] * w4 - s[2] * w4 + s[3] * w5 - s[5] * w3;
+    const double s5 = s[1] * w5 - s[2] * w5 + s[3] * w4 + s[4] * w3;
+    s[0] -= dt2 * (a + b);
+    s[1] += dt2 * (a - c);
+    s[2] += dt2 * (b + c);
+    s[3] += dt * s3;
+    s[4] += dt * s4;
+    s[5] += dt * s5;
 }
 
 __device__ __forceinline__ void jaumann2(double *s, double dt, double w2)
@@ -1032,15 +1032,20 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
                 es[cc] = p.strain[cc * ne + e];
             }
             if (ND == 3) {
-                double w3 = 0, w4 = 0, w5 = 0;
+                // the halves are taken once per sum (the same bits)
+                double w3 = v[0][0] * shp[1][0] - v[0][1] * shp[0][0];
+                double w4 = v[0][0] * shp[ND - 1][0] - v[0][ND - 1] * shp[0][0];
+                double w5 = v[0][1] * shp[ND - 1][0] - v[0][ND - 1] * shp[1][0];
 #pragma unroll
-                for (int i = 0; i < NPE; ++i) w3 += 0.5 * (v[i][0] * shp[1][i] - v[i][1] * shp[0][i]);
-#pragma unroll
-                for (int i = 0; i < NPE; ++i) w4 += 0.5 * (v[i][0] * shp[ND - 1][i] - v[i][ND - 1] * shp[0][i]);
-#pragma unroll
-                for (int i = 0; i < NPE; ++i) w5 += 0.5 * (v[i][1] * shp[ND - 1][i] - v[i][ND - 1] * shp[1][i]);
-                jaumann3(s, dt, w3, w4, w5);
-                jaumann3(es, dt, w3, w4, w5);
+                for (int i = 1; i < NPE; ++i) {
+                    w3 += v[i][0] * shp[1][i] - v[i][1] * shp[0][i];
+                    w4 += v[i][0] * shp[ND - 1][i] - v[i][ND - 1] * shp[0][i];
+                    w5 += v[i][1] * shp[ND - 1][i] - v[i][ND - 1] * shp[1][i];
+                }
+                w3 *= 0.5, w4 *= 0.5, w5 *= 0.5;
+                const double dt2 = dt + dt;
+                jaumann3(s, dt, dt2, w3, w4, w5);
+                jaumann3(es, dt, dt2, w3, w4, w5);
             } else {
                 double w2 = 0;
 #pragma unroll
@@ -1061,8 +1066,12 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
             const double rho = p.prm.is_quasi_static
                 ? ((p.mat.nmat == 1) ? p.mat.rho_pseudo : m_bulkm(p, e) / (pseudo_speed * pseudo_speed))
                 : rho_e;
-            const double me = rho * vol / NPE;
-            const double tme = p.prm.has_thermal_diffusion ? rho_e * m_cp(p, e) * vol / NPE : 0.0;
+            // in 3D the division by 4 is exact: taken once, on the volume
+            const double v4 = ND == 3 ? vol / NPE : vol;
+            const double me = ND == 3 ? rho * v4 : rho * vol / NPE;
+            double tme = 0.0;
+            if (p.prm.has_thermal_diffusion)
+                tme = ND == 3 ? rho_e * m_cp(p, e) * v4 : rho_e * m_cp(p, e) * vol / NPE;
             if constexpr (AHEAD) {
                 // what the next node pass gathers per support entry, in one
                 // 32-byte record (one sector instead of four)
