@@ -11,10 +11,12 @@
 // finite differences, not bit for bit: divisions by 3 are div3, and the
 // reciprocals of the common paths are recip_newton (~1e-14 relative), each
 // a few FP64 instructions instead of an FP64 division.
+#include <algorithm>
 #include <cfloat>
 
 #include "des_adjoint.cuh"
 #include "des_bc.cuh"
+#include "des_gather.cuh"
 #include "des_kernels.cuh"
 #include "des_rheology.cuh"
 
@@ -25,12 +27,6 @@ constexpr int TPB_A = 128;
 // DES_LAUNCH for kernels of at most TPB_A threads a block
 #define DES_LAUNCH_A(KERNEL, n, s, ...) \
     KERNEL<<<grid_blocks(n, TPB_A), block_threads(n, TPB_A), 0, (s)>>>(__VA_ARGS__)
-
-static inline int nblk(long long n, int tpb = TPB_A)
-{
-    long long b = (n + tpb - 1) / tpb;
-    return (int)(b < 1 ? 1 : b);
-}
 
 __device__ __forceinline__ double tshp(const TapeStep &t, size_t ne, int k, int i, int e)
 {
@@ -231,37 +227,35 @@ __device__ __forceinline__ double damp_deriv(const KP &p, double f, double v)
 // foundation and the damping.  Writes ax (coordinate adjoint, start of the
 // step), av (velocity adjoint, before the strain-rate share), af (adjoint
 // of the undamped force), am (mass adjoint of the start), clears atm and
-// avn, and adds the per-block sums of the prescribed-value adjoints to gvbc.
+// avn, and adds the sums of the prescribed-value adjoints to gvbc.
 // ------------------------------------------------------------------
-__global__ void __launch_bounds__(TPB_A) k_adj_motion(KP p, AdjBufs a, TapeStep t, TapeStep t1, double dt)
+template <bool STAGED>
+__global__ void __launch_bounds__(128) k_adj_motion(KP p, AdjBufs a, TapeStep t, TapeStep t1, double dt)
 {
-    __shared__ double red[DES_NBDRYTYPES][TPB_A];
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const size_t ne = p.ne, nn = p.nn;
+    double sum[6] = {};   // coordinate and velocity contributions
+    const int n = node_sums<SumF64, 6, 3, STAGED>(
+        p.sup_off, 0, p.nn, 6,
+        [&](int q, double *s) {
+            const int ent = p.sup_ent[q];
+            const int e = ent >> 2, k = ent & 3;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                s[d] = a.slotx[((size_t)d * 4 + k) * ne + e];
+                s[3 + d] = a.slot3[((size_t)d * 4 + k) * ne + e];
+            }
+        },
+        [&](int c, int m) { return c < 3 ? a.ax[c * nn + m] : a.av[(c - 3) * nn + m]; }, sum);
     double gva[DES_NBDRYTYPES];
 #pragma unroll
     for (int ib = 0; ib < DES_NBDRYTYPES; ++ib) gva[ib] = 0;
-    if (n < p.nn) {
-        double gx[3], gv[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            gx[d] = a.ax[d * nn + n];
-            gv[d] = a.av[d * nn + n];
-        }
-        for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-            const int ent = p.sup_ent[q];
-            const int e = ent >> 2, i = ent & 3;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                gx[d] += a.slotx[((size_t)d * 4 + i) * ne + e];
-                gv[d] += a.slot3[((size_t)d * 4 + i) * ne + e];
-            }
-        }
+    const unsigned flag = n >= 0 ? p.bcflag[n] : 0u;
+    if (n >= 0) {
+        double gx[3] = {sum[0], sum[1], sum[2]}, gv[3] = {sum[3], sum[4], sum[5]};
         // x' = x + v' dt
 #pragma unroll
         for (int d = 0; d < 3; ++d) gv[d] += dt * gx[d];
         // v' = BC(pre): gpre = A^T gv, gva = B^T gv
-        const unsigned flag = p.bcflag[n];
         double gpre[3] = {gv[0], gv[1], gv[2]};
         if (flag & BOUND_ANY) {
             double zero[DES_NBDRYTYPES];
@@ -302,27 +296,30 @@ __global__ void __launch_bounds__(TPB_A) k_adj_motion(KP p, AdjBufs a, TapeStep 
         a.atm[n] = 0;
         a.avn[n] = 0;
     }
-    // fixed-order block sums of the prescribed-value adjoints
+    // fixed-order sums of the prescribed-value adjoints over the warp's nodes
+    if (!__any_sync(0xffffffffu, flag & BOUND_ANY)) return;
+    const size_t part = STAGED ? blockIdx.x : (blockIdx.x * blockDim.x + threadIdx.x) / 32;
 #pragma unroll
-    for (int ib = 0; ib < DES_NBDRYTYPES; ++ib) red[ib][threadIdx.x] = gva[ib];
-    __syncthreads();
-    for (int w = TPB_A / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
+    for (int ib = 0; ib < DES_NBDRYTYPES; ++ib) {
+        double g = gva[ib];
 #pragma unroll
-            for (int ib = 0; ib < DES_NBDRYTYPES; ++ib) red[ib][threadIdx.x] += red[ib][threadIdx.x + w];
-        __syncthreads();
+        for (int w = 16; w > 0; w >>= 1) g += __shfl_down_sync(0xffffffffu, g, w);
+        if ((threadIdx.x & 31) == 0) a.gvbc[part * DES_NBDRYTYPES + ib] += g;
     }
-    if (threadIdx.x < DES_NBDRYTYPES) a.gvbc[(size_t)blockIdx.x * DES_NBDRYTYPES + threadIdx.x] += red[threadIdx.x][0];
 }
 
 int launch_adj_motion(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
                       cudaStream_t s)
 {
-    k_adj_motion<<<nblk(p.nn), TPB_A, 0, s>>>(p, a, t, t1, dt);
+    DES_NODES(k_adj_motion<STAGED>, p.nn, s, p, a, t, t1, dt);
     return 1;
 }
 
-int adj_vbc_blocks(const KP &p) { return nblk(p.nn); }
+int adj_vbc_parts(const KP &p)
+{
+    const int nodes = node_staged(p.nn) ? NPB : 32;   // a block's, or a warp's
+    return (p.nn + nodes - 1) / nodes;
+}
 
 // ------------------------------------------------------------------
 // stress BCs of one boundary facet (bc.cxx:493-566), reversed.  The facet
@@ -474,13 +471,14 @@ __global__ void __launch_bounds__(TPB_A) k_adj_force(KP p, AdjBufs a, TapeStep t
 
 // nodes: NMD nodal sum reversed (dpn = sum_e dp_e vol_e / volume_n), and the
 // facets' coordinate adjoints added to ax
-__global__ void __launch_bounds__(TPB_A) k_adj_nmd_nodes(KP p, AdjBufs a, TapeStep t)
+template <bool STAGED>
+__global__ void __launch_bounds__(128) k_adj_nmd_nodes(KP p, AdjBufs a, TapeStep t)
 {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.nn) return;
     const size_t nn = p.nn, nbf = p.nbf;
-    double acc = 0;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) acc += a.slot1[p.sup_ent[q] >> 2];
+    double acc;
+    const int n = node_sums<SumF64, 1, 3, STAGED>(
+        p.sup_off, 0, p.nn, 1, [&](int q, double *s) { *s = a.slot1[p.sup_ent[q] >> 2]; }, FromZero<SumF64>(), &acc);
+    if (n < 0) return;
     const double ivn = recip_newton(t.voln[n]);
     a.adpn[n] = acc * ivn;
     a.avn[n] -= acc * t.dpn[n] * ivn;
@@ -514,7 +512,7 @@ int launch_adj_force(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStrea
 
 int launch_adj_nmd_nodes(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStream_t s)
 {
-    DES_LAUNCH_A(k_adj_nmd_nodes, p.nn, s, p, a, t);
+    DES_NODES(k_adj_nmd_nodes<STAGED>, p.nn, s, p, a, t);
     return 1;
 }
 
@@ -947,18 +945,22 @@ __global__ void __launch_bounds__(TPB_A) k_adj_stress(KP p, AdjBufs a, TapeStep 
 // T' terms), nodal dvoldt (ntmp = sum_e tr(edot) vol / volume_n, edvoldt =
 // mean of ntmp), and the temperature update with its Dirichlet BCs
 // (fields.cxx:151-162): T' = T - tdot dt / tmass
-__global__ void __launch_bounds__(TPB_A) k_adj_nodes_heat(KP p, AdjBufs a, TapeStep t, TapeStep t1, double dt)
+template <bool STAGED>
+__global__ void __launch_bounds__(128) k_adj_nodes_heat(KP p, AdjBufs a, TapeStep t, TapeStep t1, double dt)
 {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.nn) return;
     const size_t ne = p.ne;
-    double gTp = a.aT[n], gnt = 0;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        const int ent = p.sup_ent[q];
-        const int e = ent >> 2, i = ent & 3;
-        gTp += a.slot1[(size_t)i * ne + e];
-        gnt += a.aedv[e] / 4;
-    }
+    double sum[2];   // adjoints of the updated temperature and of dvoldt
+    const int n = node_sums<SumF64, 2, 3, STAGED>(
+        p.sup_off, 0, p.nn, 2,
+        [&](int q, double *s) {
+            const int ent = p.sup_ent[q];
+            const int e = ent >> 2, k = ent & 3;
+            s[0] = a.slot1[(size_t)k * ne + e];
+            s[1] = a.aedv[e] / 4;
+        },
+        [&](int c, int m) { return c == 0 ? a.aT[m] : 0.0; }, sum);
+    if (n < 0) return;
+    const double gTp = sum[0], gnt = sum[1];
     const double vn = t.voln[n];
     a.antmp[n] = gnt / vn;
     a.avn[n] -= gnt * t.ntmp[n] / vn;
@@ -1069,23 +1071,33 @@ __global__ void __launch_bounds__(TPB_A) k_adj_kinematics(KP p, AdjBufs a, TapeS
     a.avol[e] = gvol;
 }
 
-// nodes: add the element contributions to the velocity and temperature adjoints
-__global__ void __launch_bounds__(TPB_A) k_adj_gather_vT(KP p, AdjBufs a)
+// a vector slot array and slot1 summed onto out [3][nn] and aT
+template <bool STAGED>
+__device__ __forceinline__ void gather_slots(const KP &p, const AdjBufs &a, const double *slot, double *out)
 {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.nn) return;
     const size_t ne = p.ne, nn = p.nn;
-    double gv[3] = {0, 0, 0}, gT = 0;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        const int ent = p.sup_ent[q];
-        const int e = ent >> 2, i = ent & 3;
+    double sum[4];
+    const int n = node_sums<SumF64, 4, 3, STAGED>(
+        p.sup_off, 0, p.nn, 4,
+        [&](int q, double *s) {
+            const int ent = p.sup_ent[q];
+            const int e = ent >> 2, k = ent & 3;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) gv[d] += a.slot3[((size_t)d * 4 + i) * ne + e];
-        gT += a.slot1[(size_t)i * ne + e];
-    }
+            for (int d = 0; d < 3; ++d) s[d] = slot[((size_t)d * 4 + k) * ne + e];
+            s[3] = a.slot1[(size_t)k * ne + e];
+        },
+        FromZero<SumF64>(), sum);
+    if (n < 0) return;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) a.av[d * nn + n] += gv[d];
-    a.aT[n] += gT;
+    for (int d = 0; d < 3; ++d) out[d * nn + n] += sum[d];
+    a.aT[n] += sum[3];
+}
+
+// nodes: add the element contributions to the velocity and temperature adjoints
+template <bool STAGED>
+__global__ void __launch_bounds__(128) k_adj_gather_vT(KP p, AdjBufs a)
+{
+    gather_slots<STAGED>(p, a, a.slot3, a.av);
 }
 
 // window start: adjoints of the derived fields (volume, shape functions,
@@ -1129,22 +1141,10 @@ __global__ void __launch_bounds__(TPB_A) k_adj_start_geometry(KP p, AdjBufs a, T
     }
 }
 
-__global__ void __launch_bounds__(TPB_A) k_adj_gather_xT(KP p, AdjBufs a)
+template <bool STAGED>
+__global__ void __launch_bounds__(128) k_adj_gather_xT(KP p, AdjBufs a)
 {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.nn) return;
-    const size_t ne = p.ne, nn = p.nn;
-    double gx[3] = {0, 0, 0}, gT = 0;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        const int ent = p.sup_ent[q];
-        const int e = ent >> 2, i = ent & 3;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) gx[d] += a.slotx[((size_t)d * 4 + i) * ne + e];
-        gT += a.slot1[(size_t)i * ne + e];
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) a.ax[d * nn + n] += gx[d];
-    a.aT[n] += gT;
+    gather_slots<STAGED>(p, a, a.slotx, a.ax);
 }
 
 int launch_adj_stress(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
@@ -1157,7 +1157,7 @@ int launch_adj_stress(const KP &p, const AdjBufs &a, const TapeStep &t, const Ta
 int launch_adj_nodes_heat(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
                           cudaStream_t s)
 {
-    DES_LAUNCH_A(k_adj_nodes_heat, p.nn, s, p, a, t, t1, dt);
+    DES_NODES(k_adj_nodes_heat<STAGED>, p.nn, s, p, a, t, t1, dt);
     return 1;
 }
 
@@ -1169,7 +1169,7 @@ int launch_adj_kinematics(const KP &p, const AdjBufs &a, const TapeStep &t, cuda
 
 int launch_adj_gather_vT(const KP &p, const AdjBufs &a, cudaStream_t s)
 {
-    DES_LAUNCH_A(k_adj_gather_vT, p.nn, s, p, a);
+    DES_NODES(k_adj_gather_vT<STAGED>, p.nn, s, p, a);
     return 1;
 }
 
@@ -1181,7 +1181,7 @@ int launch_adj_start_geometry(const KP &p, const AdjBufs &a, const TapeStep &t, 
 
 int launch_adj_gather_xT(const KP &p, const AdjBufs &a, cudaStream_t s)
 {
-    DES_LAUNCH_A(k_adj_gather_xT, p.nn, s, p, a);
+    DES_NODES(k_adj_gather_xT<STAGED>, p.nn, s, p, a);
     return 1;
 }
 

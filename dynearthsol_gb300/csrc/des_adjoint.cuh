@@ -55,7 +55,7 @@ struct AdjBufs {
     double *frho;                    // [nbf] facet -> element density adjoint
     const int *e2f_off, *e2f_ent;    // element -> boundary facets (ascending facet id)
     double *g;                       // [7][ne] parameter gradients (DES_EF_* order)
-    double *gvbc;                    // [nblk][DES_NBDRYTYPES] per-block partial sums
+    double *gvbc;                    // [nblk][DES_NBDRYTYPES] partial sums of a block or warp of nodes
 };
 
 // adjoint-state kernels of one step, launched in this order by the host
@@ -74,6 +74,6 @@ int launch_adj_gather_vT(const KP &p, const AdjBufs &a, cudaStream_t s);
 // adjoint of the derived fields at the window start -> coordinates and temperature
 int launch_adj_start_geometry(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStream_t s);
 int launch_adj_gather_xT(const KP &p, const AdjBufs &a, cudaStream_t s);
-int adj_vbc_blocks(const KP &p);
+int adj_vbc_parts(const KP &p);
 
 }  // namespace des

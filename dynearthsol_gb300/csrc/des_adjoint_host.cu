@@ -142,7 +142,7 @@ int alloc_buffers(des_ctx *c, AdjWork *w)
     if (w->buf_mem) return DES_OK;
     const size_t nn = c->nn, ne = c->ne, nbf = std::max(c->nbf, 1), D = sizeof(double);
     AdjBufs &a = w->a;
-    w->nblk_vbc = adj_vbc_blocks(c->kp);
+    w->nblk_vbc = adj_vbc_parts(c->kp);
     Carver cv;
     int *e2f_off, *e2f_ent;
     cv.add((void **)&a.ax, 3 * nn * D);

@@ -10,10 +10,13 @@
 // (the library is compiled without FMA contraction), so FP64 results track
 // the reference's CPU run to the last few ulps of the transcendental
 // functions.
+#include <algorithm>
+
 #include "des_kernels.cuh"
 #include "des_rheology.cuh"
 #include "des_bc.cuh"
 #include "des_dw.cuh"
+#include "des_gather.cuh"
 #include "des_mixed_elem.cuh"
 
 namespace des {
@@ -118,26 +121,28 @@ __device__ __forceinline__ double heat_term(const KP &p, int e, int i)
     return diffusion * kv - rh;
 }
 
-template <int ND, bool HEAT, bool DVOLDT>
-__global__ void __launch_bounds__(TPB) k_node_gather1(KP p)
+template <int ND, bool HEAT, bool DVOLDT, bool STAGED>
+__global__ void __launch_bounds__(128) k_node_gather1(KP p)
 {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.nn) return;
-    int b = p.sup_off[n], end = p.sup_off[n + 1];
-    double tdot = 0, dvoldt = 0;
-    for (int q = b; q < end; ++q) {
-        int ent = p.sup_ent[q];
-        int e = ent >> 2, i = ent & 3;
-        if (HEAT) tdot += heat_term<ND>(p, e, i);
-        if (DVOLDT) {
-            double dj;
-            if (ND == 3) dj = p.srate[e] + p.srate[(size_t)p.ne + e] + p.srate[2 * (size_t)p.ne + e];
-            else dj = p.srate[e] + p.srate[(size_t)p.ne + e];
-            dvoldt += dj * p.vol[e];
-        }
-    }
-    if (HEAT) p.tdot[n] = tdot;
-    if (DVOLDT) p.ntmp[n] = dvoldt / p.vol_n[n];
+    constexpr int NQ = (int)HEAT + (int)DVOLDT;
+    double sum[NQ];
+    const int n = node_sums<SumF64, NQ, ND, STAGED>(
+        p.sup_off, 0, p.nn, NQ,
+        [&](int q, double *t) {
+            const int ent = p.sup_ent[q];
+            const int e = ent >> 2, i = ent & 3;
+            if (HEAT) t[0] = heat_term<ND>(p, e, i);
+            if (DVOLDT) {
+                double dj;
+                if (ND == 3) dj = p.srate[e] + p.srate[(size_t)p.ne + e] + p.srate[2 * (size_t)p.ne + e];
+                else dj = p.srate[e] + p.srate[(size_t)p.ne + e];
+                t[NQ - 1] = dj * p.vol[e];
+            }
+        },
+        FromZero<SumF64>(), sum);
+    if (n < 0) return;
+    if (HEAT) p.tdot[n] = sum[0];
+    if (DVOLDT) p.ntmp[n] = sum[NQ - 1] / p.vol_n[n];
 }
 
 // The fused step's form of the same three functions (update_strain_rate,
@@ -199,21 +204,24 @@ __global__ void __launch_bounds__(TPB) k_elem_pass(KP p, int heat)
     }
 }
 
-template <int ND>
-__global__ void __launch_bounds__(TPB) k_node_pass(KP p, int heat)
+template <int ND, bool STAGED>
+__global__ void __launch_bounds__(128) k_node_pass(KP p, int heat)
 {
-    const int n = p.n_lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.n_hi) return;
     const size_t ne = p.ne;
-    double tdot = 0, dvoldt = 0;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        const int ent = p.sup_ent[q];
-        const int e = ent >> 2, i = ent & 3;
-        if (heat) tdot += p.hc64[(size_t)i * ne + e];
-        dvoldt += p.qv[e];
-    }
-    p.ntmp[n] = dvoldt / p.vol_n[n];
+    double sum[2] = {0, 0};   // dvoldt, tdot
+    const int n = node_sums<SumF64, 2, ND, STAGED>(
+        p.sup_off, p.n_lo, p.n_hi, heat ? 2 : 1,
+        [&](int q, double *t) {
+            const int ent = p.sup_ent[q];
+            const int e = ent >> 2, i = ent & 3;
+            if (heat) t[1] = p.hc64[(size_t)i * ne + e];
+            t[0] = p.qv[e];
+        },
+        FromZero<SumF64>(), sum);
+    if (n < 0) return;
+    p.ntmp[n] = sum[0] / p.vol_n[n];
     if (heat) {   // temperature update + Dirichlet BC (fields.cxx:151-162)
+        const double tdot = sum[1];
         p.tdot[n] = tdot;
         const unsigned flag = p.bcflag[n];
         if (flag & BOUNDZ1) p.T[n] = p.prm.surface_temperature;
@@ -298,28 +306,33 @@ __global__ void __launch_bounds__(TPB) k_update_stress(KP p, int fused)
 // ==================================================================
 // NMD_stress (geometry.cxx:182-236)
 // ==================================================================
-// stored: read the products the fused stress pass formed (KP::pv), the same
-// dw_mul of the same pairs, instead of forming them for each support entry
-template <int ND>
-__global__ void __launch_bounds__(TPB) k_nmd_gather(KP p, int stored)
+// DW (a mixed context): double-word products in a compensated FP32 sum
+// (des_dw.cuh); stored: read the products the fused stress pass formed
+// (KP::pv), the same dw_mul of the same pairs, instead of forming them for
+// each support entry
+template <int ND, bool DW, bool STAGED>
+__global__ void __launch_bounds__(128) k_nmd_gather(KP p, int stored)
 {
-    int n = p.n_lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.n_hi) return;
-    if (ND == 3 && p.shpdw) {   // a mixed context: double-word products, compensated FP32 sum (des_dw.cuh)
-        dw_sum acc;
-        for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-            const int e = p.sup_ent[q] >> 2;
-            acc.add(stored ? dw_of2(p.pv[e]) : dw_mul(dw_split(p.dp[e]), dw_split(p.vol[e])));
-        }
-        p.ntmp[n] = acc.value() / p.vol_n[n];
-        return;
+    double sum;
+    int n;
+    if constexpr (DW) {
+        n = node_sums<SumDw, 1, ND, STAGED>(
+            p.sup_off, p.n_lo, p.n_hi, 1,
+            [&](int q, float2 *t) {
+                const int e = p.sup_ent[q] >> 2;
+                *t = stored ? p.pv[e] : pair_of(dw_mul(dw_split(p.dp[e]), dw_split(p.vol[e])));
+            },
+            FromZero<SumDw>(), &sum);
+    } else {
+        n = node_sums<SumF64, 1, ND, STAGED>(
+            p.sup_off, p.n_lo, p.n_hi, 1,
+            [&](int q, double *t) {
+                const int e = p.sup_ent[q] >> 2;
+                *t = p.dp[e] * p.vol[e];
+            },
+            FromZero<SumF64>(), &sum);
     }
-    double acc = 0;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        int e = p.sup_ent[q] >> 2;
-        acc += p.dp[e] * p.vol[e];
-    }
-    p.ntmp[n] = acc / p.vol_n[n];
+    if (n >= 0) p.ntmp[n] = sum / p.vol_n[n];
 }
 
 // per-facet force of the gravity-induced stress BCs (bc.cxx:493-557);
@@ -530,57 +543,50 @@ __device__ __forceinline__ double madd(double a, double b, double c)
     return C ? fma(a, b, c) : a * b + c;
 }
 
-// CONTRACT: the mixed step's form, with the sums of products fused
-// (1 + 2 instead of 3 + 2 FP64 operations per component, and the update
-// f -= t * vol one fma), and dt f / m as dt f (1/m) with one recip_newton.
-// Rounding moves by an ulp of each force term, far below the FP32 strain
-// rate terms of the same step.
+// CONTRACT: the mixed step's form, with fused multiply-adds, and dt f / m as
+// dt f (1/m) with one recip_newton.
 template <int ND, bool CONTRACT>
 __device__ __forceinline__ void force_tail(const KP &p, int n, double *f, int fused_motion);
 
-template <int ND, bool CONTRACT = false>
-__global__ void __launch_bounds__(TPB) k_force(KP p, int fused_motion)
+// The FP64 step's force: each support entry's term -(sigma . dN_i/dx + rho g
+// / NPE z) vol, the expression the reference subtracts; then the FP64 tail.
+template <int ND, bool STAGED>
+__global__ void __launch_bounds__(128) k_force(KP p, int fused_motion)
 {
     constexpr int NSTR = ND * (ND + 1) / 2;
     constexpr int NPE = ND + 1;
-    int n = p.n_lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.n_hi) return;
     const size_t ne = p.ne;
     const double gravity = p.prm.gravity;
     double f[ND];
+    const int n = node_sums<SumF64, ND, ND, STAGED>(
+        p.sup_off, p.n_lo, p.n_hi, ND,
+        [&](int q, double *t) {
+            const int ent = p.sup_ent[q];
+            const int e = ent >> 2, i = ent & 3;
+            double s[NSTR];
 #pragma unroll
-    for (int d = 0; d < ND; ++d) f[d] = 0;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        int ent = p.sup_ent[q];
-        int e = ent >> 2, i = ent & 3;
-        double s[NSTR];
-#pragma unroll
-        for (int c = 0; c < NSTR; ++c) s[c] = p.stress[c * ne + e];
-        double vol = p.vol[e];
-        double buoy = 0;
-        if (p.buoy_e) {
-            buoy = p.buoy_e[e];
-        } else if (gravity != 0) {
-            double rho = p.rho_e ? p.rho_e[e] : m_rho<ND>(p, e);
-            buoy = rho * gravity / NPE;
-        }
-        double sx = shp_at(p, 0, i, e), sz = shp_at(p, ND - 1, i, e);
-        // f -= (sum of products) * vol, written as madd(-t, vol, f): the same
-        // bits as the reference's expression when not contracted
-        if (ND == 3) {
-            double sy = shp_at(p, 1, i, e);
-            f[0] = madd<CONTRACT>(-madd<CONTRACT>(s[4], sz, madd<CONTRACT>(s[3], sy, s[0] * sx)), vol, f[0]);
-            f[1] = madd<CONTRACT>(-madd<CONTRACT>(s[5], sz, madd<CONTRACT>(s[1], sy, s[3] * sx)), vol, f[1]);
-            const double tz = CONTRACT ? fma(s[2], sz, fma(s[5], sy, fma(s[4], sx, buoy)))
-                                       : madd<false>(s[2], sz, madd<false>(s[5], sy, s[4] * sx)) + buoy;
-            f[ND - 1] = madd<CONTRACT>(-tz, vol, f[ND - 1]);
-        } else {
-            f[0] = madd<CONTRACT>(-madd<CONTRACT>(s[2], sz, s[0] * sx), vol, f[0]);
-            const double tz = CONTRACT ? fma(s[1], sz, fma(s[2], sx, buoy)) : madd<false>(s[1], sz, s[2] * sx) + buoy;
-            f[ND - 1] = madd<CONTRACT>(-tz, vol, f[ND - 1]);
-        }
-    }
-    force_tail<ND, CONTRACT>(p, n, f, fused_motion);
+            for (int c = 0; c < NSTR; ++c) s[c] = p.stress[c * ne + e];
+            const double vol = p.vol[e];
+            double buoy = 0;
+            if (p.buoy_e) {
+                buoy = p.buoy_e[e];
+            } else if (gravity != 0) {
+                const double rho = p.rho_e ? p.rho_e[e] : m_rho<ND>(p, e);
+                buoy = rho * gravity / NPE;
+            }
+            const double sx = shp_at(p, 0, i, e), sz = shp_at(p, ND - 1, i, e);
+            if (ND == 3) {
+                const double sy = shp_at(p, 1, i, e);
+                t[0] = -(s[0] * sx + s[3] * sy + s[4] * sz) * vol;
+                t[1] = -(s[3] * sx + s[1] * sy + s[5] * sz) * vol;
+                t[ND - 1] = -(s[4] * sx + s[5] * sy + s[2] * sz + buoy) * vol;
+            } else {
+                t[0] = -(s[0] * sx + s[2] * sz) * vol;
+                t[ND - 1] = -(s[2] * sx + s[1] * sz + buoy) * vol;
+            }
+        },
+        FromZero<SumF64>(), f);
+    if (n >= 0) force_tail<ND, false>(p, n, f, fused_motion);
 }
 
 // k_force after its element gather: the gravity-induced stress BCs, the
@@ -642,22 +648,30 @@ __device__ __forceinline__ void force_tail(const KP &p, int n, double *f, int fu
 // double-word arithmetic -- whose sums are accurate relative to the exact
 // sum (Algorithm 6 of des_dw.cuh), however much the elements' terms cancel
 // -- and rounds the sum to FP64 once; the rest is k_force's FP64 tail.
-__global__ void __launch_bounds__(TPB) k_force_dw3(KP p, int fused_motion)
-{
-    const int n = p.n_lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.n_hi) return;
-    dw a0{0.0f, 0.0f}, a1{0.0f, 0.0f}, a2{0.0f, 0.0f};
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        const float4 h = __ldg(p.ft + 2 * (size_t)q), l = __ldg(p.ft + 2 * (size_t)q + 1);
-        a0 = dw_add(a0, {h.x, l.x});
-        a1 = dw_add(a1, {h.y, l.y});
-        a2 = dw_add(a2, {h.z, l.z});
+struct ForceTerms {   // the three components' terms of a support entry
+    const float4 *ft;
+    __device__ __forceinline__ void operator()(int q, float2 *t) const
+    {
+        const float4 h = __ldg(ft + 2 * (size_t)q), l = __ldg(ft + 2 * (size_t)q + 1);
+        t[0] = make_float2(h.x, l.x);
+        t[1] = make_float2(h.y, l.y);
+        t[2] = make_float2(h.z, l.z);
     }
-    double f[3] = {-f64_of(a0), -f64_of(a1), -f64_of(a2)};
+};
+
+template <bool STAGED>
+__global__ void __launch_bounds__(128) k_force_dw3(KP p, int fused_motion)
+{
+    double f[3];
+    const int n = node_sums<SumDwAcc, 3, 3, STAGED>(p.sup_off, p.n_lo, p.n_hi, 3, ForceTerms{p.ft},
+                                                    FromZero<SumDwAcc>(), f);
+    if (n < 0) return;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) f[d] = -f[d];
     force_tail<3, true>(p, n, f, fused_motion);
 }
 
-// CONTRACT: the form of k_force<ND, true>'s fused velocity update
+// CONTRACT: the form of the mixed step's fused velocity update
 template <int ND, bool CONTRACT = false>
 __global__ void __launch_bounds__(TPB) k_velocity(KP p)
 {
@@ -1142,76 +1156,66 @@ __global__ void k_dt_reset(KP p)
 // ==================================================================
 // compute_mass (geometry.cxx:313-365)
 // ==================================================================
-template <int ND>
-__global__ void __launch_bounds__(TPB) k_mass(KP p)
+// The node sums of compute_mass: volume_n, mass and, with heat, tmass.  DW (a
+// mixed context): compensated FP32 sums (des_dw.cuh).  terms(e, t) gives an
+// element's three terms.
+template <int ND, bool DW, bool STAGED, class Terms>
+__device__ __forceinline__ void mass_sums(const KP &p, int lo, int hi, Terms terms)
+{
+    const bool thermal = p.prm.has_thermal_diffusion;
+    double sum[3] = {0, 0, 0};
+    int n;
+    if constexpr (DW) {
+        n = node_sums<SumDw, 3, ND, STAGED>(
+            p.sup_off, lo, hi, thermal ? 3 : 2,
+            [&](int q, float2 *t) {
+                double d[3];
+                terms(p.sup_ent[q] >> 2, d);
+                t[0] = pair_of(dw_split(d[0]));
+                t[1] = pair_of(dw_split(d[1]));
+                if (thermal) t[2] = pair_of(dw_split(d[2]));
+            },
+            FromZero<SumDw>(), sum);
+    } else {
+        n = node_sums<SumF64, 3, ND, STAGED>(
+            p.sup_off, lo, hi, thermal ? 3 : 2, [&](int q, double *t) { terms(p.sup_ent[q] >> 2, t); },
+            FromZero<SumF64>(), sum);
+    }
+    if (n < 0) return;
+    p.vol_n[n] = sum[0];
+    p.mass[n] = sum[1];
+    p.tmass[n] = thermal ? sum[2] : 0.0;
+}
+
+template <int ND, bool DW, bool STAGED>
+__global__ void __launch_bounds__(128) k_mass(KP p)
 {
     constexpr int NPE = ND + 1;
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.nn) return;
     const double pseudo_speed = p.prm.max_vbc_val * p.prm.inertial_scaling;
     const bool quasi = p.prm.is_quasi_static, thermal = p.prm.has_thermal_diffusion;
-    const bool cs = ND == 3 && p.shpdw;   // a mixed context: compensated FP32 sums, as k_mass_sum's
-    double vn = 0, ms = 0, tm = 0;
-    dw_sum vs, mss, tms;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        int e = p.sup_ent[q] >> 2;
-        double vol = p.vol[e];
-        double rho_e = p.rho_e ? p.rho_e[e] : m_rho<ND>(p, e);
-        double rho = quasi ? ((p.mat.nmat == 1) ? p.mat.rho_pseudo : m_bulkm(p, e) / (pseudo_speed * pseudo_speed))
-                           : rho_e;
-        double m = rho * vol / NPE;
-        double tme = thermal ? rho_e * m_cp(p, e) * vol / NPE : 0.0;
-        if (cs) {
-            vs.add(dw_split(vol));
-            mss.add(dw_split(m));
-            if (thermal) tms.add(dw_split(tme));
-        } else {
-            vn += vol;
-            ms += m;
-            if (thermal) tm += tme;
-        }
-    }
-    if (cs) {
-        vn = vs.value();
-        ms = mss.value();
-        tm = tms.value();
-    }
-    p.vol_n[n] = vn;
-    p.mass[n] = ms;
-    p.tmass[n] = tm;
+    mass_sums<ND, DW, STAGED>(p, 0, p.nn, [&](int e, double *t) {
+        const double vol = p.vol[e];
+        const double rho_e = p.rho_e ? p.rho_e[e] : m_rho<ND>(p, e);
+        const double rho = quasi
+            ? ((p.mat.nmat == 1) ? p.mat.rho_pseudo : m_bulkm(p, e) / (pseudo_speed * pseudo_speed))
+            : rho_e;
+        t[0] = vol;
+        t[1] = rho * vol / NPE;
+        t[2] = thermal ? rho_e * m_cp(p, e) * vol / NPE : 0.0;
+    });
 }
 
 // the node sums of compute_mass from the element terms that the geometry
 // pass wrote (GEO_MASS_TERMS): per pair 3 additions instead of the terms
-template <int ND>
-__global__ void __launch_bounds__(TPB) k_mass_sum(KP p)
+template <int ND, bool DW, bool STAGED>
+__global__ void __launch_bounds__(128) k_mass_sum(KP p)
 {
-    int n = p.n_lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.n_hi) return;
     const bool thermal = p.prm.has_thermal_diffusion;
-    if (ND == 3 && p.shpdw) {   // a mixed context: compensated FP32 sums (des_dw.cuh), as k_mass's
-        dw_sum vs, mss, tms;
-        for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-            const int e = p.sup_ent[q] >> 2;
-            vs.add(dw_split(p.vol[e]));
-            mss.add(dw_split(p.me[e]));
-            if (thermal) tms.add(dw_split(p.tme[e]));
-        }
-        p.vol_n[n] = vs.value();
-        p.mass[n] = mss.value();
-        p.tmass[n] = thermal ? tms.value() : 0.0;
-        return;
-    }
-    double vn = 0, ms = 0, tm = 0;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        int e = p.sup_ent[q] >> 2;
-        vn += p.vol[e];
-        ms += p.me[e];
-        if (thermal) tm += p.tme[e];
-    }
-    p.vol_n[n] = vn;
-    p.mass[n] = ms;
-    p.tmass[n] = tm;
+    mass_sums<ND, DW, STAGED>(p, p.n_lo, p.n_hi, [&](int e, double *t) {
+        t[0] = p.vol[e];
+        t[1] = p.me[e];
+        t[2] = thermal ? p.tme[e] : 0.0;
+    });
 }
 
 // ==================================================================
@@ -1427,15 +1431,15 @@ int launch_strain_rate(const KP &p, cudaStream_t s, bool begin_step)
 
 int launch_heat_gather(const KP &p, cudaStream_t s)
 {
-    if (p.nd == 3) DES_LAUNCH((k_node_gather1<3, true, false>), p.nn, s, p);
-    else DES_LAUNCH((k_node_gather1<2, true, false>), p.nn, s, p);
+    if (p.nd == 3) DES_NODES((k_node_gather1<3, true, false, STAGED>), p.nn, s, p);
+    else DES_NODES((k_node_gather1<2, true, false, STAGED>), p.nn, s, p);
     return 1;
 }
 
 int launch_dvoldt(const KP &p, cudaStream_t s)
 {
-    if (p.nd == 3) DES_LAUNCH((k_node_gather1<3, false, true>), p.nn, s, p);
-    else DES_LAUNCH((k_node_gather1<2, false, true>), p.nn, s, p);
+    if (p.nd == 3) DES_NODES((k_node_gather1<3, false, true, STAGED>), p.nn, s, p);
+    else DES_NODES((k_node_gather1<2, false, true, STAGED>), p.nn, s, p);
     return 1;
 }
 
@@ -1447,14 +1451,8 @@ int launch_elem_pass(const KP &p, cudaStream_t s, bool heat)
 
 int launch_node_pass(const KP &p, cudaStream_t s, bool heat)
 {
-    DISPATCH(k_node_pass, p.n_hi - p.n_lo, p, (int)heat);
-    return 1;
-}
-
-int launch_heat_and_dvoldt(const KP &p, cudaStream_t s)
-{
-    if (p.nd == 3) DES_LAUNCH((k_node_gather1<3, true, true>), p.nn, s, p);
-    else DES_LAUNCH((k_node_gather1<2, true, true>), p.nn, s, p);
+    if (p.nd == 3) DES_NODES((k_node_pass<3, STAGED>), p.n_hi - p.n_lo, s, p, (int)heat);
+    else DES_NODES((k_node_pass<2, STAGED>), p.n_hi - p.n_lo, s, p, (int)heat);
     return 1;
 }
 
@@ -1478,7 +1476,10 @@ int launch_update_stress(const KP &p, cudaStream_t s, bool fused)
 
 int launch_nmd_gather(const KP &p, cudaStream_t s, bool stored)
 {
-    DISPATCH(k_nmd_gather, p.n_hi - p.n_lo, p, (int)(stored && p.pv));
+    const int n = p.n_hi - p.n_lo;
+    if (p.nd == 3 && p.shpdw) DES_NODES((k_nmd_gather<3, true, STAGED>), n, s, p, (int)(stored && p.pv));
+    else if (p.nd == 3) DES_NODES((k_nmd_gather<3, false, STAGED>), n, s, p, 0);
+    else DES_NODES((k_nmd_gather<2, false, STAGED>), n, s, p, 0);
     return 1;
 }
 
@@ -1509,16 +1510,10 @@ int launch_facet_forces(const KP &p, cudaStream_t s)
 
 int launch_force(const KP &p, cudaStream_t s, bool fused_motion, bool contract)
 {
-    if (contract && uses_force_terms(p)) {
-        DES_LAUNCH(k_force_dw3, p.n_hi - p.n_lo, s, p, (int)fused_motion);
-        return 1;
-    }
-    if (contract) {
-        if (p.nd == 3) DES_LAUNCH((k_force<3, true>), p.n_hi - p.n_lo, s, p, (int)fused_motion);
-        else DES_LAUNCH((k_force<2, true>), p.n_hi - p.n_lo, s, p, (int)fused_motion);
-        return 1;
-    }
-    DISPATCH(k_force, p.n_hi - p.n_lo, p, (int)fused_motion);
+    const int n = p.n_hi - p.n_lo;
+    if (contract && uses_force_terms(p)) DES_NODES(k_force_dw3<STAGED>, n, s, p, (int)fused_motion);
+    else if (p.nd == 3) DES_NODES((k_force<3, STAGED>), n, s, p, (int)fused_motion);
+    else DES_NODES((k_force<2, STAGED>), n, s, p, (int)fused_motion);
     return 1;
 }
 
@@ -1566,13 +1561,18 @@ int launch_geometry_ahead(const KP &p, cudaStream_t s, int flags)
 
 int launch_mass(const KP &p, cudaStream_t s)
 {
-    DISPATCH(k_mass, p.nn, p);
+    if (p.nd == 3 && p.shpdw) DES_NODES((k_mass<3, true, STAGED>), p.nn, s, p);
+    else if (p.nd == 3) DES_NODES((k_mass<3, false, STAGED>), p.nn, s, p);
+    else DES_NODES((k_mass<2, false, STAGED>), p.nn, s, p);
     return 1;
 }
 
 int launch_mass_sum(const KP &p, cudaStream_t s)
 {
-    DISPATCH(k_mass_sum, p.n_hi - p.n_lo, p);
+    const int n = p.n_hi - p.n_lo;
+    if (p.nd == 3 && p.shpdw) DES_NODES((k_mass_sum<3, true, STAGED>), n, s, p);
+    else if (p.nd == 3) DES_NODES((k_mass_sum<3, false, STAGED>), n, s, p);
+    else DES_NODES((k_mass_sum<2, false, STAGED>), n, s, p);
     return 1;
 }
 

@@ -51,7 +51,6 @@ int launch_strain_rate(const KP &p, cudaStream_t s, bool begin_step);
 int launch_heat_gather(const KP &p, cudaStream_t s);              // tdot -> p.tdot
 int launch_temperature_update(const KP &p, cudaStream_t s);       // T from p.tdot
 int launch_dvoldt(const KP &p, cudaStream_t s);                   // -> ntmp
-int launch_heat_and_dvoldt(const KP &p, cudaStream_t s);          // fused: tdot -> p.tdot, dvoldt -> ntmp
 // the FP64 step's element-centric form of strain rate + heat gather + dvoldt
 // (+ clock advance) and of the node sums + temperature update: the same bits
 // (needs p.qv and, with heat, p.hc64)

@@ -24,10 +24,13 @@
 // only scales the force), and in FP32 they alone moved the stress by 4e-6
 // (relative L2) after 2000 steps of the 998,400-tet workload.
 // Element volumes, shape functions, forces and masses stay FP64.
+#include <algorithm>
+
 #include "des_kernels.cuh"
 #include "des_rheology.cuh"
 #include "des_mixed.cuh"
 #include "des_dw.cuh"
+#include "des_gather.cuh"
 #include "des_mixed_elem.cuh"
 
 namespace des {
@@ -37,12 +40,6 @@ constexpr int TPB_M = 256;
 __device__ __forceinline__ float shp32_at(const KP &p, int k, int i, int e)
 {
     return p.shpdw[((size_t)k * 4 + i) * p.ne + e].x;   // the pair's high part: the nearest float
-}
-
-static inline int nblocks_m(long long n)
-{
-    long long b = (n + TPB_M - 1) / TPB_M;
-    return (int)(b < 1 ? 1 : b);
 }
 
 // exp(x) for |x| < 690 as 2^k exp(r): any integer k near x / ln 2 keeps |r|
@@ -520,40 +517,62 @@ __global__ void __launch_bounds__(TPB_M) k_strain_rate_mixed3(KP p, int begin_st
 // heat stencil on FP64 temperature differences (sum_j D_ij = 0), FP32
 // products, a compensated FP32 nodal sum of the heat terms; dvoldt in FP64
 // (fields.cxx:99-146, geometry.cxx:111-155)
-__global__ void __launch_bounds__(TPB_M) k_heat_dvoldt_mixed3(KP p, int heat, int do_dvoldt)
-{
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.nn) return;
-    const double Tn = p.T[n];
-    const bool k_const = (p.mat.nmat == 1) && !p.ef[DES_EF_THERM_COND];
-    dw_sum tsum;   // a compensated FP32 sum of the heat terms (des_dw.cuh)
-    double dvoldt = 0;
-    for (int q = p.sup_off[n]; q < p.sup_off[n + 1]; ++q) {
-        const int ent = p.sup_ent[q];
-        const int e = ent >> 2, i = ent & 3;
-        const double vol = p.vol[e];
-        if (heat) {
-            const float sxi = shp32_at(p, 0, i, e), syi = shp32_at(p, 1, i, e), szi = shp32_at(p, 2, i, e);
-            float diffusion = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (j == i) continue;
-                const float D = sxi * shp32_at(p, 0, j, e) + syi * shp32_at(p, 1, j, e)
-                    + szi * shp32_at(p, 2, j, e);
-                diffusion += D * f32_of(p.T[conn_at(p, j, e)] - Tn);
-            }
-            const float volf = f32_of(vol);
-            const float kv = f32_of(k_const ? p.mat.therm_cond[0] : m_k(p, e)) * volf;
-            const float rh = f32_of(m_hr_over_cp(p, e)) * volf;
-            tsum.add(kv * diffusion - rh);
-        }
-        if (do_dvoldt) {
-            const double dj = p.srate[e] + p.srate[(size_t)p.ne + e] + p.srate[2 * (size_t)p.ne + e];
-            dvoldt += dj * vol;
-        }
+// dvoldt (quantity 0) in FP64, the others in compensated FP32 sums
+struct SumNode {
+    using Term = double;   // the pairs travel as the FP64 value's two words
+    struct State {
+        double d = 0;
+        dw_sum w;
+    };
+    static __device__ __forceinline__ Term pack(dw w)
+    {
+        return __hiloint2double(__float_as_int(w.hi), __float_as_int(w.lo));
     }
-    if (heat) p.tdot[n] = tsum.value();
-    if (do_dvoldt) p.ntmp[n] = dvoldt / p.vol_n[n];
+    static __device__ __forceinline__ void add(int c, State &s, Term t)
+    {
+        if (c == 0) s.d += t;
+        else s.w.add(dw{__int_as_float(__double2hiint(t)), __int_as_float(__double2loint(t))});
+    }
+    static __device__ __forceinline__ double value(int c, const State &s) { return c == 0 ? s.d : s.w.value(); }
+};
+
+template <bool STAGED>
+__global__ void __launch_bounds__(128) k_heat_dvoldt_mixed3(KP p, int heat, int do_dvoldt)
+{
+    const bool k_const = (p.mat.nmat == 1) && !p.ef[DES_EF_THERM_COND];
+    double sum[2] = {0, 0};   // dvoldt, tdot
+    const int n = node_sums<SumNode, 2, 3, STAGED>(
+        p.sup_off, 0, p.nn, heat ? 2 : 1,
+        [&](int q, double *t) {
+            const int ent = p.sup_ent[q];
+            const int e = ent >> 2, i = ent & 3;
+            const double vol = p.vol[e];
+            if (heat) {
+                const double Tn = p.T[conn_at(p, i, e)];
+                const float sxi = shp32_at(p, 0, i, e), syi = shp32_at(p, 1, i, e), szi = shp32_at(p, 2, i, e);
+                float diffusion = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (j == i) continue;
+                    const float D = sxi * shp32_at(p, 0, j, e) + syi * shp32_at(p, 1, j, e)
+                        + szi * shp32_at(p, 2, j, e);
+                    diffusion += D * f32_of(p.T[conn_at(p, j, e)] - Tn);
+                }
+                const float volf = f32_of(vol);
+                const float kv = f32_of(k_const ? p.mat.therm_cond[0] : m_k(p, e)) * volf;
+                const float rh = f32_of(m_hr_over_cp(p, e)) * volf;
+                t[1] = SumNode::pack(dw{kv * diffusion - rh, 0.0f});
+            }
+            t[0] = 0;
+            if (do_dvoldt) {
+                const double dj = p.srate[e] + p.srate[(size_t)p.ne + e] + p.srate[2 * (size_t)p.ne + e];
+                t[0] = dj * vol;
+            }
+        },
+        FromZero<SumNode>(), sum);
+    if (n < 0) return;
+    if (heat) p.tdot[n] = sum[1];
+    if (do_dvoldt) p.ntmp[n] = sum[0] / p.vol_n[n];
 }
 
 // ------------------------------------------------------------------
@@ -592,61 +611,57 @@ __global__ void __launch_bounds__(TPB_M) k_elem_pass_mixed3(KP p, int heat)
 // geometry pass wrote (KP::ndpk), as k_mass_sum forms them, and (begin_step) starts the
 // step's clock, which the look-ahead pass could not: the step's dt is final
 // only after k_dt_finalize.
-__global__ void __launch_bounds__(TPB_M) k_node_pass_mixed3(KP p, int heat, int mass_sums, int begin_step)
+// The heat terms go into a compensated FP32 sum (des_dw.cuh), as
+// k_heat_dvoldt_mixed3 sums them; the dvoldt terms into an FP64 one: they
+// cancel between a node's elements, and the 2^-47 of a double-word split of
+// each moved the volumetric rate enough to change the default damping's
+// copysign at some nodes within ten steps.
+template <bool MASS, bool STAGED>
+__global__ void __launch_bounds__(128) k_node_pass_mixed3(KP p, int heat, int begin_step)
 {
     if (begin_step && blockIdx.x == 0 && threadIdx.x == 0) {   // dynearthsol.cxx:325-326
         p.clk->steps += 1;
         p.clk->time += p.clk->dt;
     }
-    int n = p.n_lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.n_hi) return;
+    constexpr int NQ = MASS ? 5 : 2;
     const size_t ne = p.ne;
-    const int q0 = p.sup_off[n], q1 = p.sup_off[n + 1];
-    double vol_n, tmass = 0;
-    // the heat terms in a compensated FP32 sum (des_dw.cuh), as
-    // k_heat_dvoldt_mixed3 sums them; the dvoldt terms in FP64: they cancel
-    // between a node's elements, and the 2^-47 of a double-word split of
-    // each moved the volumetric rate enough to change the default damping's
-    // copysign at some nodes within ten steps
-    dw_sum tsum;
-    double dvoldt = 0;
-    if (mass_sums) {
-        // one pass over the support: the mass sums in compensated FP32
-        // (des_dw.cuh), as k_mass_sum's, from the look-ahead pass's records
-        const bool thermal = p.prm.has_thermal_diffusion;
-        dw_sum vs, mss, tms;
-        for (int q = q0; q < q1; ++q) {
+    const bool thermal = p.prm.has_thermal_diffusion;
+    double sum[NQ] = {};   // dvoldt, tdot, volume_n, mass, tmass
+    const int n = node_sums<SumNode, NQ, 3, STAGED>(
+        p.sup_off, p.n_lo, p.n_hi, NQ,
+        [&](int q, double *t) {
             const int ent = p.sup_ent[q];
             const int e = ent >> 2, i = ent & 3;
-            const double4 r = p.ndpk[e];   // qv, vol, me, tme
-            vs.add(dw_split(r.y));
-            mss.add(dw_split(r.z));
-            if (thermal) tms.add(dw_split(r.w));
-            if (heat) tsum.add(p.hc[(size_t)i * ne + e]);
-            dvoldt += r.x;
-        }
-        vol_n = vs.value();
-        tmass = thermal ? tms.value() : 0.0;
+            if constexpr (MASS) {
+                const double4 r = p.ndpk[e];   // qv, vol, me, tme
+                t[0] = r.x;
+                t[2] = SumNode::pack(dw_split(r.y));
+                t[3] = SumNode::pack(dw_split(r.z));
+                t[4] = thermal ? SumNode::pack(dw_split(r.w)) : 0.0;
+            } else {
+                t[0] = p.qv[e];
+            }
+            t[1] = heat ? SumNode::pack(dw{p.hc[(size_t)i * ne + e], 0.0f}) : 0.0;
+        },
+        FromZero<SumNode>(), sum);
+    if (n < 0) return;
+    double vol_n, tmass = 0;
+    if constexpr (MASS) {
+        vol_n = sum[2];
+        tmass = thermal ? sum[4] : 0.0;
         p.vol_n[n] = vol_n;
-        p.mass[n] = mss.value();
+        p.mass[n] = sum[3];
         p.tmass[n] = tmass;
     } else {
         vol_n = p.vol_n[n];
         if (heat) tmass = p.tmass[n];
-        for (int q = q0; q < q1; ++q) {
-            const int ent = p.sup_ent[q];
-            const int e = ent >> 2, i = ent & 3;
-            if (heat) tsum.add(p.hc[(size_t)i * ne + e]);
-            dvoldt += p.qv[e];
-        }
     }
-    const double tdot = tsum.value();
-    p.ntmp[n] = dvoldt / vol_n;
+    p.ntmp[n] = sum[0] / vol_n;
     if (heat) {   // temperature update + Dirichlet BC (fields.cxx:151-162)
         const unsigned flag = p.bcflag[n];
         if (flag & BOUNDZ1) p.T[n] = p.prm.surface_temperature;
         else if ((flag & BOUNDZ0) && !p.prm.has_fixed_bottom_temperature) p.T[n] = p.prm.mantle_temperature;
-        else p.T[n] -= tdot * p.clk->dt / tmass;
+        else p.T[n] -= sum[1] * p.clk->dt / tmass;
     }
 }
 
@@ -664,7 +679,7 @@ int launch_strain_rate_mixed(const KP &p, cudaStream_t s, bool begin_step)
 
 int launch_heat_and_dvoldt_mixed(const KP &p, cudaStream_t s, bool heat, bool dvoldt)
 {
-    DES_LAUNCH(k_heat_dvoldt_mixed3, p.nn, s, p, (int)heat, (int)dvoldt);
+    DES_NODES(k_heat_dvoldt_mixed3<STAGED>, p.nn, s, p, (int)heat, (int)dvoldt);
     return 1;
 }
 
@@ -678,7 +693,9 @@ int launch_elem_pass_mixed(const KP &p, cudaStream_t s, bool heat)
 
 int launch_node_pass_mixed(const KP &p, cudaStream_t s, bool heat, bool mass_sums, bool begin_step)
 {
-    DES_LAUNCH(k_node_pass_mixed3, p.n_hi - p.n_lo, s, p, (int)heat, (int)mass_sums, (int)begin_step);
+    const int n = p.n_hi - p.n_lo;
+    if (mass_sums) DES_NODES((k_node_pass_mixed3<true, STAGED>), n, s, p, (int)heat, (int)begin_step);
+    else DES_NODES((k_node_pass_mixed3<false, STAGED>), n, s, p, (int)heat, (int)begin_step);
     return 1;
 }
 
