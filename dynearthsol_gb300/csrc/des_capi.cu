@@ -576,6 +576,12 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
                 p.mat.pt_coh_over_tan[2 * m + 1] = p.mat.cohesion1[m] / p.mat.pt_tanphi[2 * m + 1];
                 p.mat.hardening[m] = (p.mat.cohesion1[m] - p.mat.cohesion0[m]) / (p.mat.pls1[m] - p.mat.pls0[m]);
             }
+            for (int k = 0; k < 2 * nm; ++k) {
+                p.mat.pt_anphi_f[k] = (float)p.mat.pt_anphi[k];
+                p.mat.pt_sqrt_anphi_f[k] = (float)p.mat.pt_sqrt_anphi[k];
+                p.mat.pt_tanphi_f[k] = p.mat.pt_phi[k] == 0 ? 0.0f : (float)p.mat.pt_tanphi[k];
+            }
+            p.mat.tension_max_f = (float)p.mat.tension_max;
             p.mat.pt_n = 2 * nm;
         }
     }
@@ -1291,7 +1297,7 @@ int enqueue_step_mixed_chain(des_ctx *c, int part)
     const bool thermal = p.prm.has_thermal_diffusion != 0;
     if (part == 0) n += launch_elem_pass_mixed(p, s, thermal);
     n += launch_node_pass_mixed(p, s, thermal, part != 0, part != 0);
-    n += launch_update_stress_mixed(p, s, true);
+    n += launch_update_stress_mixed(p, s, true, part == 2);
     n += launch_nmd_gather(p, s, true);
     n += launch_nmd_correct(p, s, true);
     n += launch_force(p, s, true, true);

@@ -81,6 +81,10 @@ struct MatC {
     double pt_sqrt_anphi[2 * DES_MAXMAT], pt_tanphi[2 * DES_MAXMAT];
     double pt_coh_over_tan[2 * DES_MAXMAT];   // cohesion0 / tan(phi0), cohesion1 / tan(phi1)
     double hardening[DES_MAXMAT];             // (cohesion1 - cohesion0) / (pls1 - pls0)
+    // FP32 roundings for the mixed step's yield screen (tan 0 where phi is 0:
+    // the quotient by it then leaves tension_max)
+    float pt_anphi_f[2 * DES_MAXMAT], pt_sqrt_anphi_f[2 * DES_MAXMAT], pt_tanphi_f[2 * DES_MAXMAT];
+    float tension_max_f;
 };
 
 // Everything a kernel needs, passed by value.
@@ -541,6 +545,76 @@ __device__ __forceinline__ void m_plastic_props(const KP &p, int e, double pls, 
         plastic_props_one(p, e, 0, pls, amc, anphi, anpsi, hardn, ten_max);
     else
         plastic_props_blend(p, e, pls, amc, anphi, anpsi, hardn, ten_max);
+}
+
+// FP32 values of plastic_props' anphi, amc and ten_max for the mixed step's
+// yield screen, within a relative err of the FP32 roundings of the FP64 ones
+// (0: they are those roundings).  The FP64 properties cost a division where
+// the cohesion is the element's own and ~180 FP64 operations where it softens
+// (two sines, a tangent, a square root and divisions per element and step);
+// only an element that reaches the return map needs them.
+struct ScreenTerms {
+    float af, cf, tf, err;
+};
+
+// An element whose markers are all of material m and number one, with the
+// material's own friction angles, outside the softening range: the table's
+// angle terms (MatC) and one product or quotient of the cohesion, a few ulps.
+__device__ __forceinline__ ScreenTerms screen_terms_table(const KP &p, int e, int m, double pls)
+{
+    const int k = (pls < p.mat.pls0[m] || pls == p.mat.pls0[m]) ? 2 * m : 2 * m + 1;
+    const double *ef = p.ef[(k & 1) ? DES_EF_COHESION1 : DES_EF_COHESION0];
+    const float c = f32_of(ef ? ef[e] : (k & 1) ? p.mat.cohesion1[m] : p.mat.cohesion0[m]);
+    return {p.mat.pt_anphi_f[k], 2.0f * c * p.mat.pt_sqrt_anphi_f[k],
+            fminf(p.mat.tension_max_f, c / p.mat.pt_tanphi_f[k]), 0x1p-17f};
+}
+
+// Any element.  Where it softens (pls0 < plstrain < pls1), holds one marker,
+// has angles up to 60 degrees and end values of cohesion and angle within a
+// factor 16, the properties are formed in FP32: an interpolation c is then
+// off by at most 3 * 2^-24 * 16 = 2.9e-6 of itself (its end values' size over
+// its own), tan(phi) by the angle's absolute error over sin cos, also below
+// 16 * 3 * 2^-24, and anphi by twice that absolute error (1.9e-7) over cos^2
+// >= 1/4, 1.5e-6; with the FP32 functions' few ulps, all below 2^-17.
+// Otherwise they are the FP64 properties, rounded.
+static __device__ __noinline__ ScreenTerms screen_terms_any(const KP &p, int e, double pls)
+{
+    if (!p.ef[DES_EF_FRICTION0] && !p.ef[DES_EF_FRICTION1]) {
+        int n = 1, m = 0;
+        if (p.emark) {
+            n = 0;
+            for (int k = 0; k < p.mat.nmat; k++) {
+                const int c = mcount(p, e, k);
+                n += c;
+                if (c) m = k;
+            }
+        }
+        const double l0 = p.mat.pls0[m], l1 = p.mat.pls1[m];
+        if (n == 1 && !(pls > l0 && pls < l1)) return screen_terms_table(p, e, m, pls);
+        if (n == 1) {
+            const float q = f32_of(pls - l0) / f32_of(l1 - l0);
+            const double *e0 = p.ef[DES_EF_COHESION0], *e1 = p.ef[DES_EF_COHESION1];
+            const float c0 = f32_of(e0 ? e0[e] : p.mat.cohesion0[m]), c1 = f32_of(e1 ? e1[e] : p.mat.cohesion1[m]);
+            const float f0 = f32_of(p.mat.friction_angle0[m]), f1 = f32_of(p.mat.friction_angle1[m]);
+            if (fminf(c0, c1) > 0.0f && fmaxf(c0, c1) <= 16.0f * fminf(c0, c1) && fminf(f0, f1) > 0.0f
+                && fmaxf(f0, f1) <= fminf(16.0f * fminf(f0, f1), 60.0f)) {
+                const float c = c0 + q * (c1 - c0), rad = (f0 + q * (f1 - f0)) * 0.017453292519943295f;
+                const float sp = sinf(rad), af = (1.0f + sp) / (1.0f - sp);
+                return {af, 2.0f * c * sqrtf(af), fminf(p.mat.tension_max_f, c / tanf(rad)), 0x1p-17f};
+            }
+        }
+    }
+    double amc, anphi, anpsi, hardn, ten_max;
+    m_plastic_props(p, e, pls, amc, anphi, anpsi, hardn, ten_max);
+    return {f32_of(anphi), f32_of(amc), f32_of(ten_max), 0.0f};
+}
+
+__device__ __forceinline__ ScreenTerms screen_terms(const KP &p, int e, double pls)
+{
+    if (p.mat.nmat == 1 && !p.emark && !p.ef[DES_EF_FRICTION0] && !p.ef[DES_EF_FRICTION1]
+        && !(pls > p.mat.pls0[0] && pls < p.mat.pls1[0]))
+        return screen_terms_table(p, e, 0, pls);
+    return screen_terms_any(p, e, pls);
 }
 
 // ref_pressure option 0 (matprops.cxx:190-202)

@@ -197,17 +197,6 @@ __device__ __forceinline__ void elastic_mixed(double bulkm, double shearm, const
 // state's own precision: 6 FP64 additions per candidate instead of the 16
 // FP64 operations of the FP64-coefficient update.
 // ------------------------------------------------------------------
-struct MaxwellF {
-    float c1, f2;
-};
-
-__device__ __forceinline__ MaxwellF maxwell_coef_f(double shearm, double viscosity, double dt)
-{
-    const float tf = (0.5f * f32_of(dt) * f32_of(shearm)) / f32_of(viscosity);
-    const float f2 = 1.0f / (1.0f + tf);
-    return {-2.0f * tf * f2, f2};
-}
-
 // relative volume change vol / vol_old - 1 in FP32 from the FP64 difference
 // (exact for volumes within a factor 2 of each other)
 __device__ __forceinline__ float dvol_f(const KP &p, int e)
@@ -287,95 +276,311 @@ __device__ __forceinline__ double dvol_mixed(const KP &p, int e)
     return (p.vol[e] - vo) * recip_newton(vo);
 }
 
+// The element's strain rate with the anti-locking correction of its normal
+// components (rheology.cxx:527-534), as the FP64 step rounds it
+__device__ __forceinline__ void load_edot(const KP &p, int e, double edv, double *edot)
+{
+    const size_t ne = p.ne;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) edot[c] = p.srate[c * ne + e];
+    const double corr = div3(edv - (edot[0] + edot[1] + edot[2]));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) edot[i] += corr;
+}
+
+// edvoldt (geometry.cxx:158-179) from the step's nodal dvoldt
+__device__ __forceinline__ double elem_edv(const KP &p, int e)
+{
+    double dj = p.ntmp[conn_at(p, 0, e)];
+#pragma unroll
+    for (int i = 1; i < 4; ++i) dj += p.ntmp[conn_at(p, i, e)];
+    return dj / 4;
+}
+
+// the pressure change, and for the NMD gather its double-word product with
+// the volume, formed once per element instead of per node
+__device__ __forceinline__ void store_dp(const KP &p, int e, double dp, dw w, bool fused)
+{
+    p.dp[e] = dp;
+    if (fused && p.pv) {
+        const dw m = dw_mul(w, dw_split(p.vol[e]));
+        p.pv[e] = make_float2(m.hi, m.lo);
+    }
+}
+
+struct PlasticProps {
+    double amc, anphi, anpsi, hardn, ten_max;
+};
+
 // The mixed EVP branch where the FP32 screens leave it to FP64: the FP64
 // candidates -- the trial as the EP branch forms it (through the return map
 // unless the yield screen passed it) and the Maxwell update with FP64 terms
-// -- and, for an undecided choice (vless < 0), their FP64 comparison.  Out
-// of line: the elements that need it are few (yielding or near-tied), and
-// the registers of the return map stay out of the common path.
-__device__ __noinline__ unsigned evp_fp64_candidates(const KP &p, int e, double dt, double bulkm, double shearm,
-                                                     double visc, double s0, bool elastic, int vless, double amc,
-                                                     double anphi, double anpsi, double hardn, double ten_max,
-                                                     const double *edot, double *s, double &pls, double &dpls)
+// -- and, for an undecided choice (vless < 0), their FP64 comparison.  edot:
+// the corrected strain rate, s: the old stress, m: the plastic properties
+// (read unless elastic).  Out of line: the registers of the return map stay
+// out of the common path.
+static __device__ __noinline__ void evp_fp64_branch(const KP &p, int e, bool elastic, int vless, bool fused,
+                                                    const double *edot, const double *s, double pls,
+                                                    const PlasticProps &m)
 {
-    unsigned bits = 0;
-    double de[6];
+    const size_t ne = p.ne;
+    const double dt = p.clk->dt;
+    const double bulkm = m_bulkm(p, e), shearm = m_shearm(p, e);
+    double de[6], sp[6], sv[6];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) de[i] = edot[i] * dt;
-    const double dev = div3((de[0] + de[1]) + de[2]);
-    const double g2 = 2 * shearm;
-    double x[3], y[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        x[i] = s[i] - s0;
-        y[i] = g2 * (de[i] - dev);
+    for (int c = 0; c < 6; ++c) {
+        sp[c] = s[c];
+        de[c] = edot[c] * dt;
     }
-    double sp[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) sp[i] = s[i];
+    const double old_s = s[0] + s[1] + s[2];
     elastic_mixed(bulkm, shearm, de, sp);
     double depls = 0;
-    if (!elastic && mc_return_<3>(bulkm, shearm, amc, anphi, anpsi, hardn, ten_max, depls, sp))
-        bits |= DES_DEV_QL_NOCONV;
-    double sv[6];
+    if (!elastic && mc_return_<3>(bulkm, shearm, m.amc, m.anphi, m.anpsi, m.hardn, m.ten_max, depls, sp))
+        set_err(p, DES_DEV_QL_NOCONV);
     if (vless < 0) {
+        const double s0 = div3(old_s), dev = div3((de[0] + de[1]) + de[2]);
+        const double g2 = 2 * shearm;
+        double x[3], y[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            x[i] = s[i] - s0;
+            y[i] = g2 * (de[i] - dev);
+        }
+        const double visc = visc_mixed(p, e, edot, elem_avg_T<4>(p, e));
         maxwell_mixed_xy(maxwell_coef(shearm, visc, dt), g2, s0 + bulkm * dvol_mixed(p, e), x, y, s, de, sv);
         vless = second_invariant2_<3>(sv) < second_invariant2_<3>(sp);
     }
+    double out[6];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) s[i] = vless ? sv[i] : sp[i];
-    if (!vless) {
-        pls += depls;
-        dpls = depls;
+    for (int i = 0; i < 6; ++i) {
+        out[i] = vless ? sv[i] : sp[i];
+        p.stress[i * ne + e] = out[i];
     }
-    return bits;
+    if (!vless) {
+        p.pls[e] = pls + depls;
+        p.dpls[e] = depls;
+    }
+    const double dp = (out[0] + out[1] + out[2]) - old_s;
+    store_dp(p, e, dp, dw_split(dp), fused);
 }
 
-// update_stress (rheology.cxx:510-646), 3D, mixed precision
-// three blocks of 256 per SM (at most 85 registers; the spills stay in L1):
-// 24 resident warps instead of 16 at 128 registers, 15 us less at 998,400 tets
-__global__ void __launch_bounds__(TPB_M, 3) k_update_stress_mixed3(KP p, int fused)
+// the element's density and buoyancy term of the step (its temperature is final)
+__device__ __forceinline__ void store_density(const KP &p, int e, double T)
+{
+    const double rho = m_rho_T(p, e, T);
+    p.rho_e[e] = rho;
+    if (p.buoy_e) p.buoy_e[e] = p.prm.gravity != 0 ? rho * p.prm.gravity / 4 : 0.0;
+}
+
+// what is left of an element after the FP32 screens: nothing, or its FP64
+// branch with the screens' answers, or the screens again with the FP64
+// material terms
+enum EvpRest : int { EVP_DONE = 0, EVP_ELASTIC = 1, EVP_PLASTIC_BRANCH = 2, EVP_FP64 = 4, EVP_SCREEN = 8 };
+
+// The EVP branch choice of an element from its FP32 strain increments def and
+// relaxation tf, and its stress where the choice is the Maxwell branch: the
+// old stress s plus an FP32 increment.
+__device__ __forceinline__ int evp_screens(const KP &p, int e, const double *s, const float *def, float tf,
+                                           float shearf, float kf, ScreenTerms mt, bool fused)
+{
+    const size_t ne = p.ne;
+    const double s0 = div3(s[0] + s[1] + s[2]);
+    const float g2f = 2.0f * shearf;
+    const float trdef = (def[0] + def[1]) + def[2];
+    const float devf = trdef * (1.0f / 3.0f);
+    // x: the old deviator; y: the trial's deviatoric increment
+    float xf[6], yf[6], qf[6];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        xf[i] = f32_of(s[i] - s0);
+        yf[i] = g2f * (def[i] - devf);
+        xf[i + 3] = f32_of(s[i + 3]);
+        yf[i + 3] = g2f * def[i + 3];
+    }
+    const float dmp = kf * trdef;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) qf[c] = xf[c] + yf[c];
+    // the yield screen on the trial deviator qf: against the deviator of
+    // the FP64 trial elastic_mixed(s, de) it is off by xf's and qf's
+    // roundings and by yf's distance from the FP64 y (2^-22 of
+    // Lx + Ly + Y per component, taken as 2^-21 in the 2-norm) and by
+    // the FP64 roundings of the mean (22 u S, taken as 2^-44 S)
+    const float s0f = f32_of(s0);
+    float Y = 0.0f, Sdev = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) Y += fabsf(def[i]);
+    Y *= g2f;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) Sdev += fabsf(xf[c]) + fabsf(yf[c]);
+    Sdev += Y;
+    const float S = fabsf(s0f) + Sdev + 2.0f * fabsf(kf) * (Y / fmaxf(g2f, 1e-30f));
+    const int screen = yield_screen3_f(mt.af, mt.cf, mt.tf, s0f + dmp, fabsf(s0f) + fabsf(dmp), qf,
+                                       0x1p-44f * S + 0x1p-21f * Sdev, mt.err);
+    if (screen < 0) return EVP_SCREEN;
+    if (screen == 0) return EVP_FP64;
+    const int vless = evp_choice_f(xf, yf, qf, tf, Y, S);
+    if (vless != 1) return EVP_FP64 | EVP_ELASTIC | (vless == 0 ? EVP_PLASTIC_BRANCH : 0);
+    const float f2 = 1.0f / (1.0f + tf), c1 = -2.0f * tf * f2;
+    const float dmv = kf * dvol_f(p, e);
+    float dn = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const float d = fmaf(xf[i], c1, fmaf(yf[i], f2, dmv));
+        p.stress[i * ne + e] = s[i] + f64_of(d);
+        dn += d;
+        p.stress[(i + 3) * ne + e] = s[i + 3] + f64_of(fmaf(xf[i + 3], c1, yf[i + 3] * f2));
+    }
+    const double dp = f64_of(dn);
+    store_dp(p, e, dp, dw_split(dp), fused);
+    return EVP_DONE;
+}
+
+// tmp = dt G / (2 visc), the Maxwell update's relaxation
+__device__ __forceinline__ float relaxation_f(float dtf, float shearf, float viscf)
+{
+    return (0.5f * dtf * shearf) / viscf;
+}
+
+__device__ __forceinline__ void load_stress(const KP &p, int e, double *s)
+{
+#pragma unroll
+    for (int c = 0; c < 6; ++c) s[c] = p.stress[c * (size_t)p.ne + e];
+}
+
+__device__ __forceinline__ ScreenTerms exact_terms(const PlasticProps &m)
+{
+    return {f32_of(m.anphi), f32_of(m.amc), f32_of(m.ten_max), 0.0f};
+}
+
+__device__ __forceinline__ int screened_choice(int rest) { return rest & EVP_PLASTIC_BRANCH ? 0 : -1; }
+
+// what evp_screens left of element e; edot_done: p.srate holds the corrected
+// strain rate
+static __device__ __noinline__ void evp_rest(const KP &p, int e, int rest, bool fused, bool edot_done)
+{
+    double edot[6], s[6];
+    if (edot_done) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) edot[c] = p.srate[c * (size_t)p.ne + e];
+    } else {
+        load_edot(p, e, elem_edv(p, e), edot);
+    }
+    load_stress(p, e, s);
+    const double pls = p.pls[e];
+    PlasticProps m{};
+    if (!(rest & EVP_ELASTIC)) m_plastic_props(p, e, pls, m.amc, m.anphi, m.anpsi, m.hardn, m.ten_max);
+    if (rest & EVP_SCREEN) {
+        const float dtf = f32_of(p.clk->dt), shearf = f32_of(m_shearm(p, e));
+        float def[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) def[c] = f32_of(edot[c]) * dtf;
+        const float viscf = f32_of(visc_mixed(p, e, edot, elem_avg_T<4>(p, e)));
+        rest = evp_screens(p, e, s, def, relaxation_f(dtf, shearf, viscf), shearf, f32_of(m_bulkm(p, e)),
+                           exact_terms(m), fused);
+        if (rest == EVP_DONE) return;
+    }
+    evp_fp64_branch(p, e, (rest & EVP_ELASTIC) != 0, screened_choice(rest), fused, edot, s, pls, m);
+}
+
+// update_stress (rheology.cxx:510-646), 3D, mixed precision, the EVP
+// rheology.  Each thread updates its element's strain and, where the FP32
+// screens decide it (nearly all elements of a mesh that does not yield), its
+// stress by the Maxwell increments.  The others -- at or near the yield
+// surface, or with nearly tied branches -- go to a list in shared memory,
+// and once the block's common path is done its first threads run their FP64
+// branch side by side: a return map's FP64 instructions (several hundred)
+// then serve full warps instead of the few lanes of each warp that yield,
+// and its registers stay out of the common path.  An element's result does
+// not depend on its place in the list.  LIST false (a mesh of at most one
+// wave, where the length of a thread's chain shows and registers do not): the
+// thread forms the FP64 properties first and goes on to the FP64 branch with
+// what it holds.
+// outputs: write the strain rate and edvoldt, which only the end of a call
+// shows (a chained step that another follows leaves them out).
+template <bool LIST>
+__global__ void __launch_bounds__(LIST ? 128 : 64, LIST ? 8 : 4) k_update_stress_evp3(KP p, int fused, int outputs)
+{
+    __shared__ int list[128];
+    __shared__ int listed;
+    if (LIST) {
+        if (threadIdx.x == 0) listed = 0;
+        __syncthreads();
+    }
+    const int base = p.e_lo + (int)(blockIdx.x * blockDim.x), e = base + (int)threadIdx.x;
+    const size_t ne = p.ne;
+    if (e < p.e_hi) {
+        const float dtf = f32_of(p.clk->dt);
+        float def[6];
+        double edot[6];
+        {   // FP32 strain increments; the strain accumulates them in FP64
+            double edv;
+            if (fused) {
+                edv = elem_edv(p, e);
+                if (outputs) p.edvoldt[e] = edv;
+            } else {
+                edv = p.edvoldt[e];
+            }
+            load_edot(p, e, edv, edot);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                if (outputs) p.srate[c * ne + e] = edot[c];
+                def[c] = f32_of(edot[c]) * dtf;
+                p.strain[c * ne + e] += f64_of(def[c]);
+            }
+        }
+        const double T = elem_avg_T<4>(p, e);
+        const float shearf = f32_of(m_shearm(p, e));
+        const float tf = relaxation_f(dtf, shearf, f32_of(visc_mixed(p, e, edot, T)));
+        if (fused && p.rho_e) store_density(p, e, T);
+        const double pls = p.pls[e];
+        double s[6];
+        load_stress(p, e, s);
+        PlasticProps m;
+        ScreenTerms mt;
+        if (LIST) {
+            mt = screen_terms(p, e, pls);
+        } else {
+            m_plastic_props(p, e, pls, m.amc, m.anphi, m.anpsi, m.hardn, m.ten_max);
+            mt = exact_terms(m);
+        }
+        const int rest = evp_screens(p, e, s, def, tf, shearf, f32_of(m_bulkm(p, e)), mt, fused != 0);
+        if (LIST) {
+            if (rest) list[atomicAdd(&listed, 1)] = ((int)threadIdx.x << 4) | rest;
+        } else if (rest) {
+            evp_fp64_branch(p, e, (rest & EVP_ELASTIC) != 0, screened_choice(rest), fused != 0, edot, s, pls, m);
+        }
+    }
+    if (!LIST) return;
+    __syncthreads();
+    const int n = listed;
+    for (int k = threadIdx.x; k < n; k += blockDim.x)
+        evp_rest(p, base + (list[k] >> 4), list[k] & 15, fused != 0, outputs || !fused);
+}
+
+// the other rheologies
+__global__ void __launch_bounds__(128, 6) k_update_stress_mixed3(KP p, int fused)
 {
     int e = p.e_lo + blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= p.e_hi) return;
     const size_t ne = p.ne;
     double edv;
     if (fused) {
-        double dj = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) dj += p.ntmp[conn_at(p, i, e)];
-        edv = dj / 4;
+        edv = elem_edv(p, e);
         p.edvoldt[e] = edv;
     } else {
         edv = p.edvoldt[e];
     }
-    double s[6], es[6], edot[6];
+    double s[6], es[6], edot[6], de[6];
+    load_edot(p, e, edv, edot);
+    const double dt = p.clk->dt;
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
         s[c] = p.stress[c * ne + e];
-        es[c] = p.strain[c * ne + e];
-        edot[c] = p.srate[c * ne + e];
+        de[c] = edot[c] * dt;
+        es[c] = p.strain[c * ne + e] + de[c];
     }
-    double pls = p.pls[e], dpls = p.dpls[e];
-    const double dt = p.clk->dt;
     const double old_s = s[0] + s[1] + s[2];
-    {
-        const double div = edot[0] + edot[1] + edot[2];
-        const double corr = div3(edv - div);   // as the FP64 step rounds it
-#pragma unroll
-        for (int i = 0; i < 3; ++i) edot[i] += corr;
-    }
     const int rt = p.mat.rheol_type;
-    double de[6];
-    if (rt != DES_RH_EVP) {
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            de[i] = edot[i] * dt;
-            es[i] += de[i];
-        }
-    }
-    double dpv = 0;   // dpressure
-    bool dp_set = false;
     const double bulkm = m_bulkm(p, e), shearm = m_shearm(p, e);
     const double T = elem_avg_T<4>(p, e);
     unsigned bits = 0;
@@ -385,8 +590,9 @@ __global__ void __launch_bounds__(TPB_M, 3) k_update_stress_mixed3(KP p, int fus
         viscous_<3>(bulkm, visc_mixed(p, e, edot, T), es[0] + es[1] + es[2], edot, s);
     } else if (rt == DES_RH_MAXWELL) {
         maxwell_mixed(bulkm, shearm, visc_mixed(p, e, edot, T), dt, dvol_mixed(p, e), de, s);
-    } else if (rt == DES_RH_EP) {
+    } else {   // EP
         double amc, anphi, anpsi, hardn, ten_max;
+        const double pls = p.pls[e];
         m_plastic_props(p, e, pls, amc, anphi, anpsi, hardn, ten_max);
         elastic_mixed(bulkm, shearm, de, s);
         const double am = div3(s[0] + s[1] + s[2]);
@@ -395,73 +601,8 @@ __global__ void __launch_bounds__(TPB_M, 3) k_update_stress_mixed3(KP p, int fus
         if (!clearly_elastic3_dev(amc, anphi, ten_max, am, q, s)
             && mc_return_<3>(bulkm, shearm, amc, anphi, anpsi, hardn, ten_max, depls, s))
             bits |= DES_DEV_QL_NOCONV;
-        pls += depls;
-        dpls = depls;
-    } else {   // EVP: the smaller second invariant wins (rheology.cxx:594-634)
-        double amc, anphi, anpsi, hardn, ten_max;
-        m_plastic_props(p, e, pls, amc, anphi, anpsi, hardn, ten_max);
-        // FP32 strain increments; the strain accumulates them in FP64
-        const float dtf = f32_of(dt);
-        float def[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            def[i] = f32_of(edot[i]) * dtf;
-            es[i] += f64_of(def[i]);
-        }
-        const double s0 = div3(old_s);
-        const float g2f = 2.0f * f32_of(shearm), kf = f32_of(bulkm);
-        const float trdef = (def[0] + def[1]) + def[2];
-        const float devf = trdef * (1.0f / 3.0f);
-        // x: the old deviator; y: the trial's deviatoric increment
-        float xf[6], yf[6];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            xf[i] = f32_of(s[i] - s0);
-            yf[i] = g2f * (def[i] - devf);
-            xf[i + 3] = f32_of(s[i + 3]);
-            yf[i + 3] = g2f * def[i + 3];
-        }
-        const double visc = visc_mixed(p, e, edot, T);
-        const MaxwellF mc = maxwell_coef_f(shearm, visc, dt);
-        const float tf = (0.5f * dtf * f32_of(shearm)) / f32_of(visc);
-        const float dmp = kf * trdef;
-        float qf[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) qf[c] = xf[c] + yf[c];
-        // the yield screen on the trial deviator qf: against the deviator of
-        // the FP64 trial elastic_mixed(s, de) it is off by xf's and qf's
-        // roundings and by yf's distance from the FP64 y (2^-22 of
-        // Lx + Ly + Y per component, taken as 2^-21 in the 2-norm) and by
-        // the FP64 roundings of the mean (22 u S, taken as 2^-44 S)
-        const float s0f = f32_of(s0);
-        float Y = 0.0f, Sdev = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) Y += fabsf(def[i]);
-        Y *= g2f;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) Sdev += fabsf(xf[c]) + fabsf(yf[c]);
-        Sdev += Y;
-        const float S = fabsf(s0f) + Sdev + 2.0f * fabsf(kf) * (Y / fmaxf(g2f, 1e-30f));
-        const bool elastic = clearly_elastic3_f(f32_of(anphi), f32_of(amc), f32_of(ten_max), s0f + dmp,
-                                                fabsf(s0f) + fabsf(dmp), qf, 0x1p-44f * S + 0x1p-21f * Sdev);
-        int vless = elastic ? evp_choice_f(xf, yf, qf, tf, Y, S) : -1;
-        if (vless == 1) {
-            // the Maxwell update as the old stress plus its FP32 increment
-            const float dmv = kf * dvol_f(p, e);
-            float dn = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const float d = fmaf(xf[i], mc.c1, fmaf(yf[i], mc.f2, dmv));
-                s[i] += f64_of(d);
-                dn += d;
-                s[i + 3] += f64_of(fmaf(xf[i + 3], mc.c1, yf[i + 3] * mc.f2));
-            }
-            dpv = f64_of(dn);
-            dp_set = true;
-        } else {
-            bits |= evp_fp64_candidates(p, e, dt, bulkm, shearm, visc, s0, elastic, vless, amc, anphi, anpsi, hardn,
-                                        ten_max, edot, s, pls, dpls);
-        }
+        p.pls[e] = pls + depls;
+        p.dpls[e] = depls;
     }
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
@@ -469,19 +610,9 @@ __global__ void __launch_bounds__(TPB_M, 3) k_update_stress_mixed3(KP p, int fus
         p.strain[c * ne + e] = es[c];
         p.srate[c * ne + e] = edot[c];
     }
-    p.pls[e] = pls;
-    p.dpls[e] = dpls;
-    const double dpf = dp_set ? dpv : (s[0] + s[1] + s[2]) - old_s;
-    p.dp[e] = dpf;
-    if (fused && p.pv) {   // the NMD gather's double-word dp vol, formed once per element instead of per node
-        const dw w = dw_mul(dw_split(dpf), dw_split(p.vol[e]));
-        p.pv[e] = make_float2(w.hi, w.lo);
-    }
-    if (fused && p.rho_e) {
-        const double rho = m_rho_T(p, e, T);
-        p.rho_e[e] = rho;
-        if (p.buoy_e) p.buoy_e[e] = p.prm.gravity != 0 ? rho * p.prm.gravity / 4 : 0.0;
-    }
+    const double dp = (s[0] + s[1] + s[2]) - old_s;
+    store_dp(p, e, dp, dw_split(dp), fused != 0);
+    if (fused && p.rho_e) store_density(p, e, T);
     if (bits) set_err(p, bits);
 }
 
@@ -665,9 +796,15 @@ __global__ void __launch_bounds__(128) k_node_pass_mixed3(KP p, int heat, int be
     }
 }
 
-int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused)
+int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused, bool outputs)
 {
-    DES_LAUNCH(k_update_stress_mixed3, p.e_hi - p.e_lo, s, p, (int)fused);
+    const int n = p.e_hi - p.e_lo;
+    if (p.mat.rheol_type == DES_RH_EVP) {
+        if (block_threads(n) < 128) DES_LAUNCH(k_update_stress_evp3<false>, n, s, p, (int)fused, (int)(outputs || !fused));
+        else DES_LAUNCH(k_update_stress_evp3<true>, n, s, p, (int)fused, (int)(outputs || !fused));
+    } else {
+        DES_LAUNCH(k_update_stress_mixed3, n, s, p, (int)fused);
+    }
     return 1;
 }
 

@@ -7,7 +7,9 @@
 
 namespace des {
 
-int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused);
+// outputs: also write the strain rate and edvoldt of a fused step (nothing
+// in the step that follows reads them)
+int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused, bool outputs = true);
 int launch_strain_rate_mixed(const KP &p, cudaStream_t s, bool begin_step);
 int launch_heat_and_dvoldt_mixed(const KP &p, cudaStream_t s, bool heat, bool dvoldt);
 // fused step: strain rate + heat terms + dvoldt terms, then the nodal sums and the temperature update

@@ -378,18 +378,50 @@ __device__ __forceinline__ void jacobi3f(const float d[6], float w[3], float (&v
 // mf the mean stress, mag an FP32 bound on |m| that also covers the FP32
 // rounding mf carries, dev_err a bound on the 2-norm distance of d (before
 // its rounding to FP32) from the exact deviator of the FP64 stress.
-__device__ __forceinline__ bool clearly_elastic3_f(float af, float cf, float tf, float mf, float mag,
-                                                   const float d[6], float dev_err)
+// yield_screen3_f is that screen with material terms af, cf, tf that may be
+// off by up to a relative prop_err from the FP32 roundings of the FP64 ones:
+// 1 where the screen of those passes whatever the error, 0 where it fails
+// whatever the error, -1 where the error decides (never for prop_err = 0).
+__device__ __forceinline__ int yield_screen3_f(float af, float cf, float tf, float mf, float mag, const float d[6],
+                                               float dev_err, float prop_err)
 {
-    float w[3], v[3][3];
-    jacobi3f(d, w, v);
     const float nf = sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]
                            + 2.0f * (d[3] * d[3] + d[4] * d[4] + d[5] * d[5]));
     const float tol = 0x1p-12f * nf + 0x1p-19f * (mag + nf) + dev_err + 0x1p-100f;
+    const float fs_min = (1.0f + af) * tol + 0x1p-19f * fabsf(cf), ft_max = -(tol + 0x1p-19f * fabsf(tf));
+    // First with bounds in the eigenvalues' place: no eigenvalue of d exceeds
+    // ||d||_F, and the rotations' and nf's FP32 errors lie far below 2^-10 of
+    // it (2^-70 covers squares that underflow).  FP32 rounding is monotonic,
+    // so what passes here passes with the eigenvalues too: the same answer
+    // without the ~600 instructions of the rotations.  A NaN passes neither.
+    // What a relative error e of the material terms moves: fs by e (|p2| af +
+    // |cf|), ft by e |tf|, the limits by e of themselves, each taken twice,
+    // with 2^-20 of the terms for the sums' own roundings.
+    const float e2 = prop_err > 0.0f ? 2.0f * prop_err + 0x1p-20f : 0.0f;
+    const float dt = e2 * (fabsf(tf) + fabsf(ft_max));
+    const float R = 0x1.004p0f * nf + 0x1p-70f;
+    {
+        const float hi = mf + R, lo = mf - R;
+        const float ds = e2 * (fabsf(lo) + fabsf(hi) * af + fabsf(cf) + fs_min);
+        if (lo - hi * af + cf > fs_min + ds && hi - tf < ft_max - dt) return 1;
+    }
+    float w[3], v[3][3];
+    jacobi3f(d, w, v);
     const float p0 = mf + w[0], p2 = mf + w[2];
     const float fs = p0 - p2 * af + cf;
     const float ft = p2 - tf;
-    return fs > (1.0f + af) * tol + 0x1p-19f * fabsf(cf) && ft < -(tol + 0x1p-19f * fabsf(tf));
+    if (prop_err > 0.0f) {
+        const float ds = e2 * (fabsf(p0) + fabsf(p2) * af + fabsf(cf) + fs_min);
+        if (fs > fs_min + ds && ft < ft_max - dt) return 1;
+        return fs < fs_min - ds || ft > ft_max + dt ? 0 : -1;
+    }
+    return fs > fs_min && ft < ft_max;
+}
+
+__device__ __forceinline__ bool clearly_elastic3_f(float af, float cf, float tf, float mf, float mag,
+                                                   const float d[6], float dev_err)
+{
+    return yield_screen3_f(af, cf, tf, mf, mag, d, dev_err, 0.0f) == 1;
 }
 
 // The same screen given the mean stress m and the normal deviator q_i = s_i - m
