@@ -413,12 +413,12 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     int *d_sup_pos = nullptr;
     double *d_qv = nullptr, *d_hc64 = nullptr;
     add((void **)&d_qv, (size_t)ne * D);
+    add((void **)&d_ndpk, (size_t)ne * sizeof(double4));
     if (mixed3) {
         add((void **)&d_hc, (size_t)ne * npe * sizeof(float));
         add((void **)&d_ft, (size_t)ne * npe * 2 * sizeof(float4));
         add((void **)&d_shpdw, (size_t)ne * npe * nd * sizeof(float2));
         add((void **)&d_vdw, (size_t)nn * nd * sizeof(float2));
-        add((void **)&d_ndpk, (size_t)ne * sizeof(double4));
         add((void **)&d_pv, (size_t)ne * sizeof(float2));
         add((void **)&d_sup_pos, (size_t)ne * npe * I);
     } else {
@@ -1259,79 +1259,61 @@ int record_mid(cudaEvent_t mid, cudaStream_t s)
     return mid ? (cudaEventRecordWithFlags(mid, s, cudaEventRecordExternal) == cudaSuccess ? 0 : -1) : 0;
 }
 
-int enqueue_step_mixed(des_ctx *c, cudaEvent_t mid)
+// what one step's geometry pass does at the end of the step
+int step_geometry(const KP &p)
 {
-    const KP p = step_kp(c);
-    cudaStream_t s = c->stream;
-    int n = 0;
-    const bool thermal = p.prm.has_thermal_diffusion != 0;
-    n += launch_elem_pass_mixed(p, s, thermal);
-    n += launch_node_pass_mixed(p, s, thermal);
-    n += launch_update_stress_mixed(p, s, true);
-    n += launch_nmd_gather(p, s, true);
-    n += launch_nmd_correct(p, s, true);
-    if (record_mid(mid, s)) return -1;
-    n += launch_force(p, s, true, true);
-    int geo = GEO_COPY_OLD | GEO_VOLUME | GEO_SHAPE | GEO_DT | GEO_DT_IF_STEP | GEO_MASS_TERMS;
+    int geo = GEO_COPY_OLD | GEO_VOLUME | GEO_SHAPE | GEO_DT | GEO_DT_IF_STEP | GEO_DT_FINAL | GEO_MASS_TERMS;
     if (p.mat.rheol_type & DES_RH_ELASTIC) geo |= GEO_ROTATE;   // FP32 increments in a mixed context
-    n += launch_geometry(p, s, geo);
-    n += launch_mass_sum(p, s);
-    n += launch_dt_finalize(p, s, true);
-    return n;
+    return geo;
 }
 
-// The chained mixed step (part 0 first, 1 middle, 2 last of des_step(n),
-// n >= 2).  update_mesh's passes end each step but the last as one
-// look-ahead pass that also does the next step's element pass (strain rate,
-// dvoldt and heat terms: the next step reads the same velocities, shape
-// functions, volumes and temperatures), and the next step's node pass forms
-// the mass sums before its own (nothing in between reads mass, tmass or
-// volume_n).  Every kernel does the arithmetic of enqueue_step_mixed's, so
-// n chained steps give the bits of n single steps; the last step ends as a
+// The chained step (part 0 first, 1 middle, 2 last of des_step(n), n >= 2).
+// update_mesh's passes end each step but the last as one look-ahead pass that
+// also does the next step's element pass (strain rate, dvoldt and heat terms:
+// the next step reads the same velocities, shape functions, volumes and
+// temperatures), and the next step's node pass forms the mass sums before its
+// own (nothing in between reads mass, tmass or volume_n): six launches a step
+// instead of eight.  Every kernel does the arithmetic of a single step's, so n
+// chained steps give the bits of n single steps; the last step ends as a
 // single step does, leaving the same state.
-int enqueue_step_mixed_chain(des_ctx *c, int part)
+int enqueue_step_chain(des_ctx *c, int part)
 {
     const KP p = step_kp(c);
     cudaStream_t s = c->stream;
     int n = 0;
-    const bool thermal = p.prm.has_thermal_diffusion != 0;
-    if (part == 0) n += launch_elem_pass_mixed(p, s, thermal);
-    n += launch_node_pass_mixed(p, s, thermal, part != 0, part != 0);
-    n += launch_update_stress_mixed(p, s, true, part == 2);
-    n += launch_nmd_gather(p, s, true);
+    const bool thermal = p.prm.has_thermal_diffusion != 0, mixed = use_mixed(c);
+    if (part == 0) n += mixed ? launch_elem_pass_mixed(p, s, thermal) : launch_elem_pass(p, s, thermal);
+    n += mixed ? launch_node_pass_mixed(p, s, thermal, part != 0, part != 0)
+               : launch_node_pass(p, s, thermal, part != 0);
+    n += mixed ? launch_update_stress_mixed(p, s, true, part == 2) : launch_update_stress(p, s, true);
+    n += launch_nmd_gather(p, s, mixed);
     n += launch_nmd_correct(p, s, true);
-    n += launch_force(p, s, true, true);
-    int geo = GEO_COPY_OLD | GEO_VOLUME | GEO_SHAPE | GEO_DT | GEO_DT_IF_STEP | GEO_MASS_TERMS;
-    if (p.mat.rheol_type & DES_RH_ELASTIC) geo |= GEO_ROTATE;
+    n += launch_force(p, s, true, mixed);
     if (part == 2) {
-        n += launch_geometry(p, s, geo);
+        n += launch_geometry(p, s, step_geometry(p));
         n += launch_mass_sum(p, s);
     } else {
-        n += launch_geometry_ahead(p, s, geo);
+        n += launch_geometry_ahead(p, s, step_geometry(p));
     }
-    n += launch_dt_finalize(p, s, true);
     return n;
 }
 
 int enqueue_step(des_ctx *c, cudaEvent_t mid)
 {
-    if (use_mixed(c)) return enqueue_step_mixed(c, mid);
     const KP p = step_kp(c);
     cudaStream_t s = c->stream;
     int n = 0;
-    const bool thermal = p.prm.has_thermal_diffusion != 0;
-    n += launch_elem_pass(p, s, thermal);   // strain rate, element dvoldt and heat terms
-    n += launch_node_pass(p, s, thermal);   // nodal sums, temperature update
-    n += launch_update_stress(p, s, true);
-    n += launch_nmd_gather(p, s);
+    const bool thermal = p.prm.has_thermal_diffusion != 0, mixed = use_mixed(c);
+    // strain rate, element dvoldt and heat terms, then nodal sums and the temperature update
+    n += mixed ? launch_elem_pass_mixed(p, s, thermal) : launch_elem_pass(p, s, thermal);
+    n += mixed ? launch_node_pass_mixed(p, s, thermal) : launch_node_pass(p, s, thermal);
+    n += mixed ? launch_update_stress_mixed(p, s, true) : launch_update_stress(p, s, true);
+    n += launch_nmd_gather(p, s, mixed);
     n += launch_nmd_correct(p, s, true);
     if (record_mid(mid, s)) return -1;
-    n += launch_force(p, s, true);
-    int geo = GEO_COPY_OLD | GEO_VOLUME | GEO_SHAPE | GEO_DT | GEO_DT_IF_STEP | GEO_MASS_TERMS;
-    if (p.mat.rheol_type & DES_RH_ELASTIC) geo |= GEO_ROTATE;
-    n += launch_geometry(p, s, geo);
+    n += launch_force(p, s, true, mixed);
+    n += launch_geometry(p, s, step_geometry(p));
     n += launch_mass_sum(p, s);
-    n += launch_dt_finalize(p, s, true);
     return n;
 }
 
@@ -1363,7 +1345,7 @@ int build_chain_graph(des_ctx *c, int part)
 {
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int n = enqueue_step_mixed_chain(c, part);
+    int n = enqueue_step_chain(c, part);
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (e != cudaSuccess) return cuda_fail(c, e, "cudaStreamEndCapture");
     e = cudaGraphInstantiate(&c->chain_exec[part], g, 0);
@@ -1676,7 +1658,7 @@ int des_step(des_ctx *c, int nsteps)
 {
     if (!c || nsteps < 0) return DES_EINPUT;
     if (!c->has_state) return fail_msg(c->err, DES_EINPUT, "des_step before des_upload_state");
-    if (nsteps >= 2 && use_mixed(c)) {   // the chained step
+    if (nsteps >= 2) {   // the chained step
         for (int part = 0; part < 3; ++part) {
             int rc;
             if (!c->chain_exec[part] && (rc = build_chain_graph(c, part))) return rc;

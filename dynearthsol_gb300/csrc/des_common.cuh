@@ -34,7 +34,7 @@ struct Clock {
     double time;
     double dt;
     int steps;
-    int pad;
+    unsigned blocks_done;   // blocks of a dt step's geometry pass that are done
     // compute_dt accumulators: min over elements as ordered bit patterns
     unsigned long long red_minh;
     unsigned long long red_maxwell;
@@ -117,7 +117,7 @@ struct KP {
     // shp, which downloads fill from them on demand.
     float2 *shpdw;
     float2 *vdw;                         // [3][nn] a mixed context's velocities as double-word pairs, from the force pass
-    double4 *ndpk;                       // [ne] a mixed context's {qv, vol, me, tme}, from the look-ahead geometry pass
+    double4 *ndpk;                       // [ne] {qv, vol, me, tme} from the chained step's look-ahead geometry pass
     float2 *pv;                          // [ne] a mixed context's double-word dp vol, from the fused stress pass
     float *hc;                           // [4][ne] per-element heat terms of the mixed step, or null
     double *qv;                          // [ne] per-element dvoldt term of the fused steps, or null

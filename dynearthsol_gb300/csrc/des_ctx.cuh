@@ -33,7 +33,7 @@ struct des_ctx {
     unsigned long long *d_red = nullptr;
     double *d_ef[DES_EF_COUNT] = {};
     cudaGraphExec_t step_exec = nullptr;
-    // the chained mixed step of des_step(n >= 2): its first, middle and last
+    // the chained step of des_step(n >= 2): its first, middle and last
     // steps (a look-ahead geometry pass does the next step's element pass,
     // and the next node pass the mass sums; the last step ends as one step)
     cudaGraphExec_t chain_exec[3] = {};

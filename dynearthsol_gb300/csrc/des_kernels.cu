@@ -32,20 +32,13 @@ static inline int nblocks(long long n, int tpb = TPB)
 // ==================================================================
 // strain rate (fields.cxx:166-232)
 // ==================================================================
+// strain rate from the element's node velocities v[i][d] and gradients
+// dN_i/dx (sx, sy, sz; sy unused in 2D)
 template <int ND>
-__device__ __forceinline__ void strain_rate_elem(const KP &p, int e, double *s)
+__device__ __forceinline__ void strain_rate_vals(const double (*v)[ND], const double *sx, const double *sy,
+                                                 const double *sz, double *s)
 {
     constexpr int NPE = ND + 1;
-    double v[NPE][ND];
-    double sx[NPE], sy[NPE], sz[NPE];
-#pragma unroll
-    for (int i = 0; i < NPE; ++i) {
-        int n = conn_at(p, i, e);
-        load_node_v<ND>(p, n, v[i]);
-        sx[i] = shp_at(p, 0, i, e);
-        if (ND == 3) sy[i] = shp_at(p, 1, i, e);
-        sz[i] = shp_at(p, ND - 1, i, e);
-    }
     // The sums start from their first term, and the halves of the shear
     // components are taken once per sum (a scaling by two commutes with every
     // rounding above the subnormal range): the reference's bits with 15 of
@@ -73,6 +66,21 @@ __device__ __forceinline__ void strain_rate_elem(const KP &p, int e, double *s)
         s[1] = normal(ND - 1, sz);
         s[2] = shear(0, sz, ND - 1, sx);
     }
+}
+
+template <int ND>
+__device__ __forceinline__ void strain_rate_elem(const KP &p, int e, double *s)
+{
+    constexpr int NPE = ND + 1;
+    double v[NPE][ND], sx[NPE], sy[NPE], sz[NPE];
+#pragma unroll
+    for (int i = 0; i < NPE; ++i) {
+        load_node_v<ND>(p, conn_at(p, i, e), v[i]);
+        sx[i] = shp_at(p, 0, i, e);
+        sy[i] = ND == 3 ? shp_at(p, 1, i, e) : 0.0;
+        sz[i] = shp_at(p, ND - 1, i, e);
+    }
+    strain_rate_vals<ND>(v, sx, sy, sz, s);
 }
 
 template <int ND>
@@ -148,14 +156,48 @@ __global__ void __launch_bounds__(128) k_node_gather1(KP p)
 // The fused step's form of the same three functions (update_strain_rate,
 // the heat gather of update_temperature, compute_dvoldt), element-centric.
 // k_elem_pass writes the strain rate, the element's dvoldt term qv = tr(edot)
-// vol and, with heat, its contribution to each of its nodes' tdot (slot i of
-// hc64).  The stencil D_ij = dN_i . dN_j is formed once per element: D_ji is
+// vol and, with heat (elem_terms, which returns qv), its contribution to each
+// of its nodes' tdot (slot i of hc64).  The stencil D_ij = dN_i . dN_j is formed once per element: D_ji is
 // the same products in the same order, so every slot holds the very value
 // heat_term gives for (e, i), at 10 instead of 16 dot products.
 // k_node_pass sums the slots and the qv over each node's support in
 // ascending element order -- the node-centric kernels' order -- and applies
 // the temperature update.  The bits are those of k_strain_rate,
 // k_node_gather1 and k_temperature_update.
+template <int ND>
+__device__ __forceinline__ double elem_terms(const KP &p, int e, const double *sr, double vol, const double *sx,
+                                             const double *sy, const double *sz, bool heat)
+{
+    constexpr int NPE = ND + 1;
+    const size_t ne = p.ne;
+    double dj;
+    if (ND == 3) dj = sr[0] + sr[1] + sr[2];
+    else dj = sr[0] + sr[1];
+    if (heat) {
+        const double kv = m_k(p, e) * vol;
+        const double rh = m_hr_over_cp(p, e) * vol;
+        double T[NPE], D[NPE][NPE];
+#pragma unroll
+        for (int i = 0; i < NPE; ++i) T[i] = p.T[conn_at(p, i, e)];
+#pragma unroll
+        for (int i = 0; i < NPE; ++i)
+#pragma unroll
+            for (int j = i; j < NPE; ++j) {
+                D[i][j] = (ND == 3) ? (sx[i] * sx[j] + sy[i] * sy[j] + sz[i] * sz[j])
+                                    : (sx[i] * sx[j] + sz[i] * sz[j]);
+                D[j][i] = D[i][j];
+            }
+#pragma unroll
+        for (int i = 0; i < NPE; ++i) {
+            double diffusion = D[i][0] * T[0];
+#pragma unroll
+            for (int j = 1; j < NPE; ++j) diffusion += D[i][j] * T[j];
+            p.hc64[(size_t)i * ne + e] = diffusion * kv - rh;
+        }
+    }
+    return dj * vol;
+}
+
 template <int ND>
 __global__ void __launch_bounds__(TPB) k_elem_pass(KP p, int heat)
 {
@@ -171,62 +213,67 @@ __global__ void __launch_bounds__(TPB) k_elem_pass(KP p, int heat)
     strain_rate_elem<ND>(p, e, sr);
 #pragma unroll
     for (int c = 0; c < NSTR; ++c) p.srate[(size_t)c * ne + e] = sr[c];
-    const double vol = p.vol[e];
-    double dj;
-    if (ND == 3) dj = sr[0] + sr[1] + sr[2];
-    else dj = sr[0] + sr[1];
-    p.qv[e] = dj * vol;
-    if (!heat) return;
-    const double kv = m_k(p, e) * vol;
-    const double rh = m_hr_over_cp(p, e) * vol;
-    double sx[NPE], sy[NPE], sz[NPE], T[NPE];
+    double sx[NPE], sy[NPE], sz[NPE];
 #pragma unroll
     for (int i = 0; i < NPE; ++i) {
         sx[i] = shp_at(p, 0, i, e);
-        sy[i] = (ND == 3) ? shp_at(p, 1, i, e) : 0.0;
+        sy[i] = ND == 3 ? shp_at(p, 1, i, e) : 0.0;
         sz[i] = shp_at(p, ND - 1, i, e);
-        T[i] = p.T[conn_at(p, i, e)];
     }
-    double D[NPE][NPE];
-#pragma unroll
-    for (int i = 0; i < NPE; ++i)
-#pragma unroll
-        for (int j = i; j < NPE; ++j) {
-            D[i][j] = (ND == 3) ? (sx[i] * sx[j] + sy[i] * sy[j] + sz[i] * sz[j]) : (sx[i] * sx[j] + sz[i] * sz[j]);
-            D[j][i] = D[i][j];
-        }
-#pragma unroll
-    for (int i = 0; i < NPE; ++i) {
-        double diffusion = D[i][0] * T[0];
-#pragma unroll
-        for (int j = 1; j < NPE; ++j) diffusion += D[i][j] * T[j];
-        p.hc64[(size_t)i * ne + e] = diffusion * kv - rh;
-    }
+    p.qv[e] = elem_terms<ND>(p, e, sr, p.vol[e], sx, sy, sz, heat != 0);
 }
 
-template <int ND, bool STAGED>
+// MASS (a chained step): the previous step's compute_mass sums come first,
+// from the records of the look-ahead geometry pass (KP::ndpk), as k_mass_sum
+// forms them, and the step's clock is started here.
+template <int ND, bool MASS, bool STAGED>
 __global__ void __launch_bounds__(128) k_node_pass(KP p, int heat)
 {
+    if (MASS && blockIdx.x == 0 && threadIdx.x == 0) {   // dynearthsol.cxx:325-326
+        p.clk->steps += 1;
+        p.clk->time += p.clk->dt;
+    }
+    constexpr int NQ = MASS ? 5 : 2;
     const size_t ne = p.ne;
-    double sum[2] = {0, 0};   // dvoldt, tdot
-    const int n = node_sums<SumF64, 2, ND, STAGED>(
-        p.sup_off, p.n_lo, p.n_hi, heat ? 2 : 1,
+    const bool thermal = p.prm.has_thermal_diffusion;
+    double sum[NQ] = {};   // dvoldt, tdot, volume_n, mass, tmass
+    const int n = node_sums<SumF64, NQ, ND, STAGED>(
+        p.sup_off, p.n_lo, p.n_hi, NQ,
         [&](int q, double *t) {
             const int ent = p.sup_ent[q];
             const int e = ent >> 2, i = ent & 3;
-            if (heat) t[1] = p.hc64[(size_t)i * ne + e];
-            t[0] = p.qv[e];
+            t[1] = heat ? p.hc64[(size_t)i * ne + e] : 0.0;
+            if constexpr (MASS) {
+                const double4 r = p.ndpk[e];   // qv, vol, me, tme
+                t[0] = r.x;
+                t[2] = r.y;
+                t[3] = r.z;
+                t[4] = r.w;
+            } else {
+                t[0] = p.qv[e];
+            }
         },
         FromZero<SumF64>(), sum);
     if (n < 0) return;
-    p.ntmp[n] = sum[0] / p.vol_n[n];
+    double vol_n, tmass = 0;
+    if constexpr (MASS) {
+        vol_n = sum[2];
+        tmass = thermal ? sum[4] : 0.0;
+        p.vol_n[n] = vol_n;
+        p.mass[n] = sum[3];
+        p.tmass[n] = tmass;
+    } else {
+        vol_n = p.vol_n[n];
+        if (heat) tmass = p.tmass[n];
+    }
+    p.ntmp[n] = sum[0] / vol_n;
     if (heat) {   // temperature update + Dirichlet BC (fields.cxx:151-162)
         const double tdot = sum[1];
         p.tdot[n] = tdot;
         const unsigned flag = p.bcflag[n];
         if (flag & BOUNDZ1) p.T[n] = p.prm.surface_temperature;
         else if ((flag & BOUNDZ0) && !p.prm.has_fixed_bottom_temperature) p.T[n] = p.prm.mantle_temperature;
-        else p.T[n] -= tdot * p.clk->dt / p.tmass[n];
+        else p.T[n] -= tdot * p.clk->dt / tmass;
     }
 }
 
@@ -843,16 +890,51 @@ __device__ __forceinline__ void warp_block_min(unsigned long long val, unsigned 
     if ((threadIdx.x & 31) == 0) atomicMin(target, val);
 }
 
-// The element geometry pass.  AHEAD (3D mixed contexts, the chained step's
-// look-ahead): with the shape-function pairs still in registers and the
-// velocities as the pairs the force pass stored (KP::vdw), it also does the
-// next step's element pass (strain rate, dvoldt and heat terms) -- the next
-// step reads the same velocities, shape functions, volume and temperature,
-// none of which changes in between -- so the pairs are not read back and one
-// pass over the elements is saved.  What the next node pass gathers per
-// support entry (dvoldt term, volume, mass and tmass terms) goes into one
-// record per element (KP::ndpk) instead of four arrays.
-template <int ND, bool AHEAD>
+// compute_dt final combination (geometry.cxx:294-309), one thread; the
+// accumulators are read past the L1
+template <int ND>
+__device__ __forceinline__ void dt_finalize(const KP &p)
+{
+    Clock *ck = p.clk;
+    double dt;
+    if (p.prm.fixed_dt != 0) {
+        dt = p.prm.fixed_dt;
+    } else {
+        const unsigned long long minh = __ldcg(&ck->red_minh), maxwell = __ldcg(&ck->red_maxwell);
+        double minl = bitsd(minh);
+        const bool any = minh != ~0ull;
+        if (!any) minl = DBL_MAX;
+        double dt_maxwell;
+        if (uniform_maxwell_time(p)) dt_maxwell = any ? 0.5 * p.mat.visc_min / (1e-40 + m_shearm(p, 0)) : DBL_MAX;
+        else dt_maxwell = maxwell == ~0ull ? DBL_MAX : bitsd(maxwell);
+        double dt_diffusion = (any && p.prm.has_thermal_diffusion) ? 0.5 * minl * minl / p.mat.therm_diff_max : DBL_MAX;
+        double dt_advection = 0.5 * minl / p.prm.max_vbc_val;
+        double dt_elastic = p.prm.is_quasi_static
+            ? 0.5 * minl / (p.prm.max_vbc_val * p.prm.inertial_scaling)
+            : 0.5 * minl / sqrt(m_bulkm(p, 0) / m_rho<ND>(p, 0));
+        dt = dmin_(dmin_(dt_elastic, dt_maxwell), dmin_(dt_advection, dt_diffusion)) * p.prm.dt_fraction;
+        ck->last_dt_terms[0] = dt_maxwell;
+        ck->last_dt_terms[1] = dt_diffusion;
+        ck->last_dt_terms[2] = dt_advection;
+        ck->last_dt_terms[3] = dt_elastic;
+        if (dt <= 0) atomicOr(p.err, 0x100u);   // reported as DES_ERUNTIME
+    }
+    ck->dt = dt;
+    ck->red_minh = ck->red_maxwell = ck->red_diffusion = ~0ull;
+}
+
+// The element geometry pass.  MIXED: a 3D mixed context's form (FP64 volume,
+// double-word shape functions, FP32 rotation increments).  AHEAD (the chained
+// step's look-ahead): with the shape functions and velocities still in
+// registers it also does the next step's element pass (strain rate, dvoldt
+// and heat terms) -- the next step reads the same velocities, shape functions,
+// volume and temperature, none of which changes in between -- so they are not
+// read back and one pass over the elements is saved.  A mixed context reads
+// the velocities as the pairs the force pass stored (KP::vdw).  What the next
+// node pass gathers per support entry (dvoldt term, volume, mass and tmass
+// terms) goes into one record per element (KP::ndpk) instead of four arrays.
+// GEO_DT_FINAL: where compute_dt is due, the last block to finish forms dt.
+template <int ND, bool MIXED, bool AHEAD>
 __device__ __forceinline__ void geometry_body(const KP &p, int flags)
 {
     constexpr int NSTR = ND * (ND + 1) / 2;
@@ -862,6 +944,7 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
     const size_t ne = p.ne;
     bool do_dt = (flags & GEO_DT) != 0;
     if (flags & GEO_DT_IF_STEP) do_dt = do_dt && (p.clk->steps % 10 == 0);
+    const bool finish_dt = do_dt && (flags & GEO_DT_FINAL);
     do_dt = do_dt && p.prm.fixed_dt == 0;
     unsigned long long b_minh = ~0ull, b_maxwell = ~0ull;
     if (in) {
@@ -875,7 +958,7 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
         double vol;
         TetEdges te{};
         // a mixed context's 3D geometry works from the edges at node 0
-        const bool rel0 = ND == 3 && p.shpdw != nullptr;
+        constexpr bool rel0 = MIXED;
         RelEdges re{};
         if (rel0 && (flags & (GEO_VOLUME | GEO_SHAPE))) re = rel_edges(c[0], c[1], c[2], c[NPE - 1]);
         else if (ND == 3 && (flags & (GEO_VOLUME | GEO_SHAPE))) te = tet_edges(c[0], c[1], c[2], c[NPE - 1]);
@@ -917,17 +1000,17 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
                 minh = 2 * vol / maxl;
             }
             b_minh = dbits(minh);
-            // uniform, the Maxwell time is formed once by k_dt_finalize
+            // uniform, the Maxwell time is formed once by dt_finalize
             if (!uniform_maxwell_time(p)) b_maxwell = dbits(0.5 * p.mat.visc_min / (1e-40 + m_shearm(p, e)));
             // the diffusion time 0.5 minh^2 / kappa is non-decreasing in minh,
-            // so its minimum over the elements is k_dt_finalize's 0.5 min(minh)^2 / kappa
+            // so its minimum over the elements is dt_finalize's 0.5 min(minh)^2 / kappa
         }
         double shp[ND][NPE];
         float s32[ND][NPE];   // a mixed context's FP32 shape functions (its rotation's)
         dw sdw[3][4];         // a mixed context's shape-function pairs
         if (flags & GEO_SHAPE) {
             if constexpr (ND == 3) {
-                if (rel0) {   // the mixed context: double-word pairs (their high parts are the FP32 values)
+                if constexpr (rel0) {   // the mixed context: double-word pairs (their high parts are the FP32 values)
                     rel_shape_fn_dw(re, c1, vol, sdw);
 #pragma unroll
                     for (int k = 0; k < 3; ++k)
@@ -964,7 +1047,7 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
         // stored (KP::vdw), the other passes split the velocities
         dw vd[NPE][3];
         float w3 = 0, w4 = 0, w5 = 0;   // a mixed context's spin
-        if (rel0 && ((flags & GEO_ROTATE) || AHEAD)) {
+        if constexpr (rel0) if ((flags & GEO_ROTATE) || AHEAD) {
 #pragma unroll
             for (int i = 0; i < NPE; ++i) {
                 if constexpr (AHEAD) {
@@ -978,7 +1061,7 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
                 }
             }
         }
-        if ((flags & GEO_ROTATE) && rel0) {
+        if constexpr (rel0) if (flags & GEO_ROTATE) {
             // mixed step: spin from FP32 velocity differences (the pairs'
             // high parts, the nearest floats), FP32 Jaumann increments added
             // to the FP64 stress and strain.  Rounding the velocities to FP32
@@ -997,7 +1080,7 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
             }
         }
         double qv_next = 0;   // the look-ahead: the next step's dvoldt term
-        if constexpr (AHEAD && ND == 3) {   // the next step's element pass (k_elem_pass_mixed3's arithmetic)
+        if constexpr (AHEAD && MIXED) {   // the next step's element pass (k_elem_pass_mixed3's arithmetic)
             float2 h[3][3];
 #pragma unroll
             for (int k = 0; k < 3; ++k)
@@ -1008,6 +1091,21 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
 #pragma unroll
             for (int cc = 0; cc < 6; ++cc) p.srate[cc * ne + e] = sr[cc];
             qv_next = elem_terms_mixed(p, e, sr, vol, s32, p.prm.has_thermal_diffusion != 0, false);
+        }
+        // the FP64 context's node velocities, and the look-ahead's element pass (k_elem_pass's arithmetic)
+        double v[NPE][ND];
+        if constexpr (!MIXED) {
+            if ((flags & GEO_ROTATE) || AHEAD) {
+#pragma unroll
+                for (int i = 0; i < NPE; ++i) load_node_v<ND>(p, nodes[i], v[i]);
+            }
+            if constexpr (AHEAD) {
+                double sr[NSTR];
+                strain_rate_vals<ND>(v, shp[0], shp[1], shp[ND - 1], sr);
+#pragma unroll
+                for (int cc = 0; cc < NSTR; ++cc) p.srate[cc * ne + e] = sr[cc];
+                qv_next = elem_terms<ND>(p, e, sr, vol, shp[0], shp[1], shp[ND - 1], p.prm.has_thermal_diffusion != 0);
+            }
         }
         if ((flags & GEO_ROTATE) && rel0) {
             const float dtf = f32_of(p.clk->dt);
@@ -1035,9 +1133,6 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
                 for (int cc = 0; cc < 6; ++cc) arr[a][cc * ne + e] = S[cc] + f64_of(dtf * si[cc]);
             }
         } else if (flags & GEO_ROTATE) {
-            double v[NPE][ND];
-#pragma unroll
-            for (int i = 0; i < NPE; ++i) load_node_v<ND>(p, nodes[i], v[i]);
             const double dt = p.clk->dt;
             double s[NSTR], es[NSTR];
 #pragma unroll
@@ -1100,52 +1195,39 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
         warp_block_min<ND>(b_minh, &p.clk->red_minh);
         if (!uniform_maxwell_time(p)) warp_block_min<ND>(b_maxwell, &p.clk->red_maxwell);
     }
+    if (finish_dt) {   // uniform: the block that counts last forms dt, which every other block has used by then
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(&p.clk->blocks_done, 1u) == gridDim.x - 1) {
+                __threadfence();
+                p.clk->blocks_done = 0;
+                dt_finalize<ND>(p);
+            }
+        }
+    }
 }
 
 // three blocks of 256 per SM (80 registers, ~150 bytes of spills to L1):
 // 24 warps hide the node gathers' latency better than 16 with 128 registers
 // (mixed step at 998,400 tets: 23 us less per step)
-template <int ND>
-__global__ void __launch_bounds__(TPB, 3) k_geometry(KP p, int flags)
+template <int ND, bool MIXED>
+__global__ void __launch_bounds__(128, MIXED ? 8 : 6) k_geometry(KP p, int flags)
 {
-    geometry_body<ND, false>(p, flags);
+    geometry_body<ND, MIXED, false>(p, flags);
 }
 
-__global__ void __launch_bounds__(TPB, 3) k_geometry_ahead3(KP p, int flags)
+template <int ND, bool MIXED>
+__global__ void __launch_bounds__(128, MIXED ? 8 : 4) k_geometry_ahead(KP p, int flags)
 {
-    geometry_body<3, true>(p, flags);
+    geometry_body<ND, MIXED, true>(p, flags);
 }
 
-// compute_dt final combination (geometry.cxx:294-309), single thread
 template <int ND>
 __global__ void k_dt_finalize(KP p, int only_on_step)
 {
-    Clock *ck = p.clk;
-    if (only_on_step && ck->steps % 10 != 0) return;
-    double dt;
-    if (p.prm.fixed_dt != 0) {
-        dt = p.prm.fixed_dt;
-    } else {
-        double minl = bitsd(ck->red_minh);
-        const bool any = ck->red_minh != ~0ull;
-        if (!any) minl = DBL_MAX;
-        double dt_maxwell;
-        if (uniform_maxwell_time(p)) dt_maxwell = any ? 0.5 * p.mat.visc_min / (1e-40 + m_shearm(p, 0)) : DBL_MAX;
-        else dt_maxwell = ck->red_maxwell == ~0ull ? DBL_MAX : bitsd(ck->red_maxwell);
-        double dt_diffusion = (any && p.prm.has_thermal_diffusion) ? 0.5 * minl * minl / p.mat.therm_diff_max : DBL_MAX;
-        double dt_advection = 0.5 * minl / p.prm.max_vbc_val;
-        double dt_elastic = p.prm.is_quasi_static
-            ? 0.5 * minl / (p.prm.max_vbc_val * p.prm.inertial_scaling)
-            : 0.5 * minl / sqrt(m_bulkm(p, 0) / m_rho<ND>(p, 0));
-        dt = dmin_(dmin_(dt_elastic, dt_maxwell), dmin_(dt_advection, dt_diffusion)) * p.prm.dt_fraction;
-        ck->last_dt_terms[0] = dt_maxwell;
-        ck->last_dt_terms[1] = dt_diffusion;
-        ck->last_dt_terms[2] = dt_advection;
-        ck->last_dt_terms[3] = dt_elastic;
-        if (dt <= 0) atomicOr(p.err, 0x100u);   // reported as DES_ERUNTIME
-    }
-    ck->dt = dt;
-    ck->red_minh = ck->red_maxwell = ck->red_diffusion = ~0ull;
+    if (only_on_step && p.clk->steps % 10 != 0) return;
+    dt_finalize<ND>(p);
 }
 
 __global__ void k_dt_reset(KP p)
@@ -1449,10 +1531,13 @@ int launch_elem_pass(const KP &p, cudaStream_t s, bool heat)
     return 1;
 }
 
-int launch_node_pass(const KP &p, cudaStream_t s, bool heat)
+int launch_node_pass(const KP &p, cudaStream_t s, bool heat, bool mass_sums)
 {
-    if (p.nd == 3) DES_NODES((k_node_pass<3, STAGED>), p.n_hi - p.n_lo, s, p, (int)heat);
-    else DES_NODES((k_node_pass<2, STAGED>), p.n_hi - p.n_lo, s, p, (int)heat);
+    const int n = p.n_hi - p.n_lo;
+    if (p.nd == 3 && mass_sums) DES_NODES((k_node_pass<3, true, STAGED>), n, s, p, (int)heat);
+    else if (p.nd == 3) DES_NODES((k_node_pass<3, false, STAGED>), n, s, p, (int)heat);
+    else if (mass_sums) DES_NODES((k_node_pass<2, true, STAGED>), n, s, p, (int)heat);
+    else DES_NODES((k_node_pass<2, false, STAGED>), n, s, p, (int)heat);
     return 1;
 }
 
@@ -1549,13 +1634,19 @@ int launch_coordinate(const KP &p, cudaStream_t s, bool contract)
 
 int launch_geometry(const KP &p, cudaStream_t s, int flags)
 {
-    DISPATCH(k_geometry, p.e_hi - p.e_lo, p, flags);
+    const int n = p.e_hi - p.e_lo;
+    if (p.nd == 3 && p.shpdw) DES_LAUNCH((k_geometry<3, true>), n, s, p, flags);
+    else if (p.nd == 3) DES_LAUNCH((k_geometry<3, false>), n, s, p, flags);
+    else DES_LAUNCH((k_geometry<2, false>), n, s, p, flags);
     return 1;
 }
 
 int launch_geometry_ahead(const KP &p, cudaStream_t s, int flags)
 {
-    DES_LAUNCH(k_geometry_ahead3, p.e_hi - p.e_lo, s, p, flags);
+    const int n = p.e_hi - p.e_lo;
+    if (p.nd == 3 && p.shpdw) DES_LAUNCH((k_geometry_ahead<3, true>), n, s, p, flags);
+    else if (p.nd == 3) DES_LAUNCH((k_geometry_ahead<3, false>), n, s, p, flags);
+    else DES_LAUNCH((k_geometry_ahead<2, false>), n, s, p, flags);
     return 1;
 }
 

@@ -43,7 +43,8 @@ enum GeoFlags : int {
     GEO_ROTATE = 8,      // rotate_stress               (fields.cxx:411-483)
     GEO_DT = 16,         // compute_dt element terms    (geometry.cxx:254-292)
     GEO_DT_IF_STEP = 32, // ... only when steps % 10 == 0 (dynearthsol.cxx:349-361)
-    GEO_MASS_TERMS = 64  // the element's mass and tmass terms -> me, tme (for launch_mass_sum)
+    GEO_MASS_TERMS = 64, // the element's mass and tmass terms -> me, tme (for launch_mass_sum)
+    GEO_DT_FINAL = 128   // with GEO_DT, in one launch over the whole mesh: form dt too (launch_dt_finalize)
 };
 
 // Each launcher returns the number of kernels it launched.
@@ -55,7 +56,9 @@ int launch_dvoldt(const KP &p, cudaStream_t s);                   // -> ntmp
 // (+ clock advance) and of the node sums + temperature update: the same bits
 // (needs p.qv and, with heat, p.hc64)
 int launch_elem_pass(const KP &p, cudaStream_t s, bool heat);
-int launch_node_pass(const KP &p, cudaStream_t s, bool heat);
+// mass_sums (a chained step): first the compute_mass sums of the look-ahead
+// geometry pass's element terms, and the clock advance
+int launch_node_pass(const KP &p, cudaStream_t s, bool heat, bool mass_sums = false);
 int launch_edvoldt(const KP &p, cudaStream_t s);
 int launch_update_stress(const KP &p, cudaStream_t s, bool fused);
 // dp_nd -> ntmp; stored: the dp vol products of the fused mixed stress pass (KP::pv)
@@ -75,8 +78,8 @@ int launch_velocity(const KP &p, cudaStream_t s, bool contract = false);
 int launch_vbcs(const KP &p, cudaStream_t s);
 int launch_coordinate(const KP &p, cudaStream_t s, bool contract = false);
 int launch_geometry(const KP &p, cudaStream_t s, int flags);
-// the chained mixed step's geometry pass (3D mixed contexts), which also
-// does the next step's element pass (k_elem_pass_mixed3's work)
+// the chained step's geometry pass, which also does the next step's element
+// pass (k_elem_pass's or k_elem_pass_mixed3's work)
 int launch_geometry_ahead(const KP &p, cudaStream_t s, int flags);
 int launch_mass(const KP &p, cudaStream_t s);
 // compute_mass from the element terms of a GEO_MASS_TERMS geometry pass (same sums, same order)

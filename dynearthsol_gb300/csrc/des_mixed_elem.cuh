@@ -1,7 +1,7 @@
 // des_mixed_elem.cuh -- the per-element work of the mixed step's element
 // pass (strain rate, dvoldt term, heat terms) on values held in registers.
 // The element pass (k_elem_pass_mixed3) loads them from memory; the
-// look-ahead geometry pass of the chained step (k_geometry_ahead3) forms the
+// look-ahead geometry pass of the chained step (k_geometry_ahead) forms the
 // shape functions itself and hands them over directly.  Both call these
 // functions, so both form the very same bits.
 #pragma once
