@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(128) k_adj_motion(KP p, AdjBufs a, TapeStep t,
                 gpre[d] = col[0] * gv[0] + col[1] * gv[1] + col[2] * gv[2];
             }
             for (int ib = 0; ib < DES_NBDRYTYPES; ++ib) {
+                if (!(flag & (1u << ib))) continue;   // the node's BCs read only its own boundaries' values
                 double col[3] = {0, 0, 0};
                 zero[ib] = 1;
                 apply_vbcs_node_va<3>(p, flag, col, zero);
@@ -1145,6 +1146,34 @@ template <bool STAGED>
 __global__ void __launch_bounds__(128) k_adj_gather_xT(KP p, AdjBufs a)
 {
     gather_slots<STAGED>(p, a, a.slotx, a.ax);
+}
+
+// several arrays in one launch, each by its share of the blocks
+__global__ void __launch_bounds__(256) k_copy_arrays(const __grid_constant__ CopyTable t)
+{
+    int k = 0;
+    while (k + 1 < t.count && blockIdx.x >= t.first[k + 1]) ++k;
+    const size_t stride = (size_t)(t.first[k + 1] - t.first[k]) * blockDim.x, n = t.n[k];
+    const double *__restrict__ src = t.src[k];
+    double *__restrict__ dst = t.dst[k];
+    for (size_t i = (size_t)(blockIdx.x - t.first[k]) * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = src[i];
+}
+
+int launch_copy_arrays(CopyTable &t, cudaStream_t s)
+{
+    if (t.count == 0) return 0;
+    // four values a thread, at most about eight blocks per SM in all
+    size_t total = 0;
+    for (int k = 0; k < t.count; ++k) total += t.n[k];
+    const size_t per_block = std::max<size_t>(1024, (total + 152 * 8 - 1) / (152 * 8));
+    unsigned b = 0;
+    for (int k = 0; k < t.count; ++k) {
+        t.first[k] = b;
+        b += (unsigned)std::max<size_t>(1, (t.n[k] + per_block - 1) / per_block);
+    }
+    t.first[t.count] = b;
+    k_copy_arrays<<<b, 256, 0, s>>>(t);
+    return 1;
 }
 
 int launch_adj_stress(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,

@@ -58,6 +58,24 @@ struct AdjBufs {
     double *gvbc;                    // [nblk][DES_NBDRYTYPES] partial sums of a block or warp of nodes
 };
 
+// Device-to-device copies of FP64 arrays in one launch: the dozen arrays of a
+// tape record cost a few microseconds each as separate copies.
+constexpr int COPY_MAX = 14;
+struct CopyTable {
+    const double *src[COPY_MAX];
+    double *dst[COPY_MAX];
+    size_t n[COPY_MAX];
+    unsigned first[COPY_MAX + 1];   // first block of each array, filled by the launch
+    int count = 0;
+    void add(double *d, const double *s, size_t len)
+    {
+        dst[count] = d;
+        src[count] = s;
+        n[count++] = len;
+    }
+};
+int launch_copy_arrays(CopyTable &t, cudaStream_t s);
+
 // adjoint-state kernels of one step, launched in this order by the host
 int launch_adj_end_geometry(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
                             cudaStream_t s);

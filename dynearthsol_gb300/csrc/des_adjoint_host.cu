@@ -80,19 +80,26 @@ StateRef tape_state(const TapeStep &t)
     return StateRef{t.x, t.v, t.T, t.s, t.pls, t.volo, t.vol, t.shp, t.mass, t.tmass, t.voln};
 }
 
-cudaError_t copy_state(const StateRef &dst, const StateRef &src, size_t nn, size_t ne, cudaStream_t s)
+void add_copies(CopyTable &t, const StateRef &dst, const StateRef &src, size_t nn, size_t ne)
 {
-    const size_t D = sizeof(double);
-    const std::pair<std::pair<double *, const double *>, size_t> f[] = {
-        {{dst.x, src.x}, 3 * nn}, {{dst.v, src.v}, 3 * nn},     {{dst.T, src.T}, nn},
-        {{dst.s, src.s}, 6 * ne}, {{dst.pls, src.pls}, ne},     {{dst.volo, src.volo}, ne},
-        {{dst.vol, src.vol}, ne}, {{dst.shp, src.shp}, 12 * ne}, {{dst.mass, src.mass}, nn},
-        {{dst.tmass, src.tmass}, nn}, {{dst.voln, src.voln}, nn}};
-    for (auto &e : f) {
-        cudaError_t r = cudaMemcpyAsync(e.first.first, e.first.second, e.second * D, cudaMemcpyDeviceToDevice, s);
-        if (r != cudaSuccess) return r;
-    }
-    return cudaSuccess;
+    t.add(dst.x, src.x, 3 * nn);
+    t.add(dst.v, src.v, 3 * nn);
+    t.add(dst.T, src.T, nn);
+    t.add(dst.s, src.s, 6 * ne);
+    t.add(dst.pls, src.pls, ne);
+    t.add(dst.volo, src.volo, ne);
+    t.add(dst.vol, src.vol, ne);
+    t.add(dst.shp, src.shp, 12 * ne);
+    t.add(dst.mass, src.mass, nn);
+    t.add(dst.tmass, src.tmass, nn);
+    t.add(dst.voln, src.voln, nn);
+}
+
+int copy_state(const StateRef &dst, const StateRef &src, size_t nn, size_t ne, cudaStream_t s)
+{
+    CopyTable t;
+    add_copies(t, dst, src, nn, ne);
+    return launch_copy_arrays(t, s);
 }
 
 }  // namespace
@@ -265,39 +272,44 @@ int adj_step(des_ctx *c, const TapeStep *t)
         p.tape_evp = t->evp;
     }
     cudaStream_t s = c->stream;
-    const size_t nn = c->nn, ne = c->ne, D = sizeof(double);
-    auto cp = [&](double *dst, const double *src, size_t n) {
-        return cudaMemcpyAsync(dst, src, n * D, cudaMemcpyDeviceToDevice, s);
-    };
-    int n = 0;
-    if (t) CKA(copy_state(tape_state(*t), live_state(c), nn, ne, s));
-    // strain rate, heat and dvoldt as the fused FP64 step forms them
+    const size_t nn = c->nn, ne = c->ne;
     const bool thermal = p.prm.has_thermal_diffusion != 0;
+    int n = 0;
+    if (t) n += copy_state(tape_state(*t), live_state(c), nn, ne, s);
+    // strain rate, heat and dvoldt as the fused FP64 step forms them
     n += launch_elem_pass(p, s, thermal);
-    if (t) CKA(cp(t->edot, p.srate, 6 * ne));
     n += launch_node_pass(p, s, thermal);
-    if (t) {
-        if (thermal) CKA(cp(t->tdot, p.tdot, nn));
-        CKA(cp(t->ntmp, p.ntmp, nn));
+    if (t) {   // the stress pass corrects the strain rate and the NMD gather reuses ntmp
+        CopyTable ct;
+        ct.add(t->edot, p.srate, 6 * ne);
+        ct.add(t->ntmp, p.ntmp, nn);
+        if (thermal) ct.add(t->tdot, p.tdot, nn);
+        n += launch_copy_arrays(ct, s);
     }
     n += launch_update_stress(p, s, true);
-    if (t) {
-        CKA(cp(t->sstar, p.stress, 6 * ne));
-        CKA(cp(t->dp, p.dp, ne));
-        CKA(cp(t->rho, p.rho_e, ne));
-        CKA(cp(t->edv, p.edvoldt, ne));
-    }
     n += launch_nmd_gather(p, s);
-    if (t) CKA(cp(t->dpn, p.ntmp, nn));
+    if (t) {   // the stress after update_stress, before the NMD correction; dpn is final
+        CopyTable ct;
+        ct.add(t->sstar, p.stress, 6 * ne);
+        ct.add(t->dp, p.dp, ne);
+        ct.add(t->rho, p.rho_e, ne);
+        ct.add(t->edv, p.edvoldt, ne);
+        ct.add(t->dpn, p.ntmp, nn);
+        n += launch_copy_arrays(ct, s);
+    }
     n += launch_nmd_correct(p, s, true);
     n += launch_force(p, s, true);
-    if (t) CKA(cp(t->f, p.f, 3 * nn));
     // mass from the geometry pass's element terms: the same sums, in the same
     // order, as compute_mass's node gather (launch_mass), at a fifth of its cost
     int geo = GEO_COPY_OLD | GEO_VOLUME | GEO_SHAPE | GEO_MASS_TERMS;
     if (p.mat.rheol_type & DES_RH_ELASTIC) geo |= GEO_ROTATE;
     n += launch_geometry(p, s, geo);
     n += launch_mass_sum(p, s);
+    if (t) {
+        CopyTable ct;
+        ct.add(t->f, p.f, 3 * nn);
+        n += launch_copy_arrays(ct, s);
+    }
     return ctx_check_launch(c, n);
 }
 
@@ -371,10 +383,11 @@ int des_adjoint_forward(des_ctx *c, int nsteps, int checkpoint_every)
     CKA(cudaStreamSynchronize(c->stream));
     w->dt = clk.dt;
     for (int k = 0; k < nsteps; ++k) {
-        if (k % C == 0) CKA(copy_state(w->ck[k / C], live_state(c), nn, ne, c->stream));
+        if (k % C == 0 && (rc = ctx_check_launch(c, copy_state(w->ck[k / C], live_state(c), nn, ne, c->stream)))) return rc;
         if ((rc = adj_step(c, k >= last0 ? &w->tape[k - last0] : nullptr))) return rc;
     }
-    CKA(copy_state(tape_state(w->tape[nsteps - last0]), live_state(c), nn, ne, c->stream));
+    if ((rc = ctx_check_launch(c, copy_state(tape_state(w->tape[nsteps - last0]), live_state(c), nn, ne, c->stream))))
+        return rc;
     CKA(cudaMemcpyAsync(w->final_pool, c->pool, c->pool_bytes, cudaMemcpyDeviceToDevice, c->stream));
     w->K = nsteps;
     w->C = C;
@@ -410,10 +423,10 @@ int des_adjoint_backward(des_ctx *c, const des_host_state *seed, des_host_state 
         const int k0 = seg * w->C, L = std::min(w->C, w->K - k0);
         if (w->tape_seg != seg) {   // recompute the segment from its checkpoint onto the tape
             w->tape_seg = -1;
-            CKA(copy_state(live_state(c), w->ck[seg], nn, ne, s));
+            if ((rc = ctx_check_launch(c, copy_state(live_state(c), w->ck[seg], nn, ne, s)))) return rc;
             for (int j = 0; j < L; ++j)
                 if ((rc = adj_step(c, &w->tape[j]))) return rc;
-            CKA(copy_state(tape_state(w->tape[L]), live_state(c), nn, ne, s));
+            if ((rc = ctx_check_launch(c, copy_state(tape_state(w->tape[L]), live_state(c), nn, ne, s)))) return rc;
             w->tape_seg = seg;
         }
         for (int j = L - 1; j >= 0; --j)
