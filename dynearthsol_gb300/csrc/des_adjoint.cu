@@ -230,7 +230,7 @@ __device__ __forceinline__ double damp_deriv(const KP &p, double f, double v)
 // avn, and adds the sums of the prescribed-value adjoints to gvbc.
 // ------------------------------------------------------------------
 template <bool STAGED>
-__global__ void __launch_bounds__(128) k_adj_motion(KP p, AdjBufs a, TapeStep t, TapeStep t1, double dt)
+__global__ void __launch_bounds__(192) k_adj_motion(KP p, AdjBufs a, TapeStep t, TapeStep t1, double dt)
 {
     const size_t ne = p.ne, nn = p.nn;
     double sum[6] = {};   // coordinate and velocity contributions
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(TPB_A) k_adj_force(KP p, AdjBufs a, TapeStep t
 // nodes: NMD nodal sum reversed (dpn = sum_e dp_e vol_e / volume_n), and the
 // facets' coordinate adjoints added to ax
 template <bool STAGED>
-__global__ void __launch_bounds__(128) k_adj_nmd_nodes(KP p, AdjBufs a, TapeStep t)
+__global__ void __launch_bounds__(192) k_adj_nmd_nodes(KP p, AdjBufs a, TapeStep t)
 {
     const size_t nn = p.nn, nbf = p.nbf;
     double acc;
@@ -947,7 +947,7 @@ __global__ void __launch_bounds__(TPB_A) k_adj_stress(KP p, AdjBufs a, TapeStep 
 // mean of ntmp), and the temperature update with its Dirichlet BCs
 // (fields.cxx:151-162): T' = T - tdot dt / tmass
 template <bool STAGED>
-__global__ void __launch_bounds__(128) k_adj_nodes_heat(KP p, AdjBufs a, TapeStep t, TapeStep t1, double dt)
+__global__ void __launch_bounds__(192) k_adj_nodes_heat(KP p, AdjBufs a, TapeStep t, TapeStep t1, double dt)
 {
     const size_t ne = p.ne;
     double sum[2];   // adjoints of the updated temperature and of dvoldt
@@ -1096,7 +1096,7 @@ __device__ __forceinline__ void gather_slots(const KP &p, const AdjBufs &a, cons
 
 // nodes: add the element contributions to the velocity and temperature adjoints
 template <bool STAGED>
-__global__ void __launch_bounds__(128) k_adj_gather_vT(KP p, AdjBufs a)
+__global__ void __launch_bounds__(192) k_adj_gather_vT(KP p, AdjBufs a)
 {
     gather_slots<STAGED>(p, a, a.slot3, a.av);
 }
@@ -1143,7 +1143,7 @@ __global__ void __launch_bounds__(TPB_A) k_adj_start_geometry(KP p, AdjBufs a, T
 }
 
 template <bool STAGED>
-__global__ void __launch_bounds__(128) k_adj_gather_xT(KP p, AdjBufs a)
+__global__ void __launch_bounds__(192) k_adj_gather_xT(KP p, AdjBufs a)
 {
     gather_slots<STAGED>(p, a, a.slotx, a.ax);
 }

@@ -22,9 +22,15 @@
 
 namespace des {
 
-constexpr int NPB = 8, STAGED_THREADS = 96;
+constexpr int NPB = 8, STAGED_THREADS = 192;
 
-// n: nodes of the launch.  Measured (us, walk / staged, warm):
+// n: nodes of the launch.  Measured (walk / staged): on 177,147 nodes the
+// node pass takes 46 / 74 us, the force 55 / 64 us and the reverse node pass
+// 108 / 225 us; on 22,344 nodes a pass through the per-function entry points
+// takes 4.51 / 4.18 ms.  The line lies between, where a walk would put eight
+// warps on each SM, too few to hide its chain of loads.  192 threads take
+// the entries of 8 nodes (~24 each) in one chunk: 100 steps of a 648-tet mesh,
+// with the state's copies, 5.83 ms, 5.98 ms with 96 threads.
 inline bool node_staged(long long n) { return n <= 152LL * 256; }
 
 // The sums' arithmetic: a quantity's term, state, addition and value.

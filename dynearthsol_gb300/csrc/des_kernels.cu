@@ -130,7 +130,7 @@ __device__ __forceinline__ double heat_term(const KP &p, int e, int i)
 }
 
 template <int ND, bool HEAT, bool DVOLDT, bool STAGED>
-__global__ void __launch_bounds__(128) k_node_gather1(KP p)
+__global__ void __launch_bounds__(192) k_node_gather1(KP p)
 {
     constexpr int NQ = (int)HEAT + (int)DVOLDT;
     double sum[NQ];
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(TPB) k_elem_pass(KP p, int heat)
 // from the records of the look-ahead geometry pass (KP::ndpk), as k_mass_sum
 // forms them, and the step's clock is started here.
 template <int ND, bool MASS, bool STAGED>
-__global__ void __launch_bounds__(128) k_node_pass(KP p, int heat)
+__global__ void __launch_bounds__(192) k_node_pass(KP p, int heat)
 {
     if (MASS && blockIdx.x == 0 && threadIdx.x == 0) {   // dynearthsol.cxx:325-326
         p.clk->steps += 1;
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(TPB) k_update_stress(KP p, int fused)
 // (KP::pv), the same dw_mul of the same pairs, instead of forming them for
 // each support entry
 template <int ND, bool DW, bool STAGED>
-__global__ void __launch_bounds__(128) k_nmd_gather(KP p, int stored)
+__global__ void __launch_bounds__(192) k_nmd_gather(KP p, int stored)
 {
     double sum;
     int n;
@@ -598,7 +598,7 @@ __device__ __forceinline__ void force_tail(const KP &p, int n, double *f, int fu
 // The FP64 step's force: each support entry's term -(sigma . dN_i/dx + rho g
 // / NPE z) vol, the expression the reference subtracts; then the FP64 tail.
 template <int ND, bool STAGED>
-__global__ void __launch_bounds__(128) k_force(KP p, int fused_motion)
+__global__ void __launch_bounds__(192) k_force(KP p, int fused_motion)
 {
     constexpr int NSTR = ND * (ND + 1) / 2;
     constexpr int NPE = ND + 1;
@@ -707,7 +707,7 @@ struct ForceTerms {   // the three components' terms of a support entry
 };
 
 template <bool STAGED>
-__global__ void __launch_bounds__(128) k_force_dw3(KP p, int fused_motion)
+__global__ void __launch_bounds__(192) k_force_dw3(KP p, int fused_motion)
 {
     double f[3];
     const int n = node_sums<SumDwAcc, 3, 3, STAGED>(p.sup_off, p.n_lo, p.n_hi, 3, ForceTerms{p.ft},
@@ -1270,7 +1270,7 @@ __device__ __forceinline__ void mass_sums(const KP &p, int lo, int hi, Terms ter
 }
 
 template <int ND, bool DW, bool STAGED>
-__global__ void __launch_bounds__(128) k_mass(KP p)
+__global__ void __launch_bounds__(192) k_mass(KP p)
 {
     constexpr int NPE = ND + 1;
     const double pseudo_speed = p.prm.max_vbc_val * p.prm.inertial_scaling;
@@ -1290,7 +1290,7 @@ __global__ void __launch_bounds__(128) k_mass(KP p)
 // the node sums of compute_mass from the element terms that the geometry
 // pass wrote (GEO_MASS_TERMS): per pair 3 additions instead of the terms
 template <int ND, bool DW, bool STAGED>
-__global__ void __launch_bounds__(128) k_mass_sum(KP p)
+__global__ void __launch_bounds__(192) k_mass_sum(KP p)
 {
     const bool thermal = p.prm.has_thermal_diffusion;
     mass_sums<ND, DW, STAGED>(p, p.n_lo, p.n_hi, [&](int e, double *t) {

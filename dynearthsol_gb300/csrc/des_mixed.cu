@@ -668,7 +668,7 @@ struct SumNode {
 };
 
 template <bool STAGED>
-__global__ void __launch_bounds__(128) k_heat_dvoldt_mixed3(KP p, int heat, int do_dvoldt)
+__global__ void __launch_bounds__(192) k_heat_dvoldt_mixed3(KP p, int heat, int do_dvoldt)
 {
     const bool k_const = (p.mat.nmat == 1) && !p.ef[DES_EF_THERM_COND];
     double sum[2] = {0, 0};   // dvoldt, tdot
@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(TPB_M) k_elem_pass_mixed3(KP p, int heat)
 // each moved the volumetric rate enough to change the default damping's
 // copysign at some nodes within ten steps.
 template <bool MASS, bool STAGED>
-__global__ void __launch_bounds__(128) k_node_pass_mixed3(KP p, int heat, int begin_step)
+__global__ void __launch_bounds__(192) k_node_pass_mixed3(KP p, int heat, int begin_step)
 {
     if (begin_step && blockIdx.x == 0 && threadIdx.x == 0) {   // dynearthsol.cxx:325-326
         p.clk->steps += 1;
