@@ -107,6 +107,7 @@ int set_params(des_ctx *c, const des_params *prm)
     if (prm->damping_option < 0 || prm->damping_option > 4)
         return fail_msg(c->err, DES_EINPUT, "unknown damping_option: %d", prm->damping_option);
     c->kp.prm = *prm;
+    c->kp.g4 = prm->gravity / 4;
     set_rho_pseudo(c);
     invalidate_graph(c);
     return DES_OK;
@@ -426,8 +427,7 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     }
     add((void **)&c->d_rho, (size_t)ne * D);
     add((void **)&c->d_buoy, (size_t)ne * D);
-    add((void **)&p.me, (size_t)ne * D);
-    add((void **)&p.tme, (size_t)ne * D);
+    add((void **)&p.me, (size_t)ne * 2 * D);   // me, then tme
     add((void **)&p.fv, (size_t)std::max(nbf, 1) * nd * D);
     add((void **)&p.clk, sizeof(Clock));
     add((void **)&p.err, sizeof(unsigned));
@@ -460,6 +460,7 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
             off += s.bytes;
         }
     }
+    p.tme = p.me + ne;
     p.nd = nd;
     p.npe = npe;
     p.nstr = c->nstr;
@@ -480,6 +481,7 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     p.rho_e = nullptr;
     p.buoy_e = nullptr;
     p.tdot = p.ntmp;
+    p.sh32 = mixed3 ? (float *)p.me : nullptr;
     p.shpdw = d_shpdw;
     p.vdw = d_vdw;
     p.ndpk = d_ndpk;
@@ -564,6 +566,7 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
             }
             p.mat.visc_lnmin = std::log(p.mat.visc_min);
             p.mat.visc_lnmax = std::log(p.mat.visc_max);
+            p.mat.visc_ln_pos = p.mat.visc_lnmin > 0 && p.mat.visc_lnmax > 0;
             for (int k = 0; k < 2 * nm; ++k) {
                 p.mat.pt_anphi[k] = tab[nm + 4 * k + 0];
                 p.mat.pt_anpsi[k] = tab[nm + 4 * k + 1];
@@ -1285,7 +1288,7 @@ int enqueue_step_chain(des_ctx *c, int part)
     if (part == 0) n += mixed ? launch_elem_pass_mixed(p, s, thermal) : launch_elem_pass(p, s, thermal);
     n += mixed ? launch_node_pass_mixed(p, s, thermal, part != 0, part != 0)
                : launch_node_pass(p, s, thermal, part != 0);
-    n += mixed ? launch_update_stress_mixed(p, s, true, part == 2) : launch_update_stress(p, s, true);
+    n += mixed ? launch_update_stress_mixed(p, s, true, part == 2, part != 0) : launch_update_stress(p, s, true);
     n += launch_nmd_gather(p, s, mixed);
     n += launch_nmd_correct(p, s, true);
     n += launch_force(p, s, true, mixed);

@@ -67,6 +67,7 @@ struct MatC {
     double rho_pseudo;               // bulkm / (v_max * inertial_scaling)^2 (geometry.cxx:348-349), nmat == 1
     double visc_lnc[DES_MAXMAT];     // ln(0.25e6 * visc_coef[m])   (mixed step)
     double visc_lnmin, visc_lnmax;   // ln(visc_min), ln(visc_max)  (mixed step)
+    int visc_ln_pos;                 // both are positive
     double visc_qnr[DES_MAXMAT];     // Q / (n R)                   (mixed step)
     // every material's viscosity law is positive wherever T > 0 (A > 0, Q >= 0,
     // n > 0), so a material without markers in the element adds exactly +0
@@ -108,6 +109,7 @@ struct KP {
     // element fields
     double *stress, *strain, *srate, *pls, *dpls, *syy, *dp, *edvoldt, *vol, *vol_old, *shp;
     double *rho_e;                       // per-element density of the step (scratch), or null
+    double g4;                           // gravity / 4 (an exact scaling)
     double *buoy_e;                      // per-element rho g / NPE of the step (scratch), or null
     double *tdot;                        // node scratch for the heat gather (ntmp outside the fused step)
     double *fv;                          // [nd][nbf] per-facet stress-BC force (scratch)
@@ -117,6 +119,7 @@ struct KP {
     // shp, which downloads fill from them on demand.
     float2 *shpdw;
     float2 *vdw;                         // [3][nn] a mixed context's velocities as double-word pairs, from the force pass
+    float *sh32;                         // [3][ne] a chained mixed step's shear strain rates, FP32 values (in me, idle then)
     double4 *ndpk;                       // [ne] {qv, vol, me, tme} from the chained step's look-ahead geometry pass
     float2 *pv;                          // [ne] a mixed context's double-word dp vol, from the fused stress pass
     float *hc;                           // [4][ne] per-element heat terms of the mixed step, or null
@@ -199,6 +202,28 @@ __device__ __forceinline__ double div6(double x)
     const unsigned e = biased_exponent(x);
     if (e < 123u || e == 0x7ffu) return div6_slow(x);
     return div3(__hiloint2double(__double2hiint(x) - (1 << 20), __double2loint(x)));
+}
+
+// x / 2^K, K = 1 or 2, exactly: the exponent field less K in the normal range,
+// by integer instructions, which issue beside the FP64 work; zeros, results
+// below the normal range, infinities and NaN are multiplied (out of line, as
+// div3_slow).
+static __device__ __noinline__ double scale_slow(double x, double f) { return x * f; }
+
+template <int K>
+__device__ __forceinline__ double over_pow2(double x)
+{
+    const unsigned e = biased_exponent(x);
+    if (e - (K + 1u) >= 0x7ffu - (K + 1u)) return scale_slow(x, K == 1 ? 0.5 : 0.25);
+    return __hiloint2double(__double2hiint(x) - (K << 20), __double2loint(x));
+}
+
+// x / NPE of an element's node mean
+template <int NPE>
+__device__ __forceinline__ double node_mean(double sum)
+{
+    if (NPE == 4) return over_pow2<2>(sum);
+    return sum / NPE;
 }
 
 // x / ND for ND = 2 or 3, bit-identical to the division
@@ -348,7 +373,7 @@ __device__ __forceinline__ double elem_avg_T(const KP &p, int e)
     double t = p.T[p.conn[e]];
 #pragma unroll
     for (int i = 1; i < NPE; ++i) t += p.T[p.conn[(size_t)i * p.ne + e]];
-    return t / NPE;
+    return node_mean<NPE>(t);
 }
 
 // MatProps::rho (matprops.cxx:376-397) given the element's mean temperature
@@ -562,7 +587,9 @@ struct ScreenTerms {
 // angle terms (MatC) and one product or quotient of the cohesion, a few ulps.
 __device__ __forceinline__ ScreenTerms screen_terms_table(const KP &p, int e, int m, double pls)
 {
-    const int k = (pls < p.mat.pls0[m] || pls == p.mat.pls0[m]) ? 2 * m : 2 * m + 1;
+    // +0 at pls0 = 0, the state of nearly all elements, without FP64 compares
+    const bool start = __double_as_longlong(pls) == __double_as_longlong(p.mat.pls0[m]);
+    const int k = (start || pls < p.mat.pls0[m] || pls == p.mat.pls0[m]) ? 2 * m : 2 * m + 1;
     const double *ef = p.ef[(k & 1) ? DES_EF_COHESION1 : DES_EF_COHESION0];
     const float c = f32_of(ef ? ef[e] : (k & 1) ? p.mat.cohesion1[m] : p.mat.cohesion0[m]);
     return {p.mat.pt_anphi_f[k], 2.0f * c * p.mat.pt_sqrt_anphi_f[k],
@@ -612,7 +639,8 @@ static __device__ __noinline__ ScreenTerms screen_terms_any(const KP &p, int e, 
 __device__ __forceinline__ ScreenTerms screen_terms(const KP &p, int e, double pls)
 {
     if (p.mat.nmat == 1 && !p.emark && !p.ef[DES_EF_FRICTION0] && !p.ef[DES_EF_FRICTION1]
-        && !(pls > p.mat.pls0[0] && pls < p.mat.pls1[0]))
+        && (__double_as_longlong(pls) == __double_as_longlong(p.mat.pls0[0])
+            || !(pls > p.mat.pls0[0] && pls < p.mat.pls1[0])))
         return screen_terms_table(p, e, 0, pls);
     return screen_terms_any(p, e, pls);
 }

@@ -53,7 +53,7 @@ __device__ __forceinline__ void strain_rate_vals(const double (*v)[ND], const do
         double t = v[0][d] * sk[0] + v[0][k] * sd[0];
 #pragma unroll
         for (int i = 1; i < NPE; ++i) t += v[i][d] * sk[i] + v[i][k] * sd[i];
-        return 0.5 * t;
+        return over_pow2<1>(t);
     };
     s[0] = normal(0, sx);
     if (ND == 3) {
@@ -313,10 +313,10 @@ __global__ void __launch_bounds__(TPB) k_update_stress(KP p, int fused)
     double edv;
     if (fused) {
         // compute_edvoldt fused in: dvoldt of the step is in ntmp
-        double dj = 0;
+        double dj = p.ntmp[conn_at(p, 0, e)];
 #pragma unroll
-        for (int i = 0; i < ND + 1; ++i) dj += p.ntmp[conn_at(p, i, e)];
-        edv = dj / (ND + 1);
+        for (int i = 1; i < ND + 1; ++i) dj += p.ntmp[conn_at(p, i, e)];
+        edv = node_mean<ND + 1>(dj);
         p.edvoldt[e] = edv;
     } else {
         edv = p.edvoldt[e];
@@ -451,13 +451,12 @@ __global__ void __launch_bounds__(TPB) k_nmd_correct(KP p, int with_facets)
     const int t = blockIdx.x * blockDim.x + threadIdx.x, nel = p.e_hi - p.e_lo;
     if (t < nel) {
         const int e = p.e_lo + t;
-        double dpn = 0;
+        double dpn = p.ntmp[conn_at(p, 0, e)];
 #pragma unroll
-        for (int i = 0; i < ND + 1; ++i) dpn += p.ntmp[conn_at(p, i, e)];
-        double dp_el = dpn / (ND + 1);
-        double dp_orig = p.dp[e];
+        for (int i = 1; i < ND + 1; ++i) dpn += p.ntmp[conn_at(p, i, e)];
+        const double corr = divnd<ND>(-p.dp[e] + node_mean<ND + 1>(dpn));
 #pragma unroll
-        for (int i = 0; i < ND; ++i) p.stress[(size_t)i * p.ne + e] += divnd<ND>(-dp_orig + dp_el);
+        for (int i = 0; i < ND; ++i) p.stress[(size_t)i * p.ne + e] += corr;
     } else if (with_facets && t < nel + (p.f_hi - p.f_lo)) {
         const int i = p.f_lo + (t - nel);
         facet_force<ND>(p, p.fac_order ? p.fac_order[i] : i);
@@ -479,13 +478,8 @@ __global__ void __launch_bounds__(TPB) k_nmd_correct(KP p, int with_facets)
 __device__ __forceinline__ void force_terms_dw3(const KP &p, int e, const double *s)
 {
     const size_t ne = p.ne;
-    double buoy = 0;
-    if (p.buoy_e) {
-        buoy = p.buoy_e[e];
-    } else if (p.prm.gravity != 0) {
-        const double rho = p.rho_e ? p.rho_e[e] : m_rho<3>(p, e);
-        buoy = rho * p.prm.gravity / 4;
-    }
+    // rho g / 4 (the division by 4 is exact, taken on g)
+    const double buoy = p.prm.gravity != 0 ? (p.rho_e ? p.rho_e[e] : m_rho<3>(p, e)) * p.g4 : 0.0;
     const dw v = dw_split(p.vol[e]);
     dw sv[6];
 #pragma unroll
@@ -519,10 +513,10 @@ __global__ void __launch_bounds__(TPB) k_nmd_correct_ft3(KP p, int with_facets)
     if (t < nel) {
         const int e = p.e_lo + t;
         const size_t ne = p.ne;
-        double dpn = 0;
+        double dpn = p.ntmp[conn_at(p, 0, e)];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) dpn += p.ntmp[conn_at(p, i, e)];
-        const double dp_el = dpn / 4;
+        for (int i = 1; i < 4; ++i) dpn += p.ntmp[conn_at(p, i, e)];
+        const double dp_el = dpn / 4;   // a multiplication here: this kernel waits on its loads
         const double dp_orig = p.dp[e];
         double s[6];
 #pragma unroll
@@ -1017,7 +1011,8 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const size_t o = ((size_t)k * 4 + i) * ne + e;
-                            p.shpdw[o] = make_float2(sdw[k][i].hi, sdw[k][i].lo);
+                            // a step's force terms read slots 1..3: slot 0 waits for the chain's last step
+                            if (!AHEAD || i > 0) p.shpdw[o] = make_float2(sdw[k][i].hi, sdw[k][i].lo);
                             s32[k][i] = sdw[k][i].hi;
                         }
                 } else {
@@ -1087,9 +1082,13 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
 #pragma unroll
                 for (int i = 1; i < 4; ++i) h[k][i - 1] = make_float2(sdw[k][i].hi, sdw[k][i].lo);
             double sr[6];
-            strain_rate_mixed_vals(vd, h, sr);
+            float shear[3];
+            strain_rate_mixed_vals(vd, h, sr, shear);
 #pragma unroll
-            for (int cc = 0; cc < 6; ++cc) p.srate[cc * ne + e] = sr[cc];
+            for (int cc = 0; cc < 3; ++cc) {
+                p.srate[cc * ne + e] = sr[cc];
+                p.sh32[cc * ne + e] = shear[cc];
+            }
             qv_next = elem_terms_mixed(p, e, sr, vol, s32, p.prm.has_thermal_diffusion != 0, false);
         }
         // the FP64 context's node velocities, and the look-ahead's element pass (k_elem_pass's arithmetic)
@@ -1151,7 +1150,7 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
                     w4 += v[i][0] * shp[ND - 1][i] - v[i][ND - 1] * shp[0][i];
                     w5 += v[i][1] * shp[ND - 1][i] - v[i][ND - 1] * shp[1][i];
                 }
-                w3 *= 0.5, w4 *= 0.5, w5 *= 0.5;
+                w3 = over_pow2<1>(w3), w4 = over_pow2<1>(w4), w5 = over_pow2<1>(w5);
                 const double dt2 = dt + dt;
                 jaumann3(s, dt, dt2, w3, w4, w5);
                 jaumann3(es, dt, dt2, w3, w4, w5);
@@ -1176,7 +1175,7 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
                 ? ((p.mat.nmat == 1) ? p.mat.rho_pseudo : m_bulkm(p, e) / (pseudo_speed * pseudo_speed))
                 : rho_e;
             // in 3D the division by 4 is exact: taken once, on the volume
-            const double v4 = ND == 3 ? vol / NPE : vol;
+            const double v4 = ND == 3 ? node_mean<NPE>(vol) : vol;
             const double me = ND == 3 ? rho * v4 : rho * vol / NPE;
             double tme = 0.0;
             if (p.prm.has_thermal_diffusion)
@@ -1208,9 +1207,15 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
     }
 }
 
-// three blocks of 256 per SM (80 registers, ~150 bytes of spills to L1):
-// 24 warps hide the node gathers' latency better than 16 with 128 registers
-// (mixed step at 998,400 tets: 23 us less per step)
+// Bounds: the FP64 pipe (a tetrahedron's volume, heights and, in FP64
+// contexts, shape functions and rotation) and, in mixed contexts, the issue
+// of the double-word arithmetic about as much.  MIXED: 32 warps per SM at 64
+// registers (~110 bytes of spills to L1) hide the node gathers better than
+// 24 at 80.  FP64: 24 warps, and 16 with the look-ahead, whose strain rates
+// and heat terms need the registers.  998,400 tets, look-ahead pass: mixed
+// 142 us as one kernel for both precisions, 118 us apart, 115 us with the
+// halvings and quarterings off the FP64 pipe (over_pow2) and shape-function
+// slot 0 left out; FP64 689 and 675 us.
 template <int ND, bool MIXED>
 __global__ void __launch_bounds__(128, MIXED ? 8 : 6) k_geometry(KP p, int flags)
 {

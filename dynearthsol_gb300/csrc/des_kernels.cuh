@@ -19,9 +19,11 @@ namespace des {
 // 998,400 tets x 20 FP64 steps 39.5 -> 39.0 (128 and 64 alike), 998,400 tets
 // x 50 mixed steps 28.3 -> 27.6 (128); blocks of 32 are slower than 64 at
 // every size (launch and scheduling of blocks).
+inline bool one_wave(long long n) { return n <= 152LL * 2048; }
+
 inline int block_threads(long long n, int most = 256)
 {
-    const int t = n <= 152LL * 2048 ? 64 : 128;
+    const int t = one_wave(n) ? 64 : 128;
     return t < most ? t : most;
 }
 

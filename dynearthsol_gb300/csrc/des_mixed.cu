@@ -25,6 +25,7 @@
 // (relative L2) after 2000 steps of the 998,400-tet workload.
 // Element volumes, shape functions, forces and masses stay FP64.
 #include <algorithm>
+#include <cfloat>
 
 #include "des_kernels.cuh"
 #include "des_rheology.cuh"
@@ -60,8 +61,15 @@ __device__ __forceinline__ double exp_mixed(double x)
 __device__ __forceinline__ double visc_law_mixed(const KP &p, int m, double ln_ed, double r)
 {
     const double lnv = fma(p.mat.visc_qnr[m], r, fma(p.mat.visc_pw[m], ln_ed, p.mat.visc_lnc[m]));
-    if (lnv <= p.mat.visc_lnmin) return p.mat.visc_min;
-    if (!(lnv < p.mat.visc_lnmax)) return p.mat.visc_max;   // also T = 0 (1/T infinite), as the FP64 law
+    // with clamps above 1 Pa s the comparisons are those of the bit patterns,
+    // off the FP64 pipe: a negative lnv lies below every clamp, a NaN of
+    // either sign counts as above (as the FP64 law at T = 0)
+    const long long b = __double_as_longlong(lnv);
+    const bool nan = (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+    const bool low = p.mat.visc_ln_pos ? !nan && b <= __double_as_longlong(p.mat.visc_lnmin) : lnv <= p.mat.visc_lnmin;
+    const bool high = p.mat.visc_ln_pos ? nan || b >= __double_as_longlong(p.mat.visc_lnmax) : !(lnv < p.mat.visc_lnmax);
+    if (low) return p.mat.visc_min;
+    if (high) return p.mat.visc_max;   // also T = 0 (1/T infinite), as the FP64 law
     return exp_mixed(lnv);
 }
 
@@ -102,13 +110,10 @@ static __device__ __noinline__ double visc_blend_mixed(const KP &p, int e, doubl
 // limited to 50 beyond the clamps, which moves no clamped mean), then the
 // clamps.  The result is within ~2e-7 of the FP64 law.  Every FP64 <-> FP32
 // conversion is f32_of / f64_of (integer instructions).
-__device__ __forceinline__ double visc_mixed(const KP &p, int e, const double *edot, double T)
+__device__ __forceinline__ double visc_mixed(const KP &p, int e, const double *edot, const float *t, double T)
 {
     if (p.ef[DES_EF_LOG10_VISC]) return m_visc<3>(p, e, edot);
     const double LN2 = 0.6931471805599453;
-    float t[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) t[i] = f32_of(edot[i]);
     const float a = (t[0] + t[1] + t[2]) * (1.0f / 3.0f);
     const float j2 = 0.5f * ((t[0] - a) * (t[0] - a) + (t[1] - a) * (t[1] - a) + (t[2] - a) * (t[2] - a))
         + t[3] * t[3] + t[4] * t[4] + t[5] * t[5];
@@ -120,6 +125,14 @@ __device__ __forceinline__ double visc_mixed(const KP &p, int e, const double *e
     r = r * fma(-T, r, 2.0);
     if (p.mat.nmat == 1) return visc_law_mixed(p, 0, ln_ed, r);
     return visc_blend_mixed(p, e, ln_ed, r);
+}
+
+__device__ __forceinline__ double visc_mixed(const KP &p, int e, const double *edot, double T)
+{
+    float t[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) t[i] = f32_of(edot[i]);
+    return visc_mixed(p, e, edot, t, T);
 }
 
 // maxwell (rheology.cxx:118-134).  The relaxation coefficients come from
@@ -276,16 +289,24 @@ __device__ __forceinline__ double dvol_mixed(const KP &p, int e)
     return (p.vol[e] - vo) * recip_newton(vo);
 }
 
-// The element's strain rate with the anti-locking correction of its normal
-// components (rheology.cxx:527-534), as the FP64 step rounds it
-__device__ __forceinline__ void load_edot(const KP &p, int e, double edv, double *edot)
+// the anti-locking correction of the normal strain rates (rheology.cxx:527-534),
+// as the FP64 step rounds it
+__device__ __forceinline__ void correct_edot(double edv, double *edot)
 {
-    const size_t ne = p.ne;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) edot[c] = p.srate[c * ne + e];
     const double corr = div3(edv - (edot[0] + edot[1] + edot[2]));
 #pragma unroll
     for (int i = 0; i < 3; ++i) edot[i] += corr;
+}
+
+// The element's strain rate before that correction.  ahead: the shear
+// components come as the FP32 values that the look-ahead geometry pass formed.
+__device__ __forceinline__ void load_srate(const KP &p, int e, bool ahead, double *edot)
+{
+    const size_t ne = p.ne;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) edot[c] = p.srate[c * ne + e];
+#pragma unroll
+    for (int c = 3; c < 6; ++c) edot[c] = ahead ? f64_of(p.sh32[(c - 3) * ne + e]) : p.srate[c * ne + e];
 }
 
 // edvoldt (geometry.cxx:158-179) from the step's nodal dvoldt
@@ -294,7 +315,7 @@ __device__ __forceinline__ double elem_edv(const KP &p, int e)
     double dj = p.ntmp[conn_at(p, 0, e)];
 #pragma unroll
     for (int i = 1; i < 4; ++i) dj += p.ntmp[conn_at(p, i, e)];
-    return dj / 4;
+    return node_mean<4>(dj);
 }
 
 // the pressure change, and for the NMD gather its double-word product with
@@ -362,14 +383,6 @@ static __device__ __noinline__ void evp_fp64_branch(const KP &p, int e, bool ela
     }
     const double dp = (out[0] + out[1] + out[2]) - old_s;
     store_dp(p, e, dp, dw_split(dp), fused);
-}
-
-// the element's density and buoyancy term of the step (its temperature is final)
-__device__ __forceinline__ void store_density(const KP &p, int e, double T)
-{
-    const double rho = m_rho_T(p, e, T);
-    p.rho_e[e] = rho;
-    if (p.buoy_e) p.buoy_e[e] = p.prm.gravity != 0 ? rho * p.prm.gravity / 4 : 0.0;
 }
 
 // what is left of an element after the FP32 screens: nothing, or its FP64
@@ -456,15 +469,11 @@ __device__ __forceinline__ int screened_choice(int rest) { return rest & EVP_PLA
 
 // what evp_screens left of element e; edot_done: p.srate holds the corrected
 // strain rate
-static __device__ __noinline__ void evp_rest(const KP &p, int e, int rest, bool fused, bool edot_done)
+static __device__ __noinline__ void evp_rest(const KP &p, int e, int rest, bool fused, bool edot_done, bool ahead)
 {
     double edot[6], s[6];
-    if (edot_done) {
-#pragma unroll
-        for (int c = 0; c < 6; ++c) edot[c] = p.srate[c * (size_t)p.ne + e];
-    } else {
-        load_edot(p, e, elem_edv(p, e), edot);
-    }
+    load_srate(p, e, ahead && !edot_done, edot);
+    if (!edot_done) correct_edot(elem_edv(p, e), edot);
     load_stress(p, e, s);
     const double pls = p.pls[e];
     PlasticProps m{};
@@ -497,8 +506,16 @@ static __device__ __noinline__ void evp_rest(const KP &p, int e, int rest, bool 
 // what it holds.
 // outputs: write the strain rate and edvoldt, which only the end of a call
 // shows (a chained step that another follows leaves them out).
+// Bounds: the FP64 pipe (54 FP64 operations an element off the yield
+// surface, ~75% of its rate) and the issue of the FP32 work beside it.
+// 998,400 tets: 177 us with the FP64 branches in place, 121 us with the list,
+// 111 us with the shear strain rates as floats (ahead), the density's
+// buoyancy formed where the forces are, and the quarterings, clamps and
+// softening bounds taken as integer operations.  14,400 tets with a yielding
+// band: the list 9.4 ms a pass of 100 steps, in place 8.3 ms.
 template <bool LIST>
-__global__ void __launch_bounds__(LIST ? 128 : 64, LIST ? 8 : 4) k_update_stress_evp3(KP p, int fused, int outputs)
+__global__ void __launch_bounds__(LIST ? 128 : 64, LIST ? 8 : 4) k_update_stress_evp3(KP p, int fused, int outputs,
+                                                                                       int ahead)
 {
     __shared__ int list[128];
     __shared__ int listed;
@@ -512,6 +529,7 @@ __global__ void __launch_bounds__(LIST ? 128 : 64, LIST ? 8 : 4) k_update_stress
         const float dtf = f32_of(p.clk->dt);
         float def[6];
         double edot[6];
+        float edf[6];   // the strain rate in FP32
         {   // FP32 strain increments; the strain accumulates them in FP64
             double edv;
             if (fused) {
@@ -520,18 +538,33 @@ __global__ void __launch_bounds__(LIST ? 128 : 64, LIST ? 8 : 4) k_update_stress
             } else {
                 edv = p.edvoldt[e];
             }
-            load_edot(p, e, edv, edot);
+            if (ahead) {   // f32_of(f64_of(x)) is x, a subnormal's a zero
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    edot[c] = p.srate[c * ne + e];
+                    const float x = p.sh32[c * ne + e];
+                    edf[3 + c] = fabsf(x) < FLT_MIN ? copysignf(0.0f, x) : x;
+                    edot[3 + c] = f64_of(edf[3 + c]);
+                }
+            } else {
+                load_srate(p, e, false, edot);
+#pragma unroll
+                for (int c = 3; c < 6; ++c) edf[c] = f32_of(edot[c]);
+            }
+            correct_edot(edv, edot);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) edf[c] = f32_of(edot[c]);
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
                 if (outputs) p.srate[c * ne + e] = edot[c];
-                def[c] = f32_of(edot[c]) * dtf;
+                def[c] = edf[c] * dtf;
                 p.strain[c * ne + e] += f64_of(def[c]);
             }
         }
         const double T = elem_avg_T<4>(p, e);
         const float shearf = f32_of(m_shearm(p, e));
-        const float tf = relaxation_f(dtf, shearf, f32_of(visc_mixed(p, e, edot, T)));
-        if (fused && p.rho_e) store_density(p, e, T);
+        const float tf = relaxation_f(dtf, shearf, f32_of(visc_mixed(p, e, edot, edf, T)));
+        if (fused && p.rho_e) p.rho_e[e] = m_rho_T(p, e, T);   // the step's: the temperature is final
         const double pls = p.pls[e];
         double s[6];
         load_stress(p, e, s);
@@ -554,11 +587,11 @@ __global__ void __launch_bounds__(LIST ? 128 : 64, LIST ? 8 : 4) k_update_stress
     __syncthreads();
     const int n = listed;
     for (int k = threadIdx.x; k < n; k += blockDim.x)
-        evp_rest(p, base + (list[k] >> 4), list[k] & 15, fused != 0, outputs || !fused);
+        evp_rest(p, base + (list[k] >> 4), list[k] & 15, fused != 0, outputs || !fused, ahead != 0);
 }
 
 // the other rheologies
-__global__ void __launch_bounds__(128, 6) k_update_stress_mixed3(KP p, int fused)
+__global__ void __launch_bounds__(128, 6) k_update_stress_mixed3(KP p, int fused, int ahead)
 {
     int e = p.e_lo + blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= p.e_hi) return;
@@ -571,7 +604,8 @@ __global__ void __launch_bounds__(128, 6) k_update_stress_mixed3(KP p, int fused
         edv = p.edvoldt[e];
     }
     double s[6], es[6], edot[6], de[6];
-    load_edot(p, e, edv, edot);
+    load_srate(p, e, ahead != 0, edot);
+    correct_edot(edv, edot);
     const double dt = p.clk->dt;
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
@@ -612,7 +646,7 @@ __global__ void __launch_bounds__(128, 6) k_update_stress_mixed3(KP p, int fused
     }
     const double dp = (s[0] + s[1] + s[2]) - old_s;
     store_dp(p, e, dp, dw_split(dp), fused != 0);
-    if (fused && p.rho_e) store_density(p, e, T);
+    if (fused && p.rho_e) p.rho_e[e] = m_rho_T(p, e, T);
     if (bits) set_err(p, bits);
 }
 
@@ -628,7 +662,10 @@ __device__ __forceinline__ void strain_rate_mixed_elem(const KP &p, int e, doubl
     for (int k = 0; k < 3; ++k)
 #pragma unroll
         for (int i = 1; i < 4; ++i) h[k][i - 1] = p.shpdw[((size_t)k * 4 + i) * ne + e];
-    strain_rate_mixed_vals(v, h, out);
+    float shear[3];
+    strain_rate_mixed_vals(v, h, out, shear);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) out[3 + c] = f64_of(shear[c]);
 #pragma unroll
     for (int c = 0; c < 6; ++c) p.srate[c * ne + e] = out[c];
 }
@@ -796,15 +833,15 @@ __global__ void __launch_bounds__(192) k_node_pass_mixed3(KP p, int heat, int be
     }
 }
 
-int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused, bool outputs)
+int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused, bool outputs, bool ahead)
 {
-    const int n = p.e_hi - p.e_lo;
-    if (p.mat.rheol_type == DES_RH_EVP) {
-        if (block_threads(n) < 128) DES_LAUNCH(k_update_stress_evp3<false>, n, s, p, (int)fused, (int)(outputs || !fused));
-        else DES_LAUNCH(k_update_stress_evp3<true>, n, s, p, (int)fused, (int)(outputs || !fused));
-    } else {
-        DES_LAUNCH(k_update_stress_mixed3, n, s, p, (int)fused);
-    }
+    const int n = p.e_hi - p.e_lo, out = outputs || !fused;
+    if (p.mat.rheol_type != DES_RH_EVP)
+        DES_LAUNCH(k_update_stress_mixed3, n, s, p, (int)fused, (int)ahead);
+    else if (one_wave(n))
+        DES_LAUNCH(k_update_stress_evp3<false>, n, s, p, (int)fused, out, (int)ahead);
+    else
+        DES_LAUNCH(k_update_stress_evp3<true>, n, s, p, (int)fused, out, (int)ahead);
     return 1;
 }
 

@@ -8,8 +8,9 @@
 namespace des {
 
 // outputs: also write the strain rate and edvoldt of a fused step (nothing
-// in the step that follows reads them)
-int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused, bool outputs = true);
+// in the step that follows reads them); ahead: the strain rate is the
+// look-ahead geometry pass's (its shear components in KP::sh32)
+int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused, bool outputs = true, bool ahead = false);
 int launch_strain_rate_mixed(const KP &p, cudaStream_t s, bool begin_step);
 int launch_heat_and_dvoldt_mixed(const KP &p, cudaStream_t s, bool heat, bool dvoldt);
 // fused step: strain rate + heat terms + dvoldt terms, then the nodal sums and the temperature update

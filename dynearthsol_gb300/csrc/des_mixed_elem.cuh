@@ -23,7 +23,9 @@ namespace des {
 // (~2^-45 of the row's terms), the shear ones FP32 from the pairs' high parts.
 //   v: the four nodes' velocities as double-word pairs (dw_split of the FP64
 //   values); h[k][i - 1]: the pair of dN_i/dx_k, i = 1..3
-__device__ __forceinline__ void strain_rate_mixed_vals(const dw (*v)[3], const float2 (*h)[3], double *out)
+//   out: the FP64 normal components; shear: the FP32 shear components
+__device__ __forceinline__ void strain_rate_mixed_vals(const dw (*v)[3], const float2 (*h)[3], double *out,
+                                                       float *shear)
 {
     dw w0[3];
 #pragma unroll
@@ -51,9 +53,9 @@ __device__ __forceinline__ void strain_rate_mixed_vals(const dw (*v)[3], const f
         s4 += 0.5f * (dv[i][0] * sz[i] + dv[i][2] * sx[i]);
         s5 += 0.5f * (dv[i][1] * sz[i] + dv[i][2] * sy[i]);
     }
-    out[3] = f64_of(s3);
-    out[4] = f64_of(s4);
-    out[5] = f64_of(s5);
+    shear[0] = s3;
+    shear[1] = s4;
+    shear[2] = s5;
 }
 
 // the four nodes' velocities of element e as double-word pairs
