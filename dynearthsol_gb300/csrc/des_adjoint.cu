@@ -33,7 +33,7 @@ __device__ __forceinline__ double tshp(const TapeStep &t, size_t ne, int k, int 
     return t.shp[((size_t)k * 4 + i) * ne + e];
 }
 
-// the stress after NMD_stress (geometry.cxx:182-236), as k_nmd_correct forms
+// the stress after NMD_stress (geometry.cxx:182-236), as k_elem_force forms
 // it, from the tape's stress after update_stress and its pressure changes:
 // the same operations in the same order, so the same bits (the division by
 // 4 is exact, with or without a fused multiply-add)

@@ -65,7 +65,6 @@ KP step_kp(const des_ctx *c)
 {
     KP p = c->kp;
     p.rho_e = c->d_rho;
-    p.buoy_e = c->d_buoy;
     p.tdot = c->d_tdot;
     return p;
 }
@@ -412,21 +411,22 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     float2 *d_shpdw = nullptr, *d_vdw = nullptr, *d_pv = nullptr;
     double4 *d_ndpk = nullptr;
     int *d_sup_pos = nullptr;
+    double2 *d_ft64 = nullptr;
     double *d_qv = nullptr, *d_hc64 = nullptr;
     add((void **)&d_qv, (size_t)ne * D);
     add((void **)&d_ndpk, (size_t)ne * sizeof(double4));
+    add((void **)&d_sup_pos, (size_t)ne * npe * I);
     if (mixed3) {
         add((void **)&d_hc, (size_t)ne * npe * sizeof(float));
         add((void **)&d_ft, (size_t)ne * npe * 2 * sizeof(float4));
         add((void **)&d_shpdw, (size_t)ne * npe * nd * sizeof(float2));
         add((void **)&d_vdw, (size_t)nn * nd * sizeof(float2));
         add((void **)&d_pv, (size_t)ne * sizeof(float2));
-        add((void **)&d_sup_pos, (size_t)ne * npe * I);
     } else {
         add((void **)&d_hc64, (size_t)ne * npe * D);
+        add((void **)&d_ft64, (size_t)ne * npe * (nd - 1) * sizeof(double2));
     }
     add((void **)&c->d_rho, (size_t)ne * D);
-    add((void **)&c->d_buoy, (size_t)ne * D);
     add((void **)&p.me, (size_t)ne * 2 * D);   // me, then tme
     add((void **)&p.fv, (size_t)std::max(nbf, 1) * nd * D);
     add((void **)&p.clk, sizeof(Clock));
@@ -479,7 +479,6 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     p.emark = d_emark;
     p.eprop = nullptr;   // set once k_elem_props has filled d_eprop
     p.rho_e = nullptr;
-    p.buoy_e = nullptr;
     p.tdot = p.ntmp;
     p.sh32 = mixed3 ? (float *)p.me : nullptr;
     p.shpdw = d_shpdw;
@@ -491,6 +490,7 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     p.hc64 = d_hc64;
     p.ft = d_ft;
     p.sup_pos = d_sup_pos;
+    p.ft64 = d_ft64;
     p.e_lo = 0, p.e_hi = ne, p.n_lo = 0, p.n_hi = nn, p.f_lo = 0, p.f_hi = nbf;
     p.fac_order = nullptr;
     p.tape_visc = nullptr;
@@ -513,7 +513,7 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     up(d_bc, mesh->bcflag, (size_t)nn * sizeof(unsigned));
     up(d_sup_off, sup_off.data(), sup_off.size() * I);
     up(d_sup_ent, sup_ent.data(), sup_ent.size() * I);
-    if (d_sup_pos) {   // the support-list entry of each (element, slot), slot-major
+    {   // the support-list entry of each (element, slot), slot-major
         std::vector<int> pos((size_t)ne * npe);
         for (size_t q = 0; q < sup_ent.size(); ++q) pos[(size_t)(sup_ent[q] & 3) * ne + (sup_ent[q] >> 2)] = (int)q;
         up(d_sup_pos, pos.data(), pos.size() * I);
@@ -1148,8 +1148,7 @@ PERFN(des_update_stress,
 PERFN(des_NMD_stress, n += launch_nmd_gather(p, s); n += launch_nmd_correct(p, s, false))
 // in a mixed context, the fused-multiply-add forms of the mixed step
 PERFN(des_update_force,
-      n += launch_facet_forces(p, s); n += launch_force_terms(p, s);
-      n += launch_force(p, s, false, p.shpdw != nullptr))
+      n += launch_force_terms(p, s); n += launch_force(p, s, false))
 PERFN(des_update_velocity, n += launch_velocity(p, s, p.shpdw != nullptr))
 PERFN(des_apply_vbcs, n += launch_vbcs(p, s))
 PERFN(des_update_coordinate, n += launch_coordinate(p, s, p.shpdw != nullptr))
@@ -1291,7 +1290,7 @@ int enqueue_step_chain(des_ctx *c, int part)
     n += mixed ? launch_update_stress_mixed(p, s, true, part == 2, part != 0) : launch_update_stress(p, s, true);
     n += launch_nmd_gather(p, s, mixed);
     n += launch_nmd_correct(p, s, true);
-    n += launch_force(p, s, true, mixed);
+    n += launch_force(p, s, true);
     if (part == 2) {
         n += launch_geometry(p, s, step_geometry(p));
         n += launch_mass_sum(p, s);
@@ -1314,7 +1313,7 @@ int enqueue_step(des_ctx *c, cudaEvent_t mid)
     n += launch_nmd_gather(p, s, mixed);
     n += launch_nmd_correct(p, s, true);
     if (record_mid(mid, s)) return -1;
-    n += launch_force(p, s, true, mixed);
+    n += launch_force(p, s, true);
     n += launch_geometry(p, s, step_geometry(p));
     n += launch_mass_sum(p, s);
     return n;
@@ -1549,7 +1548,7 @@ int capture_pipelined(des_ctx *c, const std::vector<SlabField> &F, cudaGraphExec
             case 4: n += mixed ? launch_update_stress_mixed(q, cs, true) : launch_update_stress(q, cs, true); break;
             case 5: n += launch_nmd_gather(q, cs, mixed); break;
             case 6: n += launch_nmd_correct(q, cs, true); break;
-            case 7: n += launch_force(q, cs, true, mixed); break;
+            case 7: n += launch_force(q, cs, true); break;
             case 8: {
                 int geo = GEO_COPY_OLD | GEO_VOLUME | GEO_SHAPE | GEO_DT | GEO_DT_IF_STEP | GEO_MASS_TERMS;
                 if (q.mat.rheol_type & DES_RH_ELASTIC) geo |= GEO_ROTATE;

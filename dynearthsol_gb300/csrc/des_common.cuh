@@ -110,7 +110,6 @@ struct KP {
     double *stress, *strain, *srate, *pls, *dpls, *syy, *dp, *edvoldt, *vol, *vol_old, *shp;
     double *rho_e;                       // per-element density of the step (scratch), or null
     double g4;                           // gravity / 4 (an exact scaling)
-    double *buoy_e;                      // per-element rho g / NPE of the step (scratch), or null
     double *tdot;                        // node scratch for the heat gather (ntmp outside the fused step)
     double *fv;                          // [nd][nbf] per-facet stress-BC force (scratch)
     // mixed 3D step (a mixed context is one with shpdw): the shape functions
@@ -131,6 +130,9 @@ struct KP {
     // of (element e, slot i): q = sup_pos[i ne + e], the inverse of sup_ent
     float4 *ft;
     const int *sup_pos;
+    // the FP64 step's: -(sigma . dN_i/dx + buoyancy z) vol, one (2D) or two
+    // (3D, the last value unused) double2 per support-list entry
+    double2 *ft64;
     // set only by the reverse mode's forward recompute: the viscosity the
     // rheology used and the EVP branch it took (1: elasto-plastic), per element
     double *tape_visc;

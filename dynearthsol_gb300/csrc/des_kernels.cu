@@ -341,12 +341,7 @@ __global__ void __launch_bounds__(TPB) k_update_stress(KP p, int fused)
     p.pls[e] = pls;
     p.dpls[e] = dpls;
     p.dp[e] = dpr;
-    if (fused && p.rho_e) {   // temperature is final for this step
-        const double rho = m_rho<ND>(p, e);
-        p.rho_e[e] = rho;
-        // the force gather's buoyancy term, once per element instead of per node
-        if (p.buoy_e) p.buoy_e[e] = p.prm.gravity != 0 ? rho * p.prm.gravity / (ND + 1) : 0.0;
-    }
+    if (fused && p.rho_e) p.rho_e[e] = m_rho<ND>(p, e);   // temperature is final for this step
     if (bits) set_err(p, bits);
 }
 
@@ -445,24 +440,6 @@ __device__ void facet_force(const KP &p, int q)
     for (int d = 0; d < ND; ++d) p.fv[(size_t)d * p.nbf + q] = out[d];
 }
 
-template <int ND>
-__global__ void __launch_bounds__(TPB) k_nmd_correct(KP p, int with_facets)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, nel = p.e_hi - p.e_lo;
-    if (t < nel) {
-        const int e = p.e_lo + t;
-        double dpn = p.ntmp[conn_at(p, 0, e)];
-#pragma unroll
-        for (int i = 1; i < ND + 1; ++i) dpn += p.ntmp[conn_at(p, i, e)];
-        const double corr = divnd<ND>(-p.dp[e] + node_mean<ND + 1>(dpn));
-#pragma unroll
-        for (int i = 0; i < ND; ++i) p.stress[(size_t)i * p.ne + e] += corr;
-    } else if (with_facets && t < nel + (p.f_hi - p.f_lo)) {
-        const int i = p.f_lo + (t - nel);
-        facet_force<ND>(p, p.fac_order ? p.fac_order[i] : i);
-    }
-}
-
 // The mixed 3D step's force terms of one element (fields.cxx:291-340, the
 // element's part): for each node slot i the vector
 //   T_i = (sigma . dN_i/dx + rho g / 4 z) vol,
@@ -505,50 +482,88 @@ __device__ __forceinline__ void force_terms_dw3(const KP &p, int e, const double
     }
 }
 
-// k_nmd_correct<3> for the mixed step, which also forms the element's force
-// terms from the corrected stress (the same bits of stress as k_nmd_correct)
-__global__ void __launch_bounds__(TPB) k_nmd_correct_ft3(KP p, int with_facets)
+// The FP64 step's force term of an element's node slot i:
+// -(sigma . dN_i/dx + rho g / NPE z) vol, the expression the reference
+// subtracts, to the support-list entry of (e, i).
+template <int ND>
+__device__ __forceinline__ double buoyancy(const KP &p, int e)   // rho g / NPE
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, nel = p.e_hi - p.e_lo;
-    if (t < nel) {
-        const int e = p.e_lo + t;
-        const size_t ne = p.ne;
-        double dpn = p.ntmp[conn_at(p, 0, e)];
-#pragma unroll
-        for (int i = 1; i < 4; ++i) dpn += p.ntmp[conn_at(p, i, e)];
-        const double dp_el = dpn / 4;   // a multiplication here: this kernel waits on its loads
-        const double dp_orig = p.dp[e];
-        double s[6];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            s[i] = p.stress[(size_t)i * ne + e] + divnd<3>(-dp_orig + dp_el);
-            p.stress[(size_t)i * ne + e] = s[i];
-        }
-#pragma unroll
-        for (int i = 3; i < 6; ++i) s[i] = p.stress[(size_t)i * ne + e];
-        force_terms_dw3(p, e, s);
-    } else if (with_facets && t < nel + (p.f_hi - p.f_lo)) {
-        const int i = p.f_lo + (t - nel);
-        facet_force<3>(p, p.fac_order ? p.fac_order[i] : i);
-    }
-}
-
-// the force terms alone (des_update_force in a mixed context)
-__global__ void __launch_bounds__(TPB) k_force_terms3(KP p)
-{
-    const int e = p.e_lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= p.e_hi) return;
-    double s[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) s[c] = p.stress[(size_t)c * p.ne + e];
-    force_terms_dw3(p, e, s);
+    if (p.prm.gravity == 0) return 0;
+    const double rho = p.rho_e ? p.rho_e[e] : m_rho<ND>(p, e);
+    return ND == 3 ? rho * p.g4 : rho * p.prm.gravity / (ND + 1);   // the division by 4 is exact, taken on g
 }
 
 template <int ND>
-__global__ void __launch_bounds__(TPB) k_facet_forces(KP p)
+__device__ __forceinline__ void force_term(const KP &p, int e, int i, const double *s, double buoy, double vol)
 {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < p.nbf) facet_force<ND>(p, q);
+    const size_t q = p.sup_pos[(size_t)i * p.ne + e];
+    const double sx = shp_at(p, 0, i, e), sz = shp_at(p, ND - 1, i, e);
+    if (ND == 3) {
+        const double sy = shp_at(p, 1, i, e);
+        p.ft64[2 * q] = make_double2(-(s[0] * sx + s[3] * sy + s[4] * sz) * vol,
+                                     -(s[3] * sx + s[1] * sy + s[5] * sz) * vol);
+        p.ft64[2 * q + 1] = make_double2(-(s[4] * sx + s[5] * sy + s[2] * sz + buoy) * vol, 0.0);
+    } else {
+        p.ft64[q] = make_double2(-(s[0] * sx + s[2] * sz) * vol, -(s[2] * sx + s[1] * sz + buoy) * vol);
+    }
+}
+
+// CORRECT: the NMD correction of the normal stresses from the nodal dp of
+// p.ntmp.  TERMS: the element's force terms, from the corrected stress (the
+// element's stress and volume read once for its four nodes, where a node
+// gather read them four times), and one thread per stress-BC facet after the
+// elements.  PAIRS: the mixed 3D step's terms.  SPLIT: four threads to an
+// element, a slot each.
+// Bounds: in FP64 the FP64 pipe (88 operations an element, ~80% of its rate);
+// with pairs the memory (328 B an element).  998,400 tets: 175 us and 58 us
+// for the sums of k_force, where the correction alone and a gather that
+// formed the terms per support entry took 27 and 220 us; pairs 70 us.
+template <int ND, bool CORRECT, bool TERMS, bool PAIRS, bool SPLIT>
+__global__ void __launch_bounds__(TPB) k_elem_force(KP p)
+{
+    constexpr int NSTR = ND * (ND + 1) / 2;
+    static_assert(!SPLIT || (TERMS && !PAIRS), "only the FP64 terms are formed slot by slot");
+    const int nel = p.e_hi - p.e_lo;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < (SPLIT ? 4 : 1) * nel) {
+        const int e = p.e_lo + (SPLIT ? t >> 2 : t);
+        const size_t ne = p.ne;
+        double s[NSTR];
+        if (TERMS) {
+#pragma unroll
+            for (int c = 0; c < NSTR; ++c) s[c] = p.stress[c * ne + e];
+        }
+        if (CORRECT) {
+            double dpn = p.ntmp[conn_at(p, 0, e)];
+#pragma unroll
+            for (int i = 1; i < ND + 1; ++i) dpn += p.ntmp[conn_at(p, i, e)];
+            // the pairs' kernel waits on its loads: there a multiplication
+            const double dp_el = PAIRS ? dpn / (ND + 1) : node_mean<ND + 1>(dpn);
+            const double corr = divnd<ND>(-p.dp[e] + dp_el);
+            // an element's four threads have read its stress
+            if (SPLIT) __syncwarp(0xfu << (threadIdx.x & 28));
+#pragma unroll
+            for (int c = 0; c < ND; ++c) {
+                if (TERMS) s[c] += corr;
+                else s[c] = p.stress[c * ne + e] + corr;
+                if (!SPLIT || (t & 3) == 0) p.stress[c * ne + e] = s[c];
+            }
+        }
+        if constexpr (PAIRS) {
+            force_terms_dw3(p, e, s);
+        } else if constexpr (TERMS) {
+            const double buoy = buoyancy<ND>(p, e), vol = p.vol[e];
+            if constexpr (SPLIT) {
+                if ((t & 3) <= ND) force_term<ND>(p, e, t & 3, s, buoy, vol);
+            } else {
+#pragma unroll
+                for (int i = 0; i < ND + 1; ++i) force_term<ND>(p, e, i, s, buoy, vol);
+            }
+        }
+    } else if (TERMS && t < (SPLIT ? 4 : 1) * nel + (p.f_hi - p.f_lo)) {
+        const int i = p.f_lo + (t - (SPLIT ? 4 : 1) * nel);
+        facet_force<ND>(p, p.fac_order ? p.fac_order[i] : i);
+    }
 }
 
 // ==================================================================
@@ -588,47 +603,6 @@ __device__ __forceinline__ double madd(double a, double b, double c)
 // dt f (1/m) with one recip_newton.
 template <int ND, bool CONTRACT>
 __device__ __forceinline__ void force_tail(const KP &p, int n, double *f, int fused_motion);
-
-// The FP64 step's force: each support entry's term -(sigma . dN_i/dx + rho g
-// / NPE z) vol, the expression the reference subtracts; then the FP64 tail.
-template <int ND, bool STAGED>
-__global__ void __launch_bounds__(192) k_force(KP p, int fused_motion)
-{
-    constexpr int NSTR = ND * (ND + 1) / 2;
-    constexpr int NPE = ND + 1;
-    const size_t ne = p.ne;
-    const double gravity = p.prm.gravity;
-    double f[ND];
-    const int n = node_sums<SumF64, ND, ND, STAGED>(
-        p.sup_off, p.n_lo, p.n_hi, ND,
-        [&](int q, double *t) {
-            const int ent = p.sup_ent[q];
-            const int e = ent >> 2, i = ent & 3;
-            double s[NSTR];
-#pragma unroll
-            for (int c = 0; c < NSTR; ++c) s[c] = p.stress[c * ne + e];
-            const double vol = p.vol[e];
-            double buoy = 0;
-            if (p.buoy_e) {
-                buoy = p.buoy_e[e];
-            } else if (gravity != 0) {
-                const double rho = p.rho_e ? p.rho_e[e] : m_rho<ND>(p, e);
-                buoy = rho * gravity / NPE;
-            }
-            const double sx = shp_at(p, 0, i, e), sz = shp_at(p, ND - 1, i, e);
-            if (ND == 3) {
-                const double sy = shp_at(p, 1, i, e);
-                t[0] = -(s[0] * sx + s[3] * sy + s[4] * sz) * vol;
-                t[1] = -(s[3] * sx + s[1] * sy + s[5] * sz) * vol;
-                t[ND - 1] = -(s[4] * sx + s[5] * sy + s[2] * sz + buoy) * vol;
-            } else {
-                t[0] = -(s[0] * sx + s[2] * sz) * vol;
-                t[ND - 1] = -(s[2] * sx + s[1] * sz + buoy) * vol;
-            }
-        },
-        FromZero<SumF64>(), f);
-    if (n >= 0) force_tail<ND, false>(p, n, f, fused_motion);
-}
 
 // k_force after its element gather: the gravity-induced stress BCs, the
 // elastic foundation, damping and the force store, then (fused_motion) the
@@ -684,8 +658,8 @@ __device__ __forceinline__ void force_tail(const KP &p, int n, double *f, int fu
 }
 
 // update_force of the mixed 3D step: each node sums the force terms T of its
-// support (k_nmd_correct_ft3 / k_force_terms3, stored in the support list's
-// order: one contiguous run per node) in ascending element order in
+// support (k_elem_force, stored in the support list's order: one contiguous run per
+// node) in ascending element order in
 // double-word arithmetic -- whose sums are accurate relative to the exact
 // sum (Algorithm 6 of des_dw.cuh), however much the elements' terms cancel
 // -- and rounds the sum to FP64 once; the rest is k_force's FP64 tail.
@@ -699,6 +673,28 @@ struct ForceTerms {   // the three components' terms of a support entry
         t[2] = make_float2(h.z, l.z);
     }
 };
+
+// The FP64 step's force: the sums of its terms (force_terms) in FP64.
+template <int ND>
+struct ForceTerms64 {
+    const double2 *ft;
+    __device__ __forceinline__ void operator()(int q, double *t) const
+    {
+        const double2 a = __ldg(ft + (ND - 1) * (size_t)q);
+        t[0] = a.x;
+        t[1] = a.y;
+        if (ND == 3) t[ND - 1] = __ldg((const double *)(ft + 2 * (size_t)q + 1));
+    }
+};
+
+template <int ND, bool STAGED>
+__global__ void __launch_bounds__(192) k_force(KP p, int fused_motion)
+{
+    double f[ND];
+    const int n = node_sums<SumF64, ND, ND, STAGED>(p.sup_off, p.n_lo, p.n_hi, ND, ForceTerms64<ND>{p.ft64},
+                                                    FromZero<SumF64>(), f);
+    if (n >= 0) force_tail<ND, false>(p, n, f, fused_motion);
+}
 
 template <bool STAGED>
 __global__ void __launch_bounds__(192) k_force_dw3(KP p, int fused_motion)
@@ -1573,35 +1569,51 @@ int launch_nmd_gather(const KP &p, cudaStream_t s, bool stored)
     return 1;
 }
 
-int launch_nmd_correct(const KP &p, cudaStream_t s, bool with_facets)
+// The force terms of [e_lo, e_hi) and the facets' forces, with or without
+// the correction first.  Up to a wave of slots the element's four slots go
+// side by side, where a thread's chain of 76 FP64 operations is what a launch
+// takes: a pass of 100 steps of 648 tets 5.79 ms, a thread per element 6.03
+// ms; beyond, four threads repeat the element's loads and correction for
+// nothing: 20 steps of 998,400 tets 36.0 ms split, 34.7 ms not, 118,326 tets
+// 4.10 and 4.05 ms.
+template <int ND, bool CORRECT>
+void launch_elem_force(const KP &p, cudaStream_t s)
 {
-    long long n = (long long)(p.e_hi - p.e_lo) + (with_facets ? p.f_hi - p.f_lo : 0);
-    if (uses_force_terms(p)) {
-        DES_LAUNCH(k_nmd_correct_ft3, n, s, p, (int)with_facets);
-        return 1;
+    const long long nel = p.e_hi - p.e_lo, nf = p.f_hi - p.f_lo;
+    if (4 * nel <= 152 * 2048) DES_LAUNCH((k_elem_force<ND, CORRECT, true, false, true>), 4 * nel + nf, s, p);
+    else DES_LAUNCH((k_elem_force<ND, CORRECT, true, false, false>), nel + nf, s, p);
+}
+
+int launch_nmd_correct(const KP &p, cudaStream_t s, bool fused)
+{
+    const long long nel = p.e_hi - p.e_lo;
+    if (!fused) {
+        if (p.nd == 3) DES_LAUNCH((k_elem_force<3, true, false, false, false>), nel, s, p);
+        else DES_LAUNCH((k_elem_force<2, true, false, false, false>), nel, s, p);
+    } else if (p.ft) {
+        DES_LAUNCH((k_elem_force<3, true, true, true, false>), nel + (p.f_hi - p.f_lo), s, p);
+    } else {
+        if (p.nd == 3) launch_elem_force<3, true>(p, s);
+        else launch_elem_force<2, true>(p, s);
     }
-    DISPATCH(k_nmd_correct, n, p, (int)with_facets);
     return 1;
 }
 
 int launch_force_terms(const KP &p, cudaStream_t s)
 {
-    if (!uses_force_terms(p)) return 0;
-    DES_LAUNCH(k_force_terms3, p.e_hi - p.e_lo, s, p);
+    if (p.ft) {
+        DES_LAUNCH((k_elem_force<3, false, true, true, false>), (long long)(p.e_hi - p.e_lo) + (p.f_hi - p.f_lo), s, p);
+    } else {
+        if (p.nd == 3) launch_elem_force<3, false>(p, s);
+        else launch_elem_force<2, false>(p, s);
+    }
     return 1;
 }
 
-int launch_facet_forces(const KP &p, cudaStream_t s)
-{
-    if (p.nbf == 0) return 0;
-    DISPATCH(k_facet_forces, p.nbf, p);
-    return 1;
-}
-
-int launch_force(const KP &p, cudaStream_t s, bool fused_motion, bool contract)
+int launch_force(const KP &p, cudaStream_t s, bool fused_motion)
 {
     const int n = p.n_hi - p.n_lo;
-    if (contract && uses_force_terms(p)) DES_NODES(k_force_dw3<STAGED>, n, s, p, (int)fused_motion);
+    if (p.ft) DES_NODES(k_force_dw3<STAGED>, n, s, p, (int)fused_motion);
     else if (p.nd == 3) DES_NODES((k_force<3, STAGED>), n, s, p, (int)fused_motion);
     else DES_NODES((k_force<2, STAGED>), n, s, p, (int)fused_motion);
     return 1;
