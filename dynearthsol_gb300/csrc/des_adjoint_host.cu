@@ -315,7 +315,7 @@ int adj_step(des_ctx *c, const TapeStep *t)
     n += launch_nmd_correct(p, s, true);
     n += launch_force(p, s, true);
     // mass from the geometry pass's element terms: the same sums, in the same
-    // order, as compute_mass's node gather (launch_mass), at a fifth of its cost
+    // order, as compute_mass's
     int geo = GEO_COPY_OLD | GEO_VOLUME | GEO_SHAPE | GEO_MASS_TERMS;
     if (p.mat.rheol_type & DES_RH_ELASTIC) geo |= GEO_ROTATE;
     n += launch_geometry(p, s, geo);

@@ -935,14 +935,15 @@ int des_upload_state(des_ctx *c, const des_host_state *st)
         CK(cudaStreamSynchronize(c->stream));   // ck lives on this stack frame
     }
     KP q = p;   // per-function form
-    if (!st->volume && (rc = check_launch(c, launch_geometry(q, c->stream, GEO_VOLUME)))) return rc;
     // a mixed 3D context forms its double-word shape functions from the
     // coordinates: FP64 values do not split into pairs exactly, and so do not
     // carry its own pairs through a download and an upload
-    if (!have_shp || p.shpdw) {
-        if ((rc = check_launch(c, launch_geometry(q, c->stream, GEO_SHAPE)))) return rc;
-    }
-    if (!have_mass && (rc = check_launch(c, launch_mass(q, c->stream)))) return rc;
+    int geo = 0;
+    if (!st->volume) geo |= GEO_VOLUME;
+    if (!have_shp || p.shpdw) geo |= GEO_SHAPE;
+    if (!have_mass) geo |= GEO_MASS_TERMS;
+    if (geo && (rc = check_launch(c, launch_geometry(q, c->stream, geo)))) return rc;
+    if (!have_mass && (rc = check_launch(c, launch_mass_sum(q, c->stream)))) return rc;
     CK(cudaStreamSynchronize(c->stream));
     c->has_state = true;
     return DES_OK;
@@ -1136,8 +1137,8 @@ int des_set_clock(des_ctx *c, double time, double dt, int steps)
     }
 
 PERFN(des_update_temperature,
-      n += (p.shpdw ? launch_heat_and_dvoldt_mixed(p, s, true, false) : launch_heat_gather(p, s));
-      n += launch_temperature_update(p, s))
+      n += (p.shpdw ? launch_heat_and_dvoldt_mixed(p, s, true, false) + launch_temperature_update(p, s)
+                    : launch_update_temperature(p, s)))
 PERFN(des_update_strain_rate,
       n += (p.shpdw ? launch_strain_rate_mixed(p, s, false) : launch_strain_rate(p, s, false)))
 PERFN(des_compute_dvoldt, n += launch_dvoldt(p, s))
@@ -1154,12 +1155,12 @@ PERFN(des_apply_vbcs, n += launch_vbcs(p, s))
 PERFN(des_update_coordinate, n += launch_coordinate(p, s, p.shpdw != nullptr))
 PERFN(des_swap_volume, n += launch_geometry(p, s, GEO_COPY_OLD))
 PERFN(des_compute_volume, n += launch_geometry(p, s, GEO_VOLUME))
-PERFN(des_compute_mass, n += launch_mass(p, s))
+PERFN(des_compute_mass, n += launch_geometry(p, s, GEO_MASS_TERMS); n += launch_mass_sum(p, s))
 PERFN(des_compute_shape_fn, n += launch_geometry(p, s, GEO_SHAPE))
 PERFN(des_rotate_stress, n += launch_geometry(p, s, GEO_ROTATE))
 PERFN(des_update_mesh, n += launch_coordinate(p, s, p.shpdw != nullptr);
-      n += launch_geometry(p, s, GEO_COPY_OLD | GEO_VOLUME); n += launch_mass(p, s);
-      n += launch_geometry(p, s, GEO_SHAPE))
+      n += launch_geometry(p, s, GEO_COPY_OLD | GEO_VOLUME | GEO_SHAPE | GEO_MASS_TERMS);
+      n += launch_mass_sum(p, s))
 
 int des_compute_dt(des_ctx *c, double *dt_out)
 {

@@ -68,18 +68,26 @@ __device__ __forceinline__ void strain_rate_vals(const double (*v)[ND], const do
     }
 }
 
+// dN_i/dx of element e (sy: zero in 2D)
+template <int ND>
+__device__ __forceinline__ void load_shp(const KP &p, int e, double *sx, double *sy, double *sz)
+{
+#pragma unroll
+    for (int i = 0; i < ND + 1; ++i) {
+        sx[i] = shp_at(p, 0, i, e);
+        sy[i] = ND == 3 ? shp_at(p, 1, i, e) : 0.0;
+        sz[i] = shp_at(p, ND - 1, i, e);
+    }
+}
+
 template <int ND>
 __device__ __forceinline__ void strain_rate_elem(const KP &p, int e, double *s)
 {
     constexpr int NPE = ND + 1;
     double v[NPE][ND], sx[NPE], sy[NPE], sz[NPE];
 #pragma unroll
-    for (int i = 0; i < NPE; ++i) {
-        load_node_v<ND>(p, conn_at(p, i, e), v[i]);
-        sx[i] = shp_at(p, 0, i, e);
-        sy[i] = ND == 3 ? shp_at(p, 1, i, e) : 0.0;
-        sz[i] = shp_at(p, ND - 1, i, e);
-    }
+    for (int i = 0; i < NPE; ++i) load_node_v<ND>(p, conn_at(p, i, e), v[i]);
+    load_shp<ND>(p, e, sx, sy, sz);
     strain_rate_vals<ND>(v, sx, sy, sz, s);
 }
 
@@ -103,98 +111,109 @@ __global__ void __launch_bounds__(TPB) k_strain_rate(KP p, int begin_step)
 // ==================================================================
 // nodal gathers: heat (fields.cxx:99-146) and dvoldt (geometry.cxx:111-155)
 // ==================================================================
-// contribution of element e to tdot of its local node i
+// The element's contributions to its nodes' tdot (slot i of hc64).  The
+// stencil D_ij = dN_i . dN_j is formed once per element: D_ji is the same
+// products in the same order, so every slot holds the value that a gather's
+// term for (e, i) has, at 10 instead of 16 dot products.
 template <int ND>
-__device__ __forceinline__ double heat_term(const KP &p, int e, int i)
+__device__ __forceinline__ void heat_terms(const KP &p, int e, double vol, const double *sx, const double *sy,
+                                           const double *sz)
 {
     constexpr int NPE = ND + 1;
-    double vol = p.vol[e];
-    double kv = m_k(p, e) * vol;
-    double rh = m_hr_over_cp(p, e) * vol;
-    double sxi = shp_at(p, 0, i, e), szi = shp_at(p, ND - 1, i, e);
-    double syi = (ND == 3) ? shp_at(p, 1, i, e) : 0.0;
-    double diffusion = 0;
+    const double kv = m_k(p, e) * vol;
+    const double rh = m_hr_over_cp(p, e) * vol;
+    double T[NPE], D[NPE][NPE];
 #pragma unroll
-    for (int j = 0; j < NPE; ++j) {
-        double sxj = shp_at(p, 0, j, e), szj = shp_at(p, ND - 1, j, e);
-        double D;
-        if (ND == 3) {
-            double syj = shp_at(p, 1, j, e);
-            D = (sxi * sxj + syi * syj + szi * szj);
-        } else {
-            D = (sxi * sxj + szi * szj);
+    for (int i = 0; i < NPE; ++i) T[i] = p.T[conn_at(p, i, e)];
+#pragma unroll
+    for (int i = 0; i < NPE; ++i)
+#pragma unroll
+        for (int j = i; j < NPE; ++j) {
+            D[i][j] = (ND == 3) ? (sx[i] * sx[j] + sy[i] * sy[j] + sz[i] * sz[j])
+                                : (sx[i] * sx[j] + sz[i] * sz[j]);
+            D[j][i] = D[i][j];
         }
-        diffusion += D * p.T[conn_at(p, j, e)];
+#pragma unroll
+    for (int i = 0; i < NPE; ++i) {
+        double diffusion = D[i][0] * T[0];
+#pragma unroll
+        for (int j = 1; j < NPE; ++j) diffusion += D[i][j] * T[j];
+        p.hc64[(size_t)i * p.ne + e] = diffusion * kv - rh;
     }
-    return diffusion * kv - rh;
 }
 
-template <int ND, bool HEAT, bool DVOLDT, bool STAGED>
-__global__ void __launch_bounds__(192) k_node_gather1(KP p)
+// des_update_temperature: the elements' heat terms (bound by the FP64 pipe),
+// then each node's sum and update (bound by the gather's latency).  118,326
+// tets: 26 and 14 us, where a gather that formed each entry's stencil took 42
+// us and the update its own launch.
+template <int ND>
+__global__ void __launch_bounds__(TPB) k_heat_terms(KP p)
 {
-    constexpr int NQ = (int)HEAT + (int)DVOLDT;
-    double sum[NQ];
-    const int n = node_sums<SumF64, NQ, ND, STAGED>(
-        p.sup_off, 0, p.nn, NQ,
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= p.ne) return;
+    double sx[ND + 1], sy[ND + 1], sz[ND + 1];
+    load_shp<ND>(p, e, sx, sy, sz);
+    heat_terms<ND>(p, e, p.vol[e], sx, sy, sz);
+}
+
+// temperature update + Dirichlet BC (fields.cxx:151-162)
+__device__ __forceinline__ void update_temperature(const KP &p, int n, double tdot, double tmass)
+{
+    const unsigned flag = p.bcflag[n];
+    if (flag & BOUNDZ1) p.T[n] = p.prm.surface_temperature;
+    else if ((flag & BOUNDZ0) && !p.prm.has_fixed_bottom_temperature) p.T[n] = p.prm.mantle_temperature;
+    else p.T[n] -= tdot * p.clk->dt / tmass;
+}
+
+template <int ND, bool STAGED>
+__global__ void __launch_bounds__(192) k_heat_sum(KP p)
+{
+    double tdot;
+    const int n = node_sums<SumF64, 1, ND, STAGED>(
+        p.sup_off, 0, p.nn, 1,
         [&](int q, double *t) {
             const int ent = p.sup_ent[q];
-            const int e = ent >> 2, i = ent & 3;
-            if (HEAT) t[0] = heat_term<ND>(p, e, i);
-            if (DVOLDT) {
-                double dj;
-                if (ND == 3) dj = p.srate[e] + p.srate[(size_t)p.ne + e] + p.srate[2 * (size_t)p.ne + e];
-                else dj = p.srate[e] + p.srate[(size_t)p.ne + e];
-                t[NQ - 1] = dj * p.vol[e];
-            }
+            *t = p.hc64[(size_t)(ent & 3) * p.ne + (ent >> 2)];
         },
-        FromZero<SumF64>(), sum);
+        FromZero<SumF64>(), &tdot);
     if (n < 0) return;
-    if (HEAT) p.tdot[n] = sum[0];
-    if (DVOLDT) p.ntmp[n] = sum[NQ - 1] / p.vol_n[n];
+    p.tdot[n] = tdot;
+    update_temperature(p, n, tdot, p.tmass[n]);
+}
+
+template <int ND, bool STAGED>
+__global__ void __launch_bounds__(192) k_dvoldt(KP p)
+{
+    double sum;
+    const int n = node_sums<SumF64, 1, ND, STAGED>(
+        p.sup_off, 0, p.nn, 1,
+        [&](int q, double *t) {
+            const int e = p.sup_ent[q] >> 2;
+            double dj;
+            if (ND == 3) dj = p.srate[e] + p.srate[(size_t)p.ne + e] + p.srate[2 * (size_t)p.ne + e];
+            else dj = p.srate[e] + p.srate[(size_t)p.ne + e];
+            *t = dj * p.vol[e];
+        },
+        FromZero<SumF64>(), &sum);
+    if (n >= 0) p.ntmp[n] = sum / p.vol_n[n];
 }
 
 // The fused step's form of the same three functions (update_strain_rate,
 // the heat gather of update_temperature, compute_dvoldt), element-centric.
 // k_elem_pass writes the strain rate, the element's dvoldt term qv = tr(edot)
-// vol and, with heat (elem_terms, which returns qv), its contribution to each
-// of its nodes' tdot (slot i of hc64).  The stencil D_ij = dN_i . dN_j is formed once per element: D_ji is
-// the same products in the same order, so every slot holds the very value
-// heat_term gives for (e, i), at 10 instead of 16 dot products.
+// vol and, with heat, its heat terms (elem_terms, which returns qv).
 // k_node_pass sums the slots and the qv over each node's support in
 // ascending element order -- the node-centric kernels' order -- and applies
-// the temperature update.  The bits are those of k_strain_rate,
-// k_node_gather1 and k_temperature_update.
+// the temperature update.  The bits are those of k_strain_rate, k_dvoldt and
+// k_heat_sum.
 template <int ND>
 __device__ __forceinline__ double elem_terms(const KP &p, int e, const double *sr, double vol, const double *sx,
                                              const double *sy, const double *sz, bool heat)
 {
-    constexpr int NPE = ND + 1;
-    const size_t ne = p.ne;
     double dj;
     if (ND == 3) dj = sr[0] + sr[1] + sr[2];
     else dj = sr[0] + sr[1];
-    if (heat) {
-        const double kv = m_k(p, e) * vol;
-        const double rh = m_hr_over_cp(p, e) * vol;
-        double T[NPE], D[NPE][NPE];
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) T[i] = p.T[conn_at(p, i, e)];
-#pragma unroll
-        for (int i = 0; i < NPE; ++i)
-#pragma unroll
-            for (int j = i; j < NPE; ++j) {
-                D[i][j] = (ND == 3) ? (sx[i] * sx[j] + sy[i] * sy[j] + sz[i] * sz[j])
-                                    : (sx[i] * sx[j] + sz[i] * sz[j]);
-                D[j][i] = D[i][j];
-            }
-#pragma unroll
-        for (int i = 0; i < NPE; ++i) {
-            double diffusion = D[i][0] * T[0];
-#pragma unroll
-            for (int j = 1; j < NPE; ++j) diffusion += D[i][j] * T[j];
-            p.hc64[(size_t)i * ne + e] = diffusion * kv - rh;
-        }
-    }
+    if (heat) heat_terms<ND>(p, e, vol, sx, sy, sz);
     return dj * vol;
 }
 
@@ -214,12 +233,7 @@ __global__ void __launch_bounds__(TPB) k_elem_pass(KP p, int heat)
 #pragma unroll
     for (int c = 0; c < NSTR; ++c) p.srate[(size_t)c * ne + e] = sr[c];
     double sx[NPE], sy[NPE], sz[NPE];
-#pragma unroll
-    for (int i = 0; i < NPE; ++i) {
-        sx[i] = shp_at(p, 0, i, e);
-        sy[i] = ND == 3 ? shp_at(p, 1, i, e) : 0.0;
-        sz[i] = shp_at(p, ND - 1, i, e);
-    }
+    load_shp<ND>(p, e, sx, sy, sz);
     p.qv[e] = elem_terms<ND>(p, e, sr, p.vol[e], sx, sy, sz, heat != 0);
 }
 
@@ -267,25 +281,17 @@ __global__ void __launch_bounds__(192) k_node_pass(KP p, int heat)
         if (heat) tmass = p.tmass[n];
     }
     p.ntmp[n] = sum[0] / vol_n;
-    if (heat) {   // temperature update + Dirichlet BC (fields.cxx:151-162)
-        const double tdot = sum[1];
-        p.tdot[n] = tdot;
-        const unsigned flag = p.bcflag[n];
-        if (flag & BOUNDZ1) p.T[n] = p.prm.surface_temperature;
-        else if ((flag & BOUNDZ0) && !p.prm.has_fixed_bottom_temperature) p.T[n] = p.prm.mantle_temperature;
-        else p.T[n] -= tdot * p.clk->dt / tmass;
+    if (heat) {
+        p.tdot[n] = sum[1];
+        update_temperature(p, n, sum[1], tmass);
     }
 }
 
-// temperature update + Dirichlet BC (fields.cxx:151-162)
+// the update alone, from p.tdot (mixed contexts)
 __global__ void __launch_bounds__(TPB) k_temperature_update(KP p)
 {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.nn) return;
-    unsigned flag = p.bcflag[n];
-    if (flag & BOUNDZ1) p.T[n] = p.prm.surface_temperature;
-    else if ((flag & BOUNDZ0) && !p.prm.has_fixed_bottom_temperature) p.T[n] = p.prm.mantle_temperature;
-    else p.T[n] -= p.tdot[n] * p.clk->dt / p.tmass[n];
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n < p.nn) update_temperature(p, n, p.tdot[n], p.tmass[n]);
 }
 
 // compute_edvoldt (geometry.cxx:158-179)
@@ -1164,7 +1170,7 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
             }
         }
         if (flags & GEO_MASS_TERMS) {
-            // compute_mass element terms (geometry.cxx:313-365), as k_mass forms them
+            // compute_mass element terms (geometry.cxx:313-365)
             const double rho_e = p.rho_e ? p.rho_e[e] : m_rho<ND>(p, e);
             const double pseudo_speed = p.prm.max_vbc_val * p.prm.inertial_scaling;
             const double rho = p.prm.is_quasi_static
@@ -1239,66 +1245,42 @@ __global__ void k_dt_reset(KP p)
 // ==================================================================
 // compute_mass (geometry.cxx:313-365)
 // ==================================================================
-// The node sums of compute_mass: volume_n, mass and, with heat, tmass.  DW (a
-// mixed context): compensated FP32 sums (des_dw.cuh).  terms(e, t) gives an
-// element's three terms.
-template <int ND, bool DW, bool STAGED, class Terms>
-__device__ __forceinline__ void mass_sums(const KP &p, int lo, int hi, Terms terms)
+// The node sums of compute_mass -- volume_n, mass and, with heat, tmass --
+// from the element terms that the geometry pass wrote (GEO_MASS_TERMS).  DW
+// (a mixed context): compensated FP32 sums (des_dw.cuh).  Bound by the
+// gather's latency; 118,326 tets in FP64 11 us beside the geometry pass, where
+// a gather that formed the terms for each support entry took 26 us.
+template <int ND, bool DW, bool STAGED>
+__global__ void __launch_bounds__(192) k_mass_sum(KP p)
 {
     const bool thermal = p.prm.has_thermal_diffusion;
     double sum[3] = {0, 0, 0};
     int n;
     if constexpr (DW) {
         n = node_sums<SumDw, 3, ND, STAGED>(
-            p.sup_off, lo, hi, thermal ? 3 : 2,
+            p.sup_off, p.n_lo, p.n_hi, thermal ? 3 : 2,
             [&](int q, float2 *t) {
-                double d[3];
-                terms(p.sup_ent[q] >> 2, d);
-                t[0] = pair_of(dw_split(d[0]));
-                t[1] = pair_of(dw_split(d[1]));
-                if (thermal) t[2] = pair_of(dw_split(d[2]));
+                const int e = p.sup_ent[q] >> 2;
+                t[0] = pair_of(dw_split(p.vol[e]));
+                t[1] = pair_of(dw_split(p.me[e]));
+                if (thermal) t[2] = pair_of(dw_split(p.tme[e]));
             },
             FromZero<SumDw>(), sum);
     } else {
         n = node_sums<SumF64, 3, ND, STAGED>(
-            p.sup_off, lo, hi, thermal ? 3 : 2, [&](int q, double *t) { terms(p.sup_ent[q] >> 2, t); },
+            p.sup_off, p.n_lo, p.n_hi, thermal ? 3 : 2,
+            [&](int q, double *t) {
+                const int e = p.sup_ent[q] >> 2;
+                t[0] = p.vol[e];
+                t[1] = p.me[e];
+                if (thermal) t[2] = p.tme[e];
+            },
             FromZero<SumF64>(), sum);
     }
     if (n < 0) return;
     p.vol_n[n] = sum[0];
     p.mass[n] = sum[1];
     p.tmass[n] = thermal ? sum[2] : 0.0;
-}
-
-template <int ND, bool DW, bool STAGED>
-__global__ void __launch_bounds__(192) k_mass(KP p)
-{
-    constexpr int NPE = ND + 1;
-    const double pseudo_speed = p.prm.max_vbc_val * p.prm.inertial_scaling;
-    const bool quasi = p.prm.is_quasi_static, thermal = p.prm.has_thermal_diffusion;
-    mass_sums<ND, DW, STAGED>(p, 0, p.nn, [&](int e, double *t) {
-        const double vol = p.vol[e];
-        const double rho_e = p.rho_e ? p.rho_e[e] : m_rho<ND>(p, e);
-        const double rho = quasi
-            ? ((p.mat.nmat == 1) ? p.mat.rho_pseudo : m_bulkm(p, e) / (pseudo_speed * pseudo_speed))
-            : rho_e;
-        t[0] = vol;
-        t[1] = rho * vol / NPE;
-        t[2] = thermal ? rho_e * m_cp(p, e) * vol / NPE : 0.0;
-    });
-}
-
-// the node sums of compute_mass from the element terms that the geometry
-// pass wrote (GEO_MASS_TERMS): per pair 3 additions instead of the terms
-template <int ND, bool DW, bool STAGED>
-__global__ void __launch_bounds__(192) k_mass_sum(KP p)
-{
-    const bool thermal = p.prm.has_thermal_diffusion;
-    mass_sums<ND, DW, STAGED>(p, p.n_lo, p.n_hi, [&](int e, double *t) {
-        t[0] = p.vol[e];
-        t[1] = p.me[e];
-        t[2] = thermal ? p.tme[e] : 0.0;
-    });
 }
 
 // ==================================================================
@@ -1512,17 +1494,18 @@ int launch_strain_rate(const KP &p, cudaStream_t s, bool begin_step)
     return 1;
 }
 
-int launch_heat_gather(const KP &p, cudaStream_t s)
+int launch_update_temperature(const KP &p, cudaStream_t s)
 {
-    if (p.nd == 3) DES_NODES((k_node_gather1<3, true, false, STAGED>), p.nn, s, p);
-    else DES_NODES((k_node_gather1<2, true, false, STAGED>), p.nn, s, p);
-    return 1;
+    DISPATCH(k_heat_terms, p.ne, p);
+    if (p.nd == 3) DES_NODES((k_heat_sum<3, STAGED>), p.nn, s, p);
+    else DES_NODES((k_heat_sum<2, STAGED>), p.nn, s, p);
+    return 2;
 }
 
 int launch_dvoldt(const KP &p, cudaStream_t s)
 {
-    if (p.nd == 3) DES_NODES((k_node_gather1<3, false, true, STAGED>), p.nn, s, p);
-    else DES_NODES((k_node_gather1<2, false, true, STAGED>), p.nn, s, p);
+    if (p.nd == 3) DES_NODES((k_dvoldt<3, STAGED>), p.nn, s, p);
+    else DES_NODES((k_dvoldt<2, STAGED>), p.nn, s, p);
     return 1;
 }
 
@@ -1664,14 +1647,6 @@ int launch_geometry_ahead(const KP &p, cudaStream_t s, int flags)
     if (p.nd == 3 && p.shpdw) DES_LAUNCH((k_geometry_ahead<3, true>), n, s, p, flags);
     else if (p.nd == 3) DES_LAUNCH((k_geometry_ahead<3, false>), n, s, p, flags);
     else DES_LAUNCH((k_geometry_ahead<2, false>), n, s, p, flags);
-    return 1;
-}
-
-int launch_mass(const KP &p, cudaStream_t s)
-{
-    if (p.nd == 3 && p.shpdw) DES_NODES((k_mass<3, true, STAGED>), p.nn, s, p);
-    else if (p.nd == 3) DES_NODES((k_mass<3, false, STAGED>), p.nn, s, p);
-    else DES_NODES((k_mass<2, false, STAGED>), p.nn, s, p);
     return 1;
 }
 

@@ -51,7 +51,7 @@ enum GeoFlags : int {
 
 // Each launcher returns the number of kernels it launched.
 int launch_strain_rate(const KP &p, cudaStream_t s, bool begin_step);
-int launch_heat_gather(const KP &p, cudaStream_t s);              // tdot -> p.tdot
+int launch_update_temperature(const KP &p, cudaStream_t s);       // tdot -> p.tdot, T (FP64 contexts)
 int launch_temperature_update(const KP &p, cudaStream_t s);       // T from p.tdot
 int launch_dvoldt(const KP &p, cudaStream_t s);                   // -> ntmp
 // the FP64 step's element-centric form of strain rate + heat gather + dvoldt
