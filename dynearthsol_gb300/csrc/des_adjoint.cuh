@@ -60,7 +60,7 @@ struct AdjBufs {
 
 // Device-to-device copies of FP64 arrays in one launch: the dozen arrays of a
 // tape record cost a few microseconds each as separate copies.
-constexpr int COPY_MAX = 14;
+constexpr int COPY_MAX = 16;
 struct CopyTable {
     const double *src[COPY_MAX];
     double *dst[COPY_MAX];

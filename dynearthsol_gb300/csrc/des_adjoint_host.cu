@@ -4,9 +4,14 @@
 //
 // Memory: a checkpoint holds the state and its derived fields (~180 B per
 // tet); the tape of one segment holds checkpoint_every + 1 step records
-// (~319 B per tet each, the forward values the reverse kernels read; the
+// (~311 B per tet each, the forward values the reverse kernels read; the
 // stress after NMD_stress is rebuilt from them).  At 1M tets and 50 steps
 // per segment that is ~16 GB of HBM.
+//
+// A taped step works on the tape: it reads its start state from its record,
+// writes its intermediates there and the state it ends with to the next
+// record.  Only the nodes' x, v and T, which the step updates in place, are
+// copied (56 B per node).
 //
 // The forward tapes the window's last segment itself: it writes each of
 // its steps' records as it goes, so the backward, which reverses that
@@ -102,6 +107,14 @@ int copy_state(const StateRef &dst, const StateRef &src, size_t nn, size_t ne, c
     CopyTable t;
     add_copies(t, dst, src, nn, ne);
     return launch_copy_arrays(t, s);
+}
+
+// the nodes' part of a state that a taped step does not leave on the tape
+void add_motion(CopyTable &ct, const TapeStep &t, const KP &p, size_t nn)
+{
+    ct.add(t.x, p.x, 3 * nn);
+    ct.add(t.v, p.v, 3 * nn);
+    ct.add(t.T, p.T, nn);
 }
 
 // Writes to every page of an output array that a copy is about to fill.  The
@@ -215,7 +228,7 @@ int alloc_buffers(des_ctx *c, AdjWork *w)
     return DES_OK;
 }
 
-void add_tape_step(Carver &cv, TapeStep &t, size_t nn, size_t ne)
+void add_tape_step(Carver &cv, TapeStep &t, size_t nn, size_t ne, bool first)
 {
     const size_t D = sizeof(double);
     cv.add((void **)&t.x, 3 * nn * D);
@@ -223,7 +236,7 @@ void add_tape_step(Carver &cv, TapeStep &t, size_t nn, size_t ne)
     cv.add((void **)&t.T, nn * D);
     cv.add((void **)&t.s, 6 * ne * D);
     cv.add((void **)&t.pls, ne * D);
-    cv.add((void **)&t.volo, ne * D);
+    if (first) cv.add((void **)&t.volo, ne * D);   // the others': the volume of the step before
     cv.add((void **)&t.vol, ne * D);
     cv.add((void **)&t.shp, 12 * ne * D);
     cv.add((void **)&t.mass, nn * D);
@@ -254,16 +267,17 @@ int alloc_tape(des_ctx *c, AdjWork *w, int cap)
     // the whole tape against the free device memory, before any allocation
     // (the host records too are sized by cap)
     TapeStep probe{};
-    Carver one;
-    add_tape_step(one, probe, nn, ne);
-    const size_t need = one.total() * ((size_t)cap + 1);
+    Carver first, other;
+    add_tape_step(first, probe, nn, ne, true);
+    add_tape_step(other, probe, nn, ne, false);
+    const size_t need = first.total() + other.total() * (size_t)cap;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need > free_b)
         return ctx_fail(c, DES_ENOMEM, "adjoint tape of %d steps: %zu bytes, %zu free on the device", cap, need,
                         free_b);
     w->tape.assign((size_t)cap + 1, TapeStep{});
     Carver cv2;
-    for (auto &t : w->tape) add_tape_step(cv2, t, nn, ne);
+    for (auto &t : w->tape) add_tape_step(cv2, t, nn, ne, &t == w->tape.data());
     cudaError_t e = cudaMalloc((void **)&w->tape_mem, cv2.total());
     if (e != cudaSuccess) {
         (void)cudaGetLastError();   // reported here, not at the next launch check
@@ -272,58 +286,69 @@ int alloc_tape(des_ctx *c, AdjWork *w, int cap)
                         cudaGetErrorString(e));
     }
     cv2.assign(w->tape_mem);
+    for (size_t k = 1; k < w->tape.size(); ++k) w->tape[k].volo = w->tape[k - 1].vol;
     w->cap = cap;
     return DES_OK;
 }
 
-// one FP64 step with dt held (the fused step's kernels without compute_dt);
-// with a tape record, the start state and the forward values the reverse
-// kernels read are copied into it
-int adj_step(des_ctx *c, const TapeStep *t)
+// One FP64 step with dt held: the chained step's kernels without compute_dt
+// (a segment's first step forms its element terms itself, its last leaves
+// the state complete).  With a tape record t the step works on the tape: its
+// arrays are t's where the reverse kernels read them and the next record's
+// (tn) for the state it ends with, so that nothing is copied but the nodes'
+// x, v and T.  Copied instead (the start state and the intermediates, ~319 B
+// per tet read and written in four launches) and with a pass of its own for
+// the element terms, a step took: a window of 50 steps of 14,400 tets and its
+// reverse 14.1 ms, now 12.4 ms; 40 steps of 998,400 tets 156 and 147 ms.
+int adj_step(des_ctx *c, const TapeStep *t, const TapeStep *tn, bool first, bool last)
 {
     KP p = ctx_step_kp(c);
-    if (t) {   // the rheology writes the viscosity and the EVP branch it took
-        p.tape_visc = t->visc;
-        p.tape_evp = t->evp;
-    }
     cudaStream_t s = c->stream;
-    const size_t nn = c->nn, ne = c->ne;
+    const size_t nn = c->nn;
     const bool thermal = p.prm.has_thermal_diffusion != 0;
     int n = 0;
-    if (t) n += copy_state(tape_state(*t), live_state(c), nn, ne, s);
-    // strain rate, heat and dvoldt as the fused FP64 step forms them
-    n += launch_elem_pass(p, s, thermal);
-    n += launch_node_pass(p, s, thermal);
-    if (t) {   // the stress pass corrects the strain rate and the NMD gather reuses ntmp
-        CopyTable ct;
-        ct.add(t->edot, p.srate, 6 * ne);
-        ct.add(t->ntmp, p.ntmp, nn);
-        if (thermal) ct.add(t->tdot, p.tdot, nn);
-        n += launch_copy_arrays(ct, s);
+    if (t) {
+        if (first) {
+            n += copy_state(tape_state(*t), live_state(c), nn, c->ne, s);
+        } else {
+            CopyTable ct;
+            add_motion(ct, *t, p, nn);
+            n += launch_copy_arrays(ct, s);
+        }
+        p.stress = t->s, p.sstar = t->sstar;
+        p.pls = t->pls, p.pls_out = tn->pls;
+        p.vol_old = t->volo, p.vol = t->vol, p.shp = t->shp;
+        p.mass = t->mass, p.tmass = t->tmass, p.vol_n = t->voln;
+        p.srate = t->edot;
+        p.tdot = t->tdot, p.ntmp = t->ntmp;
+        p.edvoldt = t->edv, p.dp = t->dp, p.rho_e = t->rho, p.f = t->f;
+        p.tape_visc = t->visc;   // the viscosity and the EVP branch the rheology takes
+        p.tape_evp = t->evp;
     }
+    if (first) n += launch_elem_pass(p, s, thermal);
+    n += launch_node_pass(p, s, thermal, !first);
     n += launch_update_stress(p, s, true);
-    n += launch_nmd_gather(p, s);
-    if (t) {   // the stress after update_stress, before the NMD correction; dpn is final
-        CopyTable ct;
-        ct.add(t->sstar, p.stress, 6 * ne);
-        ct.add(t->dp, p.dp, ne);
-        ct.add(t->rho, p.rho_e, ne);
-        ct.add(t->edv, p.edvoldt, ne);
-        ct.add(t->dpn, p.ntmp, nn);
-        n += launch_copy_arrays(ct, s);
+    if (t) {   // the NMD correction and what follows write the next record's stress
+        p.ntmp = t->dpn;
+        p.stress = tn->s;
     }
+    n += launch_nmd_gather(p, s);
     n += launch_nmd_correct(p, s, true);
     n += launch_force(p, s, true);
-    // mass from the geometry pass's element terms: the same sums, in the same
-    // order, as compute_mass's
-    int geo = GEO_COPY_OLD | GEO_VOLUME | GEO_SHAPE | GEO_MASS_TERMS;
+    int geo = GEO_VOLUME | GEO_SHAPE | GEO_MASS_TERMS;
     if (p.mat.rheol_type & DES_RH_ELASTIC) geo |= GEO_ROTATE;
-    n += launch_geometry(p, s, geo);
-    n += launch_mass_sum(p, s);
     if (t) {
-        CopyTable ct;
-        ct.add(t->f, p.f, 3 * nn);
-        n += launch_copy_arrays(ct, s);
+        p.vol = tn->vol, p.shp = tn->shp;
+        p.mass = tn->mass, p.tmass = tn->tmass, p.vol_n = tn->voln;
+        p.srate = tn->edot;
+    } else {
+        geo |= GEO_COPY_OLD;
+    }
+    if (last) {
+        n += launch_geometry(p, s, geo);
+        n += launch_mass_sum(p, s);
+    } else {
+        n += launch_geometry_ahead(p, s, geo);
     }
     return ctx_check_launch(c, n);
 }
@@ -399,10 +424,29 @@ int des_adjoint_forward(des_ctx *c, int nsteps, int checkpoint_every)
     w->dt = clk.dt;
     for (int k = 0; k < nsteps; ++k) {
         if (k % C == 0 && (rc = ctx_check_launch(c, copy_state(w->ck[k / C], live_state(c), nn, ne, c->stream)))) return rc;
-        if ((rc = adj_step(c, k >= last0 ? &w->tape[k - last0] : nullptr))) return rc;
+        const TapeStep *t = k >= last0 ? &w->tape[k - last0] : nullptr;
+        const bool last = (k + 1) % C == 0 || k + 1 == nsteps;
+        if ((rc = adj_step(c, t, t ? t + 1 : nullptr, k % C == 0, last))) return rc;
     }
-    if ((rc = ctx_check_launch(c, copy_state(tape_state(w->tape[nsteps - last0]), live_state(c), nn, ne, c->stream))))
-        return rc;
+    {   // the final record's nodes, and the context's arrays from the tape's
+        const KP &p = c->kp;
+        const TapeStep &t = w->tape[nsteps - last0 - 1], &tn = w->tape[nsteps - last0];
+        CopyTable ct;
+        add_motion(ct, tn, p, nn);
+        ct.add(p.stress, tn.s, 6 * ne);
+        ct.add(p.pls, tn.pls, ne);
+        ct.add(p.vol_old, tn.volo, ne);
+        ct.add(p.vol, tn.vol, ne);
+        ct.add(p.shp, tn.shp, 12 * ne);
+        ct.add(p.mass, tn.mass, nn);
+        ct.add(p.tmass, tn.tmass, nn);
+        ct.add(p.vol_n, tn.voln, nn);
+        ct.add(p.edvoldt, t.edv, ne);
+        ct.add(p.dp, t.dp, ne);
+        ct.add(p.ntmp, t.dpn, nn);
+        ct.add(p.f, t.f, 3 * nn);
+        if ((rc = ctx_check_launch(c, launch_copy_arrays(ct, c->stream)))) return rc;
+    }
     CKA(cudaMemcpyAsync(w->final_pool, c->pool, c->pool_bytes, cudaMemcpyDeviceToDevice, c->stream));
     w->K = nsteps;
     w->C = C;
@@ -440,8 +484,10 @@ int des_adjoint_backward(des_ctx *c, const des_host_state *seed, des_host_state 
             w->tape_seg = -1;
             if ((rc = ctx_check_launch(c, copy_state(live_state(c), w->ck[seg], nn, ne, s)))) return rc;
             for (int j = 0; j < L; ++j)
-                if ((rc = adj_step(c, &w->tape[j]))) return rc;
-            if ((rc = ctx_check_launch(c, copy_state(tape_state(w->tape[L]), live_state(c), nn, ne, s)))) return rc;
+                if ((rc = adj_step(c, &w->tape[j], &w->tape[j + 1], j == 0, j + 1 == L))) return rc;
+            CopyTable ct;
+            add_motion(ct, w->tape[L], c->kp, nn);
+            if ((rc = ctx_check_launch(c, launch_copy_arrays(ct, s)))) return rc;
             w->tape_seg = seg;
         }
         for (int j = L - 1; j >= 0; --j)

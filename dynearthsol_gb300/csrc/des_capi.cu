@@ -480,6 +480,9 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     p.eprop = nullptr;   // set once k_elem_props has filled d_eprop
     p.rho_e = nullptr;
     p.tdot = p.ntmp;
+    p.srate_out = p.srate;
+    p.sstar = p.stress;
+    p.pls_out = p.pls;
     p.sh32 = mixed3 ? (float *)p.me : nullptr;
     p.shpdw = d_shpdw;
     p.vdw = d_vdw;

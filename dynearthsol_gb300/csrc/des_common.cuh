@@ -133,6 +133,11 @@ struct KP {
     // the FP64 step's: -(sigma . dN_i/dx + buoyancy z) vol, one (2D) or two
     // (3D, the last value unused) double2 per support-list entry
     double2 *ft64;
+    // where the FP64 stress pass writes what it forms from srate, stress and
+    // pls: the corrected strain rate, the stress before the NMD correction and
+    // the plastic strain.  The same arrays, but for the reverse mode's taped
+    // steps, whose inputs stay on the tape.
+    double *srate_out, *sstar, *pls_out;
     // set only by the reverse mode's forward recompute: the viscosity the
     // rheology used and the EVP branch it took (1: elasto-plastic), per element
     double *tape_visc;

@@ -339,12 +339,12 @@ __global__ void __launch_bounds__(TPB) k_update_stress(KP p, int fused)
                                            p.vol_old[e], dpr);
 #pragma unroll
     for (int c = 0; c < NSTR; ++c) {
-        p.stress[c * ne + e] = s[c];
+        p.sstar[c * ne + e] = s[c];
         p.strain[c * ne + e] = es[c];
-        p.srate[c * ne + e] = edot[c];
+        p.srate_out[c * ne + e] = edot[c];
     }
     p.syy[e] = syy;
-    p.pls[e] = pls;
+    p.pls_out[e] = pls;
     p.dpls[e] = dpls;
     p.dp[e] = dpr;
     if (fused && p.rho_e) p.rho_e[e] = m_rho<ND>(p, e);   // temperature is final for this step
@@ -535,10 +535,9 @@ __global__ void __launch_bounds__(TPB) k_elem_force(KP p)
         const int e = p.e_lo + (SPLIT ? t >> 2 : t);
         const size_t ne = p.ne;
         double s[NSTR];
-        if (TERMS) {
+        const double *from = CORRECT ? p.sstar : p.stress;
 #pragma unroll
-            for (int c = 0; c < NSTR; ++c) s[c] = p.stress[c * ne + e];
-        }
+        for (int c = 0; c < (TERMS ? NSTR : ND); ++c) s[c] = from[c * ne + e];
         if (CORRECT) {
             double dpn = p.ntmp[conn_at(p, 0, e)];
 #pragma unroll
@@ -550,9 +549,13 @@ __global__ void __launch_bounds__(TPB) k_elem_force(KP p)
             if (SPLIT) __syncwarp(0xfu << (threadIdx.x & 28));
 #pragma unroll
             for (int c = 0; c < ND; ++c) {
-                if (TERMS) s[c] += corr;
-                else s[c] = p.stress[c * ne + e] + corr;
+                s[c] += corr;
                 if (!SPLIT || (t & 3) == 0) p.stress[c * ne + e] = s[c];
+            }
+            // a taped step: the shear components too, to the next record
+            if (TERMS && !PAIRS && p.sstar != p.stress && (!SPLIT || (t & 3) == 0)) {
+#pragma unroll
+                for (int c = ND; c < NSTR; ++c) p.stress[c * ne + e] = s[c];
             }
         }
         if constexpr (PAIRS) {
