@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(TPB_A) k_adj_end_geometry(KP p, AdjBufs a, Tap
 int launch_adj_end_geometry(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
                             cudaStream_t s)
 {
-    DES_LAUNCH_A(k_adj_end_geometry, p.ne, s, p, a, t, t1, dt);
+    DES_LAUNCH_W(k_adj_end_geometry, p.ne, s, p, a, t, t1, dt);
     return 1;
 }
 
@@ -507,7 +507,7 @@ int launch_adj_force(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStrea
         DES_LAUNCH_A(k_adj_facets, p.nbf, s, p, a, t);
         ++n;
     }
-    DES_LAUNCH_A(k_adj_force, p.ne, s, p, a, t);
+    DES_LAUNCH_W(k_adj_force, p.ne, s, p, a, t);
     return n + 1;
 }
 
@@ -1179,7 +1179,7 @@ int launch_copy_arrays(CopyTable &t, cudaStream_t s)
 int launch_adj_stress(const KP &p, const AdjBufs &a, const TapeStep &t, const TapeStep &t1, double dt,
                       cudaStream_t s)
 {
-    DES_LAUNCH_A(k_adj_stress, p.ne, s, p, a, t, t1, dt);
+    DES_LAUNCH_W(k_adj_stress, p.ne, s, p, a, t, t1, dt);
     return 1;
 }
 
@@ -1192,7 +1192,7 @@ int launch_adj_nodes_heat(const KP &p, const AdjBufs &a, const TapeStep &t, cons
 
 int launch_adj_kinematics(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStream_t s)
 {
-    DES_LAUNCH_A(k_adj_kinematics, p.ne, s, p, a, t);
+    DES_LAUNCH_W(k_adj_kinematics, p.ne, s, p, a, t);
     return 1;
 }
 

@@ -1639,7 +1639,7 @@ int launch_geometry(const KP &p, cudaStream_t s, int flags)
 {
     const int n = p.e_hi - p.e_lo;
     if (p.nd == 3 && p.shpdw) DES_LAUNCH((k_geometry<3, true>), n, s, p, flags);
-    else if (p.nd == 3) DES_LAUNCH((k_geometry<3, false>), n, s, p, flags);
+    else if (p.nd == 3) DES_LAUNCH_W((k_geometry<3, false>), n, s, p, flags);
     else DES_LAUNCH((k_geometry<2, false>), n, s, p, flags);
     return 1;
 }
@@ -1648,7 +1648,7 @@ int launch_geometry_ahead(const KP &p, cudaStream_t s, int flags)
 {
     const int n = p.e_hi - p.e_lo;
     if (p.nd == 3 && p.shpdw) DES_LAUNCH((k_geometry_ahead<3, true>), n, s, p, flags);
-    else if (p.nd == 3) DES_LAUNCH((k_geometry_ahead<3, false>), n, s, p, flags);
+    else if (p.nd == 3) DES_LAUNCH_W((k_geometry_ahead<3, false>), n, s, p, flags);
     else DES_LAUNCH((k_geometry_ahead<2, false>), n, s, p, flags);
     return 1;
 }

@@ -37,6 +37,20 @@ inline int grid_blocks(long long n, int most = 256)
 #define DES_LAUNCH(KERNEL, n, s, ...) \
     KERNEL<<<des::grid_blocks(n), des::block_threads(n), 0, (s)>>>(__VA_ARGS__)
 
+// DES_LAUNCH for the 3D FP64 geometry and reverse element kernels, which a
+// small mesh's warps share an SM's FP64 pipe for: up to one wave a warp to a
+// block, so that no SM has more of them than it must.  Measured (blocks of 64
+// / 32 threads): a window of 50 steps of 14,400 tets and its reverse 12.36 /
+// 12.08 ms.  The other kernels, and 2D, take the same time or 0.3% more.
+#define DES_LAUNCH_W(KERNEL, n, s, ...)                                                  \
+    do {                                                                                 \
+        const long long nw_ = (n);                                                       \
+        if (des::one_wave(nw_))                                                          \
+            KERNEL<<<(unsigned)((nw_ + 31) / 32), 32, 0, (s)>>>(__VA_ARGS__);            \
+        else                                                                             \
+            DES_LAUNCH(KERNEL, nw_, s, __VA_ARGS__);                                     \
+    } while (0)
+
 // flags of the element geometry pass
 enum GeoFlags : int {
     GEO_COPY_OLD = 1,    // volume_old <- volume        (dynearthsol.cxx:226)
