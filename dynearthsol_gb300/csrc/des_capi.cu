@@ -312,7 +312,7 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
         std::vector<int> fill(nf_off.begin(), nf_off.end() - 1);
         for (int qq = 0; qq < nbf; ++qq) {
             int e = fac_elem[qq], f = fac_f[qq];
-            for (int j = 0; j < nd; ++j) nf_ent[fill[cn[(size_t)e * npe + (nd == 3 ? F3[f][j] : F2[f][j])]]++] = qq;
+            for (int j = 0; j < nd; ++j) nf_ent[fill[cn[(size_t)e * npe + (nd == 3 ? F3[f][j] : F2[f][j])]]++] = qq * 4 + j;
         }
     }
 

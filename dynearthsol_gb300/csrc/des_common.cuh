@@ -101,7 +101,7 @@ struct KP {
     const int *conn;
     const unsigned *bcflag;
     const int *sup_off, *sup_ent;
-    const int *nf_off, *nf_ent;          // node -> boundary facets (ascending facet id)
+    const int *nf_off, *nf_ent;          // node -> boundary facets (ascending facet id): facet * 4 + the node's corner
     const int *fac_elem, *fac_f, *fac_bdry;
     const int *emark;                    // [nmat][ne] marker counts, or null
     // node fields

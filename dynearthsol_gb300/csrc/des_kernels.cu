@@ -621,7 +621,7 @@ __device__ __forceinline__ void force_tail(const KP &p, int n, double *f, int fu
 {
     // gravity-induced stress BCs, in the reference's facet order
     for (int q = p.nf_off[n]; q < p.nf_off[n + 1]; ++q) {
-        int fq = p.nf_ent[q];
+        const int fq = p.nf_ent[q] >> 2;
 #pragma unroll
         for (int d = 0; d < ND; ++d) f[d] -= p.fv[(size_t)d * p.nbf + fq];
     }
