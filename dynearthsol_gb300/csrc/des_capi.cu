@@ -516,10 +516,9 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     up(d_bc, mesh->bcflag, (size_t)nn * sizeof(unsigned));
     up(d_sup_off, sup_off.data(), sup_off.size() * I);
     up(d_sup_ent, sup_ent.data(), sup_ent.size() * I);
-    {   // the support-list entry of each (element, slot), slot-major
-        std::vector<int> pos((size_t)ne * npe);
-        for (size_t q = 0; q < sup_ent.size(); ++q) pos[(size_t)(sup_ent[q] & 3) * ne + (sup_ent[q] >> 2)] = (int)q;
-        up(d_sup_pos, pos.data(), pos.size() * I);
+    if (e1 == cudaSuccess) {   // done when the stream is waited for below
+        launch_sup_pos(d_sup_ent, d_sup_pos, ne, (long long)sup_ent.size(), c->stream);
+        e1 = cudaGetLastError();
     }
     up(d_nf_off, nf_off.data(), nf_off.size() * I);
     up(d_nf_ent, nf_ent.data(), nf_ent.size() * I);

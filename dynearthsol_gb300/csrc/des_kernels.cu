@@ -1695,16 +1695,15 @@ int launch_quality_scans(const KP &p, cudaStream_t s, double smallest_vol, doubl
     return 1;
 }
 
-__global__ void k_f64_to_f32(const double *__restrict__ a, float *__restrict__ b, long long n)
+__global__ void k_sup_pos(const int *__restrict__ ent, int *__restrict__ pos, int ne, int n)
 {
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < n) b[i] = f32_of(a[i]);   // as the mixed geometry pass rounds them
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < n) pos[(size_t)(ent[q] & 3) * ne + (ent[q] >> 2)] = q;
 }
 
-int launch_f64_to_f32(const double *a, float *b, long long n, cudaStream_t s)
+void launch_sup_pos(const int *ent, int *pos, int ne, long long n, cudaStream_t s)
 {
-    DES_LAUNCH(k_f64_to_f32, n, s, a, b, n);
-    return 1;
+    DES_LAUNCH(k_sup_pos, n, s, ent, pos, ne, (int)n);
 }
 
 // a mixed 3D context's shape functions: the double-word pairs -> FP64 (for downloads)

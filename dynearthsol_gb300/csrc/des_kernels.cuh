@@ -109,8 +109,8 @@ int launch_material_table(const KP &p, cudaStream_t s, double *out);
 // counts; run whenever the counts change
 int launch_elem_props(const KP &p, cudaStream_t s, double *out);
 
-// FP32 copy of an FP64 array
-int launch_f64_to_f32(const double *a, float *b, long long n, cudaStream_t s);
+// the support-list entry of each (element, slot), slot-major, from the lists' n entries
+void launch_sup_pos(const int *ent, int *pos, int ne, long long n, cudaStream_t s);
 // a mixed 3D context's shape functions (p.shpdw non-null; else no launch):
 // the double-word pairs -> FP64 p.shp, for a download
 int launch_shp_join(const KP &p, cudaStream_t s);

@@ -13,17 +13,21 @@
 //   diagonalised in FP32 (branch-free cyclic Jacobi) to screen out the
 //   elements that are elastic by a margin above the FP32 error bound; the
 //   others -- everything at or beyond yield -- run the FP64 return map
-//   (FP64 eigen-solve), so plastic flow is never computed in FP32;
+//   (FP64 eigen-solve), so plastic flow is never computed in FP32.  In the
+//   EVP rheology (k_update_stress_evp3) a cheaper screen on an upper bound
+//   comes first, and the FP64 branches of a block are listed and run side
+//   by side;
 // * the shear strain rates, the spin and the heat stencil: sums of products
 //   of shape function derivatives with nodal values whose sum over the
 //   element vanishes, evaluated in FP32 on FP64 differences (v_i - v_0,
 //   T_j - T_i); the Jaumann rotation increments.  The normal strain rates
-//   stay FP64 (see k_strain_rate_mixed3).
+//   are double-word (see k_strain_rate_mixed3).
 // The elastic and Maxwell increments stay FP64: the quasi-static explicit
 // scheme integrates their rounding without dissipating it (damping option 2
 // only scales the force), and in FP32 they alone moved the stress by 4e-6
 // (relative L2) after 2000 steps of the 998,400-tet workload.
-// Element volumes, shape functions, forces and masses stay FP64.
+// Element volumes and masses stay FP64; shape functions and forces are
+// double-word (des_kernels.cu).
 #include <algorithm>
 #include <cfloat>
 
