@@ -492,7 +492,7 @@ def main():
     alg = STRESS_BYTES_PER_ELEM_FP64 * ne + 16 * nn
     achieved = alg / (k_ms / 1e3) / 1e9
     traffic = profile_traffic(f"update_stress_{args.precision}", args.workload)
-    roofline = {"bound": "hbm", "kernel": "k_update_stress" + ("_mixed3" if args.precision == "mixed" else "<3>"),
+    roofline = {"bound": "hbm", "kernel": "k_update_stress" + ("_evp3" if args.precision == "mixed" else "<3>"),
                 "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                 "traffic": traffic, "kernel_ms": k_ms, "algorithmic_bytes_per_launch": alg,
                 "peak_kind": peak_kind}

@@ -510,8 +510,8 @@ static __device__ __noinline__ void evp_rest(const KP &p, int e, int rest, bool 
 // what it holds.
 // outputs: write the strain rate and edvoldt, which only the end of a call
 // shows (a chained step that another follows leaves them out).
-// Bounds: the FP64 pipe (54 FP64 operations an element off the yield
-// surface, ~75% of its rate) and the issue of the FP32 work beside it.
+// Bounds: the FP64 pipe (48 FP64-pipe instructions an element off the yield
+// surface, 72% of its rate) and the issue of the FP32 work beside it.
 // 998,400 tets: 177 us with the FP64 branches in place, 121 us with the list,
 // 111 us with the shear strain rates as floats (ahead), the density's
 // buoyancy formed where the forces are, and the quarterings, clamps and
