@@ -523,7 +523,7 @@ __device__ __forceinline__ void force_term(const KP &p, int e, int i, const doub
 // Bounds: in FP64 the FP64 pipe (88 operations an element, ~80% of its rate);
 // with pairs the memory (328 B an element).  998,400 tets: 175 us and 58 us
 // for the sums of k_force, where the correction alone and a gather that
-// formed the terms per support entry took 27 and 220 us; pairs 70 us.
+// formed the terms per support entry took 27 and 220 us; pairs 66 us.
 template <int ND, bool CORRECT, bool TERMS, bool PAIRS, bool SPLIT>
 __global__ void __launch_bounds__(TPB) k_elem_force(KP p)
 {
