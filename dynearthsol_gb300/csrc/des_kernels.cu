@@ -1240,11 +1240,6 @@ __global__ void k_dt_finalize(KP p, int only_on_step)
     dt_finalize<ND>(p);
 }
 
-__global__ void k_dt_reset(KP p)
-{
-    p.clk->red_minh = p.clk->red_maxwell = p.clk->red_diffusion = ~0ull;
-}
-
 // ==================================================================
 // compute_mass (geometry.cxx:313-365)
 // ==================================================================
@@ -1666,12 +1661,6 @@ int launch_dt_finalize(const KP &p, cudaStream_t s, bool only_on_step)
 {
     if (p.nd == 3) k_dt_finalize<3><<<1, 1, 0, s>>>(p, (int)only_on_step);
     else k_dt_finalize<2><<<1, 1, 0, s>>>(p, (int)only_on_step);
-    return 1;
-}
-
-int launch_dt_reset(const KP &p, cudaStream_t s)
-{
-    k_dt_reset<<<1, 1, 0, s>>>(p);
     return 1;
 }
 

@@ -101,7 +101,6 @@ int launch_quality_scans(const KP &p, cudaStream_t s, double smallest_vol, doubl
                          int check_bottom, unsigned long long *red);
 // out[4][ne]: density, mesh quality, viscosity, material of an output frame
 int launch_output_elem(const KP &p, double *out, cudaStream_t s);
-int launch_dt_reset(const KP &p, cudaStream_t s);
 // material constants: visc_coef[nmat], then 4 values per plastic table entry
 int launch_material_table(const KP &p, cudaStream_t s, double *out);
 // the per-element blended material properties (KP::eprop) from the marker
