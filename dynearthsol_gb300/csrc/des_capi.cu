@@ -587,6 +587,8 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
                 p.mat.pt_tanphi_f[k] = p.mat.pt_phi[k] == 0 ? 0.0f : (float)p.mat.pt_tanphi[k];
             }
             p.mat.tension_max_f = (float)p.mat.tension_max;
+            p.mat.softens = 0;
+            for (int m = 0; m < nm; ++m) p.mat.softens |= (unsigned)(p.mat.pls0[m] < p.mat.pls1[m]) << m;
             p.mat.pt_n = 2 * nm;
         }
     }

@@ -86,6 +86,7 @@ struct MatC {
     // the quotient by it then leaves tension_max)
     float pt_anphi_f[2 * DES_MAXMAT], pt_sqrt_anphi_f[2 * DES_MAXMAT], pt_tanphi_f[2 * DES_MAXMAT];
     float tension_max_f;
+    unsigned softens;                // bit m: pls0[m] < pls1[m], else the strength drops at once at pls0
 };
 
 // Everything a kernel needs, passed by value.
@@ -592,11 +593,15 @@ struct ScreenTerms {
 // An element whose markers are all of material m and number one, with the
 // material's own friction angles, outside the softening range: the table's
 // angle terms (MatC) and one product or quotient of the cohesion, a few ulps.
+// The ends are plastic_props_one's: at pls0 the start values where the
+// interval is not empty, else the saturated ones.
 __device__ __forceinline__ ScreenTerms screen_terms_table(const KP &p, int e, int m, double pls)
 {
     // +0 at pls0 = 0, the state of nearly all elements, without FP64 compares
-    const bool start = __double_as_longlong(pls) == __double_as_longlong(p.mat.pls0[m]);
-    const int k = (start || pls < p.mat.pls0[m] || pls == p.mat.pls0[m]) ? 2 * m : 2 * m + 1;
+    const bool at0 = __double_as_longlong(pls) == __double_as_longlong(p.mat.pls0[m]);
+    const bool softens = (p.mat.softens >> m) & 1u;
+    const bool start = at0 ? softens : pls < p.mat.pls0[m] || (softens && pls == p.mat.pls0[m]);
+    const int k = start ? 2 * m : 2 * m + 1;
     const double *ef = p.ef[(k & 1) ? DES_EF_COHESION1 : DES_EF_COHESION0];
     const float c = f32_of(ef ? ef[e] : (k & 1) ? p.mat.cohesion1[m] : p.mat.cohesion0[m]);
     return {p.mat.pt_anphi_f[k], 2.0f * c * p.mat.pt_sqrt_anphi_f[k],
