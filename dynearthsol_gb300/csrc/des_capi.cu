@@ -516,10 +516,6 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     up(d_bc, mesh->bcflag, (size_t)nn * sizeof(unsigned));
     up(d_sup_off, sup_off.data(), sup_off.size() * I);
     up(d_sup_ent, sup_ent.data(), sup_ent.size() * I);
-    if (e1 == cudaSuccess) {   // done when the stream is waited for below
-        launch_sup_pos(d_sup_ent, d_sup_pos, ne, (long long)sup_ent.size(), c->stream);
-        e1 = cudaGetLastError();
-    }
     up(d_nf_off, nf_off.data(), nf_off.size() * I);
     up(d_nf_ent, nf_ent.data(), nf_ent.size() * I);
     up(d_fe, fac_elem.data(), fac_elem.size() * I);
@@ -531,17 +527,23 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
         for (int e = 0; e < ne; ++e)
             for (int m = 0; m < mat->nmat; ++m) em[(size_t)m * ne + e] = mat->elemmarkers[(size_t)e * mat->nmat + m];
         up(d_emark, em.data(), em.size() * I);
-        if (e1 == cudaSuccess) {
-            launch_elem_props(p, c->stream, d_eprop);
-            e1 = cudaGetLastError();
-            if (e1 == cudaSuccess) e1 = cudaStreamSynchronize(c->stream);
-            p.eprop = d_eprop;
-        }
     }
-    if (e1 == cudaSuccess) {
-        Clock ck{};
-        ck.red_minh = ck.red_maxwell = ck.red_diffusion = ~0ull;
-        e1 = cudaMemcpy(p.clk, &ck, sizeof ck, cudaMemcpyHostToDevice);
+    Clock ck{};
+    ck.red_minh = ck.red_maxwell = ck.red_diffusion = ~0ull;
+    up(p.clk, &ck, sizeof ck);
+    // a copy from pageable memory may return before its transfer has ended,
+    // and a non-blocking stream is not ordered after it: the kernels that
+    // follow on c->stream read what was copied
+    if (e1 == cudaSuccess) e1 = cudaStreamSynchronize(nullptr);
+    if (e1 == cudaSuccess) {   // done when the stream is waited for below
+        launch_sup_pos(d_sup_ent, d_sup_pos, ne, (long long)sup_ent.size(), c->stream);
+        e1 = cudaGetLastError();
+    }
+    if (d_emark && e1 == cudaSuccess) {
+        launch_elem_props(p, c->stream, d_eprop);
+        e1 = cudaGetLastError();
+        if (e1 == cudaSuccess) e1 = cudaStreamSynchronize(c->stream);
+        p.eprop = d_eprop;
     }
     if (e1 == cudaSuccess) {
         // material constants computed by the device's own functions
