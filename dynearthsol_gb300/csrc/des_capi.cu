@@ -411,29 +411,37 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     float2 *d_shpdw = nullptr, *d_vdw = nullptr, *d_pv = nullptr;
     double4 *d_ndpk = nullptr;
     int *d_sup_pos = nullptr;
-    double2 *d_ft64 = nullptr;
-    double *d_qv = nullptr, *d_hc64 = nullptr;
-    add((void **)&d_qv, (size_t)ne * D);
-    add((void **)&d_ndpk, (size_t)ne * sizeof(double4));
+    double *d_qv = nullptr;
     add((void **)&d_sup_pos, (size_t)ne * npe * I);
+    // a field's AoS rows, or the material table of the context's creation
+    c->stage_doubles = std::max((size_t)ne * std::max(c->nstr, npe), (size_t)nn * nd);
+    c->stage_doubles = std::max(c->stage_doubles, (size_t)9 * DES_MAXMAT);
+    const size_t stage = c->stage_doubles * D, ndpk = (size_t)ne * sizeof(double4), hc = (size_t)ne * npe * D;
+    char *d_scr = nullptr;   // the FP64 contexts' step scratch
     if (mixed3) {
+        add((void **)&d_qv, (size_t)ne * D);
+        add((void **)&d_ndpk, ndpk);
+        add((void **)&p.me, (size_t)ne * 2 * D);   // me, then tme
+        add((void **)&c->d_stage, stage);
         add((void **)&d_hc, (size_t)ne * npe * sizeof(float));
         add((void **)&d_ft, (size_t)ne * npe * 2 * sizeof(float4));
         add((void **)&d_shpdw, (size_t)ne * npe * nd * sizeof(float2));
         add((void **)&d_vdw, (size_t)nn * nd * sizeof(float2));
         add((void **)&d_pv, (size_t)ne * sizeof(float2));
     } else {
-        add((void **)&d_hc64, (size_t)ne * npe * D);
-        add((void **)&d_ft64, (size_t)ne * npe * (nd - 1) * sizeof(double2));
+        // One block for what no two of a step's passes hold at the same
+        // time, all of them on c->stream: the force terms (nd doubles per
+        // support entry, from the stress correction to the force), the terms
+        // that a node pass or a mass sum reads (from the element or geometry
+        // pass before it) and the staging of a field between steps.  Each in
+        // its own array, a 3D context took 651 bytes per tetrahedron; so, 483.
+        add((void **)&d_scr, std::max({hc * nd, ndpk + hc, stage}));
     }
     add((void **)&c->d_rho, (size_t)ne * D);
-    add((void **)&p.me, (size_t)ne * 2 * D);   // me, then tme
     add((void **)&p.fv, (size_t)std::max(nbf, 1) * nd * D);
     add((void **)&p.clk, sizeof(Clock));
     add((void **)&p.err, sizeof(unsigned));
     add((void **)&c->d_red, 4 * sizeof(unsigned long long));
-    c->stage_doubles = std::max((size_t)ne * std::max(c->nstr, npe), (size_t)nn * nd);
-    add((void **)&c->d_stage, c->stage_doubles * D);
     size_t total = 0;
     for (auto &s : slots) total += s.bytes;
     cudaError_t ce = cudaMalloc((void **)&c->pool, total);
@@ -459,6 +467,16 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
             *s.dst = c->pool + off;
             off += s.bytes;
         }
+    }
+    if (!mixed3) {
+        // {ndpk} and, outside the chained step, {qv, me, tme} in its place, then {hc64}
+        d_ndpk = (double4 *)d_scr;
+        d_qv = (double *)d_scr;
+        p.me = d_qv + ne;
+        p.hc64 = (double *)(d_scr + ndpk);
+        p.ft64 = (double2 *)d_scr;
+        p.ft64z = nd == 3 ? (double *)(d_scr + 2 * hc) : nullptr;
+        c->d_stage = (double *)d_scr;
     }
     p.tme = p.me + ne;
     p.nd = nd;
@@ -490,10 +508,8 @@ int create_context(const des_mesh *mesh, const des_params *param, const des_mate
     p.pv = d_pv;
     p.hc = d_hc;
     p.qv = d_qv;
-    p.hc64 = d_hc64;
     p.ft = d_ft;
     p.sup_pos = d_sup_pos;
-    p.ft64 = d_ft64;
     p.e_lo = 0, p.e_hi = ne, p.n_lo = 0, p.n_hi = nn, p.f_lo = 0, p.f_hi = nbf;
     p.fac_order = nullptr;
     p.tape_visc = nullptr;
@@ -630,8 +646,8 @@ void release_context(des_ctx *c)
         cudaStreamSynchronize(c->ystream);
         cudaStreamDestroy(c->ystream);
         for (cudaEvent_t e : c->pipe_ev) cudaEventDestroy(e);
-        cudaFree(c->d_pipe_sink);
     }
+    cudaFree(c->d_pipe_sink);
     if (c->xstream) {
         cudaStreamSynchronize(c->xstream);
         cudaStreamDestroy(c->xstream);
@@ -1480,7 +1496,13 @@ int capture_pipelined(des_ctx *c, const std::vector<SlabField> &F, cudaGraphExec
 {
     const int B = c->nslab, NF = c->nfine;
     const bool mixed = use_mixed(c);
-    const KP p0 = step_kp(c);
+    KP p0 = step_kp(c);
+    if (c->d_pipe_terms) {
+        p0.hc64 = c->d_pipe_terms;
+        p0.qv = p0.hc64 + (size_t)c->npe * c->ne;
+        p0.me = p0.qv + c->ne;
+        p0.tme = p0.me + c->ne;
+    }
     const bool thermal = p0.prm.has_thermal_diffusion != 0;
     cudaStream_t cs = c->stream, xs = c->xstream, ys = c->ystream;
     std::vector<cudaEvent_t> &ev = c->pipe_ev;   // [0,B) uploaded, [B,2B) slab done, 2B fork, 2B+1/2 joins
@@ -1613,12 +1635,22 @@ end:
     return DES_OK;
 }
 
+// The slabs are in different stages of the step at a time, so that an FP64
+// context's element terms cannot share the force terms' memory: they get 8
+// (npe + 3) bytes per element of their own.  A mesh that leaves no room for
+// them takes the general path.
 int ensure_pipe(des_ctx *c)
 {
     if (c->ystream) return DES_OK;
+    const size_t sink = 2 * (size_t)c->nn, terms = use_mixed(c) ? 0 : (size_t)(c->npe + 3) * c->ne;
+    if (!c->d_pipe_sink && cudaMalloc((void **)&c->d_pipe_sink, (sink + terms) * sizeof(double)) != cudaSuccess) {
+        (void)cudaGetLastError();   // not a failure of the call
+        c->nslab = 1;
+        return DES_OK;
+    }
+    c->d_pipe_terms = terms ? c->d_pipe_sink + sink : nullptr;
     c->pipe_ev.assign(2 * c->nslab + 3, nullptr);
     for (cudaEvent_t &e : c->pipe_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    CK(cudaMalloc((void **)&c->d_pipe_sink, 2 * (size_t)c->nn * sizeof(double)));
     CK(cudaStreamCreateWithFlags(&c->ystream, cudaStreamNonBlocking));
     return DES_OK;
 }
@@ -1629,9 +1661,11 @@ int step_host_pipelined(des_ctx *c, des_host_state *st, bool *done)
     *done = false;
     if (c->nslab < 2) return DES_OK;
     int rc;
-    if ((rc = ensure_xfer(c)) || (rc = ensure_pipe(c))) return rc;
+    if ((rc = ensure_xfer(c))) return rc;
     std::vector<SlabField> F;
     if (!slab_fields(c, st, F)) return DES_OK;
+    if ((rc = ensure_pipe(c))) return rc;
+    if (c->nslab < 2) return DES_OK;
     std::vector<const void *> key;
     for (const SlabField &f : F) key.push_back(f.host);
     if (!c->pipe_exec || key != c->pipe_key) {

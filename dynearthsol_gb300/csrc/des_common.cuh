@@ -131,9 +131,12 @@ struct KP {
     // of (element e, slot i): q = sup_pos[i ne + e], the inverse of sup_ent
     float4 *ft;
     const int *sup_pos;
-    // the FP64 step's: -(sigma . dN_i/dx + buoyancy z) vol, one (2D) or two
-    // (3D, the last value unused) double2 per support-list entry
+    // the FP64 step's: -(sigma . dN_i/dx + buoyancy z) vol per support-list
+    // entry, the first two components and (3D) the third.  An FP64 context's
+    // ndpk, qv, me, tme and hc64 lie in the same memory (create_context): none
+    // of them is held from the stress correction to the force.
     double2 *ft64;
+    double *ft64z;
     // where the FP64 stress pass writes what it forms from srate, stress and
     // pls: the corrected strain rate, the stress before the NMD correction and
     // the plastic strain.  The same arrays, but for the reverse mode's taped

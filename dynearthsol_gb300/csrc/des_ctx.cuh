@@ -27,7 +27,7 @@ struct des_ctx {
     size_t pool_bytes = 0;
     double *d_tdot = nullptr;     // node scratch of the fused step
     double *d_rho = nullptr;      // element scratch of the fused step
-    double *d_stage = nullptr;    // AoS staging buffer
+    double *d_stage = nullptr;    // AoS staging buffer (FP64 contexts: within the step scratch)
     size_t stage_doubles = 0;
     unsigned long long *d_red = nullptr;
     double *d_ef[DES_EF_COUNT] = {};
@@ -56,6 +56,7 @@ struct des_ctx {
     std::vector<const void *> pipe_key;
     std::vector<cudaEvent_t> pipe_ev;
     double *d_pipe_sink = nullptr;         // [2][nn]: node sums the pipelined step forms but keeps uploaded
+    double *d_pipe_terms = nullptr;        // FP64: the pipelined step's hc64, qv, me and tme (behind the sink)
     int pipe_kernels = 0;
     int step_kernels = 0;
     long long launches = 0;

@@ -506,9 +506,9 @@ __device__ __forceinline__ void force_term(const KP &p, int e, int i, const doub
     const double sx = shp_at(p, 0, i, e), sz = shp_at(p, ND - 1, i, e);
     if (ND == 3) {
         const double sy = shp_at(p, 1, i, e);
-        p.ft64[2 * q] = make_double2(-(s[0] * sx + s[3] * sy + s[4] * sz) * vol,
-                                     -(s[3] * sx + s[1] * sy + s[5] * sz) * vol);
-        p.ft64[2 * q + 1] = make_double2(-(s[4] * sx + s[5] * sy + s[2] * sz + buoy) * vol, 0.0);
+        p.ft64[q] = make_double2(-(s[0] * sx + s[3] * sy + s[4] * sz) * vol,
+                                 -(s[3] * sx + s[1] * sy + s[5] * sz) * vol);
+        p.ft64z[q] = -(s[4] * sx + s[5] * sy + s[2] * sz + buoy) * vol;
     } else {
         p.ft64[q] = make_double2(-(s[0] * sx + s[2] * sz) * vol, -(s[2] * sx + s[1] * sz + buoy) * vol);
     }
@@ -687,12 +687,13 @@ struct ForceTerms {   // the three components' terms of a support entry
 template <int ND>
 struct ForceTerms64 {
     const double2 *ft;
+    const double *z;
     __device__ __forceinline__ void operator()(int q, double *t) const
     {
-        const double2 a = __ldg(ft + (ND - 1) * (size_t)q);
+        const double2 a = __ldg(ft + q);
         t[0] = a.x;
         t[1] = a.y;
-        if (ND == 3) t[ND - 1] = __ldg((const double *)(ft + 2 * (size_t)q + 1));
+        if (ND == 3) t[ND - 1] = __ldg(z + q);
     }
 };
 
@@ -700,7 +701,7 @@ template <int ND, bool STAGED>
 __global__ void __launch_bounds__(192) k_force(KP p, int fused_motion)
 {
     double f[ND];
-    const int n = node_sums<SumF64, ND, ND, STAGED>(p.sup_off, p.n_lo, p.n_hi, ND, ForceTerms64<ND>{p.ft64},
+    const int n = node_sums<SumF64, ND, ND, STAGED>(p.sup_off, p.n_lo, p.n_hi, ND, ForceTerms64<ND>{p.ft64, p.ft64z},
                                                     FromZero<SumF64>(), f);
     if (n >= 0) force_tail<ND, false>(p, n, f, fused_motion);
 }
