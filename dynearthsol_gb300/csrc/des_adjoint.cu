@@ -321,7 +321,7 @@ int launch_adj_motion(const KP &p, const AdjBufs &a, const TapeStep &t, const Ta
 
 int adj_vbc_parts(const KP &p)
 {
-    const int nodes = node_staged(p.nn) ? NPB : 32;   // a block's, or a warp's
+    const int nodes = node_staged(p, p.nn) ? NPB : 32;   // a block's, or a warp's
     return (p.nn + nodes - 1) / nodes;
 }
 

@@ -24,14 +24,23 @@ namespace des {
 
 constexpr int NPB = 8, STAGED_THREADS = 192;
 
-// n: nodes of the launch.  Measured (walk / staged): on 177,147 nodes the
-// node pass takes 46 / 74 us, the force 55 / 64 us and the reverse node pass
-// 108 / 225 us; on 22,344 nodes a pass through the per-function entry points
-// takes 4.51 / 4.18 ms.  The line lies between, where a walk would put eight
-// warps on each SM, too few to hide its chain of loads.  192 threads take
-// the entries of 8 nodes (~24 each) in one chunk: 100 steps of a 648-tet mesh,
-// with the state's copies, 5.83 ms, 5.98 ms with 96 threads.
-inline bool node_staged(long long n) { return n <= 152LL * 256; }
+// p: the launch's context, n: its nodes.  Staging pays while the walk would
+// put too few warps on each SM to hide its chain of loads; beyond about a wave
+// of blocks it only adds the trip through shared memory.  The lines lie where
+// the two take the same time, at 56 nodes per SM with FP64 sums and at 160 with
+// the double-word sums of a mixed context, whose additions cost the few adding
+// threads less.  Measured, staged / walk:
+// * FP64, 200 steps in 2D: 12,000 triangles (6,191 nodes) 7.7 / 8.1 ms, 16,000
+//   (8,241) 8.1 / 8.1, 24,000 (12,291) 10.5 / 8.9, 36,000 (18,361) 12.1 / 9.8;
+//   100 steps in 3D: 14,400 tets (3,087 nodes) 6.2 / 7.3, 42,336 (8,410) 11.0 /
+//   11.6, 56,448 (10,933) 13.1 / 13.1, 73,728 (14,157) 16.7 / 15.9; windows of
+//   20 steps and their reverse: 14,400 tets 3.95 / 4.55, 42,336 6.14 / 6.16,
+//   73,728 8.47 / 8.01.
+// * mixed, 100 steps: 73,728 tets 6.90 / 7.74 ms, 121,296 (22,815 nodes) 10.03 /
+//   10.14, 134,400 (25,215) 10.78 / 10.57, 162,624 (30,375) 13.36 / 12.64.
+// 192 threads take the entries of 8 nodes (~24 each) in one chunk: 100 steps of
+// a 648-tet mesh, with the state's copies, 5.83 ms, 5.98 ms with 96 threads.
+inline bool node_staged(const KP &p, long long n) { return n <= 152LL * (p.shpdw ? 160 : 56); }
 
 // The sums' arithmetic: a quantity's term, state, addition and value.
 struct SumF64 {   // FP64 additions
@@ -134,18 +143,19 @@ struct FromZero {
     __device__ __forceinline__ typename P::State operator()(int, int) const { return typename P::State{}; }
 };
 
-// KERNEL<..., STAGED> over n nodes on stream s; KERNEL names the template
-// argument STAGED where it takes the shape
-#define DES_NODES(KERNEL, n, s, ...)                                                                              \
-    do {                                                                                                          \
-        const long long n_ = (n);                                                                                 \
-        if (des::node_staged(n_)) {                                                                               \
-            constexpr bool STAGED = true;                                                                         \
+// KERNEL<..., STAGED> over n nodes of the context p on stream s; KERNEL names
+// the template argument STAGED where it takes the shape
+#define DES_NODES(KERNEL, n, s, ...) DES_NODES_IF(des::node_staged(p, (n)), KERNEL, n, s, __VA_ARGS__)
+#define DES_NODES_IF(IN_BLOCKS, KERNEL, n, s, ...)                                                                    \
+    do {                                                                                                              \
+        const long long n_ = (n);                                                                                     \
+        if (IN_BLOCKS) {                                                                                              \
+            constexpr bool STAGED = true;                                                                             \
             KERNEL<<<(int)std::max(1LL, (n_ + des::NPB - 1) / des::NPB), des::STAGED_THREADS, 0, (s)>>>(__VA_ARGS__); \
-        } else {                                                                                                  \
-            constexpr bool STAGED = false;                                                                        \
-            DES_LAUNCH(KERNEL, n_, (s), __VA_ARGS__);                                                             \
-        }                                                                                                         \
+        } else {                                                                                                      \
+            constexpr bool STAGED = false;                                                                            \
+            DES_LAUNCH(KERNEL, n_, (s), __VA_ARGS__);                                                                 \
+        }                                                                                                             \
     } while (0)
 
 }  // namespace des

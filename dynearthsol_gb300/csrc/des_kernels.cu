@@ -1552,17 +1552,18 @@ int launch_nmd_gather(const KP &p, cudaStream_t s, bool stored)
 }
 
 // The force terms of [e_lo, e_hi) and the facets' forces, with or without
-// the correction first.  Up to a wave of slots the element's four slots go
-// side by side, where a thread's chain of 76 FP64 operations is what a launch
-// takes: a pass of 100 steps of 648 tets 5.79 ms, a thread per element 6.03
-// ms; beyond, four threads repeat the element's loads and correction for
-// nothing: 20 steps of 998,400 tets 36.0 ms split, 34.7 ms not, 118,326 tets
-// 4.10 and 4.05 ms.
+// the correction first.  Up to 96 elements per SM the element's four slots go
+// side by side: a thread's chain of 76 FP64 operations is then what a launch
+// takes.  Beyond, four threads repeat the element's loads and correction for
+// nothing.  Measured, split / not: 100 steps of 648 tets 5.79 / 6.03 ms, 12,288
+// 6.04 / 6.21, 14,400 6.23 / 6.22, 42,336 11.04 / 10.85, 116,640 25.8 / 25.1;
+// 200 steps of 4,000 triangles 6.87 / 7.23, 12,000 7.67 / 7.69, 16,000 8.11 /
+// 8.07, 36,000 (walked) 11.0 / 9.8.
 template <int ND, bool CORRECT>
 void launch_elem_force(const KP &p, cudaStream_t s)
 {
     const long long nel = p.e_hi - p.e_lo, nf = p.f_hi - p.f_lo;
-    if (4 * nel <= 152 * 2048) DES_LAUNCH((k_elem_force<ND, CORRECT, true, false, true>), 4 * nel + nf, s, p);
+    if (nel <= 152 * 96) DES_LAUNCH((k_elem_force<ND, CORRECT, true, false, true>), 4 * nel + nf, s, p);
     else DES_LAUNCH((k_elem_force<ND, CORRECT, true, false, false>), nel + nf, s, p);
 }
 

@@ -21,6 +21,7 @@ def load(directory):
     lib = capi.load_library(path)
     lib.fake_first_violation.restype = C.c_char_p
     lib.fake_allocated.restype = C.c_size_t
+    lib.fake_block_of.argtypes = [C.c_char_p]
     lib.fake_malloc_limit.argtypes = [C.c_size_t]
     return lib
 
