@@ -1159,7 +1159,7 @@ int des_set_clock(des_ctx *c, double time, double dt, int steps)
     }
 
 PERFN(des_update_temperature,
-      n += (p.shpdw ? launch_heat_and_dvoldt_mixed(p, s, true, false) + launch_temperature_update(p, s)
+      n += (p.shpdw ? launch_heat_gather_mixed(p, s) + launch_temperature_update(p, s)
                     : launch_update_temperature(p, s)))
 PERFN(des_update_strain_rate,
       n += (p.shpdw ? launch_strain_rate_mixed(p, s, false) : launch_strain_rate(p, s, false)))
@@ -1175,7 +1175,7 @@ PERFN(des_update_force,
 PERFN(des_update_velocity, n += launch_velocity(p, s, p.shpdw != nullptr))
 PERFN(des_apply_vbcs, n += launch_vbcs(p, s))
 PERFN(des_update_coordinate, n += launch_coordinate(p, s, p.shpdw != nullptr))
-PERFN(des_swap_volume, n += launch_geometry(p, s, GEO_COPY_OLD))
+PERFN(des_swap_volume, n += launch_swap_volume(p, s))
 PERFN(des_compute_volume, n += launch_geometry(p, s, GEO_VOLUME))
 PERFN(des_compute_mass, n += launch_geometry(p, s, GEO_MASS_TERMS); n += launch_mass_sum(p, s))
 PERFN(des_compute_shape_fn, n += launch_geometry(p, s, GEO_SHAPE))
@@ -1187,7 +1187,7 @@ PERFN(des_update_mesh, n += launch_coordinate(p, s, p.shpdw != nullptr);
 int des_compute_dt(des_ctx *c, double *dt_out)
 {
     if (!c) return DES_EINPUT;
-    int rc = check_launch(c, launch_geometry(c->kp, c->stream, GEO_DT) + launch_dt_finalize(c->kp, c->stream, false));
+    int rc = check_launch(c, launch_dt_terms(c->kp, c->stream) + launch_dt_finalize(c->kp, c->stream, false));
     if (rc) return rc;
     double dt;
     rc = des_get_clock(c, nullptr, &dt, nullptr);

@@ -15,6 +15,8 @@
 //   degree (and any mix of degrees) is summed.
 // node_staged() draws the line.
 #pragma once
+#include <type_traits>
+
 #include <cuda_runtime.h>
 
 #include "des_common.cuh"
@@ -40,7 +42,8 @@ constexpr int NPB = 8, STAGED_THREADS = 192;
 //   10.14, 134,400 (25,215) 10.78 / 10.57, 162,624 (30,375) 13.36 / 12.64.
 // 192 threads take the entries of 8 nodes (~24 each) in one chunk: 100 steps of
 // a 648-tet mesh, with the state's copies, 5.83 ms, 5.98 ms with 96 threads.
-inline bool node_staged(const KP &p, long long n) { return n <= 152LL * (p.shpdw ? 160 : 56); }
+inline bool node_staged_fp64(long long n) { return n <= 152LL * 56; }
+inline bool node_staged(const KP &p, long long n) { return p.shpdw ? n <= 152LL * 160 : node_staged_fp64(n); }
 
 // The sums' arithmetic: a quantity's term, state, addition and value.
 struct SumF64 {   // FP64 additions
@@ -73,12 +76,20 @@ struct Staged {
     __device__ __forceinline__ T &operator[](int r) { return v[r + r / ROW]; }
 };
 
+template <class P, class Term>
+__device__ __forceinline__ void entry_terms(Term &term, int q, typename P::Term *t, int n)
+{
+    if constexpr (std::is_invocable_v<Term, int, typename P::Term *, int>) term(q, t, n);
+    else term(q, t);
+}
+
 // The sums of NQ quantities over the support of the nodes [lo, hi) of a
-// launch, by the calling kernel's whole grid: term(q, t) forms the NQ terms
-// of support entry q; first(c, n) is the value that quantity c of node n
+// launch, by the calling kernel's whole grid: term(q, t) or term(q, t, n) forms
+// the NQ terms of support entry q (n: its node in a walk; entries staged side by
+// side are not told); first(c, n) is the value that quantity c of node n
 // starts from.  Returns the node whose NQ sums the thread holds in out, or -1
-// when it holds none.  Every thread of the block calls it, and nq <= NQ
-// quantities are summed (the others are left as they are).
+// when it holds none.  Every thread of the block calls it; of the NQ sums, the
+// first nq are formed and the others hold nothing.
 template <class P, int NQ, int ND, bool STAGED, class Term, class First>
 __device__ __forceinline__ int node_sums(const int *__restrict__ off, int lo, int hi, int nq, Term term, First first,
                                          double *out)
@@ -91,7 +102,7 @@ __device__ __forceinline__ int node_sums(const int *__restrict__ off, int lo, in
         for (int c = 0; c < NQ; ++c) s[c] = first(c, n);
         for (int q = off[n]; q < off[n + 1]; ++q) {
             typename P::Term t[NQ];
-            term(q, t);
+            entry_terms<P>(term, q, t, n);
 #pragma unroll
             for (int c = 0; c < NQ; ++c)
                 if (c < nq) P::add(c, s[c], t[c]);
@@ -118,7 +129,7 @@ __device__ __forceinline__ int node_sums(const int *__restrict__ off, int lo, in
             const int end = min(base + CAP, q1);
             for (int q = base + (int)threadIdx.x; q < end; q += STAGED_THREADS) {
                 typename P::Term t[NQ];
-                term(q, t);
+                entry_terms<P>(term, q, t, -1);
 #pragma unroll
                 for (int k = 0; k < NQ; ++k)
                     if (k < nq) slot[k][q - base] = t[k];

@@ -923,6 +923,55 @@ __device__ __forceinline__ void dt_finalize(const KP &p)
     ck->red_minh = ck->red_maxwell = ck->red_diffusion = ~0ull;
 }
 
+// compute_dt element terms (geometry.cxx:254-292): the smallest height of the
+// element and its Maxwell time.  The diffusion time 0.5 minh^2 / kappa is
+// non-decreasing in minh, so its minimum over the elements is dt_finalize's
+// 0.5 min(minh)^2 / kappa.
+template <int ND>
+__device__ __forceinline__ double min_height(const double (*c)[ND], double vol)
+{
+    if (ND == 3) {
+        // the largest face area: sqrt is correctly rounded and
+        // monotonic and /2 exact, so max_i sqrt(s_i) / 2 equals
+        // sqrt(max_i s_i) / 2 -- one square root instead of four
+        const double s2 = dmax_(dmax_(tri_area2_3d(c[0], c[1], c[2]), tri_area2_3d(c[0], c[1], c[ND])),
+                                dmax_(tri_area2_3d(c[2], c[ND], c[0]), tri_area2_3d(c[2], c[ND], c[1])));
+        return 3 * vol / (sqrt(s2) / 2);
+    }
+    double d01 = 0, d12 = 0, d02 = 0;
+#pragma unroll
+    for (int k = 0; k < ND; ++k) {
+        double a = c[1][k] - c[0][k], b = c[2][k] - c[1][k], cc = c[2][k] - c[0][k];
+        d01 += a * a;
+        d12 += b * b;
+        d02 += cc * cc;
+    }
+    return 2 * vol / sqrt(dmax_(dmax_(d01, d12), d02));
+}
+
+__device__ __forceinline__ double maxwell_time(const KP &p, int e)
+{
+    return 0.5 * p.mat.visc_min / (1e-40 + m_shearm(p, e));
+}
+
+// des_compute_dt's element pass; the step's geometry pass forms the same terms
+// with the coordinates at hand.  Bound by the FP64 pipe.
+template <int ND>
+__global__ void __launch_bounds__(128) k_dt_terms(KP p)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long b_minh = ~0ull, b_maxwell = ~0ull;
+    if (e < p.ne) {
+        double c[ND + 1][ND];
+#pragma unroll
+        for (int i = 0; i < ND + 1; ++i) load_node_x<ND>(p, conn_at(p, i, e), c[i]);
+        b_minh = dbits(min_height<ND>(c, p.vol[e]));
+        if (!uniform_maxwell_time(p)) b_maxwell = dbits(maxwell_time(p, e));
+    }
+    warp_block_min<ND>(b_minh, &p.clk->red_minh);
+    if (!uniform_maxwell_time(p)) warp_block_min<ND>(b_maxwell, &p.clk->red_maxwell);
+}
+
 // The element geometry pass.  MIXED: a 3D mixed context's form (FP64 volume,
 // double-word shape functions, FP32 rotation increments).  AHEAD (the chained
 // step's look-ahead): with the shape functions and velocities still in
@@ -976,34 +1025,10 @@ __device__ __forceinline__ void geometry_body(const KP &p, int flags)
             vol = p.vol[e];
         }
         if (do_dt) {
-            // compute_dt element terms (geometry.cxx:254-292), while the coordinates are at hand
-            double minh;
-            if (ND == 3) {
-                // the largest face area: sqrt is correctly rounded and
-                // monotonic and /2 exact, so max_i sqrt(s_i) / 2 equals
-                // sqrt(max_i s_i) / 2 -- one square root instead of four
-                const double s2 = dmax_(dmax_(tri_area2_3d(c[0], c[1], c[2]), tri_area2_3d(c[0], c[1], c[NPE - 1])),
-                                        dmax_(tri_area2_3d(c[2], c[NPE - 1], c[0]),
-                                              tri_area2_3d(c[2], c[NPE - 1], c[1])));
-                double maxa = sqrt(s2) / 2;
-                minh = 3 * vol / maxa;
-            } else {
-                double d01 = 0, d12 = 0, d02 = 0;
-#pragma unroll
-                for (int k = 0; k < ND; ++k) {
-                    double a = c[1][k] - c[0][k], b = c[2][k] - c[1][k], cc = c[2][k] - c[0][k];
-                    d01 += a * a;
-                    d12 += b * b;
-                    d02 += cc * cc;
-                }
-                double maxl = sqrt(dmax_(dmax_(d01, d12), d02));
-                minh = 2 * vol / maxl;
-            }
-            b_minh = dbits(minh);
+            // while the coordinates are at hand
+            b_minh = dbits(min_height<ND>(c, vol));
             // uniform, the Maxwell time is formed once by dt_finalize
-            if (!uniform_maxwell_time(p)) b_maxwell = dbits(0.5 * p.mat.visc_min / (1e-40 + m_shearm(p, e)));
-            // the diffusion time 0.5 minh^2 / kappa is non-decreasing in minh,
-            // so its minimum over the elements is dt_finalize's 0.5 min(minh)^2 / kappa
+            if (!uniform_maxwell_time(p)) b_maxwell = dbits(maxwell_time(p, e));
         }
         double shp[ND][NPE];
         float s32[ND][NPE];   // a mixed context's FP32 shape functions (its rotation's)
@@ -1503,8 +1528,10 @@ int launch_update_temperature(const KP &p, cudaStream_t s)
 
 int launch_dvoldt(const KP &p, cudaStream_t s)
 {
-    if (p.nd == 3) DES_NODES((k_dvoldt<3, STAGED>), p.nn, s, p);
-    else DES_NODES((k_dvoldt<2, STAGED>), p.nn, s, p);
+    // an FP64 sum in mixed contexts too
+    const bool blocks = node_staged_fp64(p.nn);
+    if (p.nd == 3) DES_NODES_IF(blocks, (k_dvoldt<3, STAGED>), p.nn, s, p);
+    else DES_NODES_IF(blocks, (k_dvoldt<2, STAGED>), p.nn, s, p);
     return 1;
 }
 
@@ -1526,7 +1553,7 @@ int launch_node_pass(const KP &p, cudaStream_t s, bool heat, bool mass_sums)
 
 int launch_temperature_update(const KP &p, cudaStream_t s)
 {
-    DES_LAUNCH(k_temperature_update, p.nn, s, p);
+    DES_LAUNCH_LIGHT(k_temperature_update, p.nn, s, p);
     return 1;
 }
 
@@ -1606,17 +1633,18 @@ int launch_velocity(const KP &p, cudaStream_t s, bool contract)
 {
     const long long g = (long long)p.nn * p.nd;
     if (contract) {
-        if (p.nd == 3) DES_LAUNCH((k_velocity<3, true>), g, s, p);
-        else DES_LAUNCH((k_velocity<2, true>), g, s, p);
+        DES_LAUNCH_LIGHT((k_velocity<3, true>), g, s, p);
         return 1;
     }
-    DISPATCH(k_velocity, g, p);
+    if (p.nd == 3) DES_LAUNCH_LIGHT(k_velocity<3>, g, s, p);
+    else DES_LAUNCH_LIGHT(k_velocity<2>, g, s, p);
     return 1;
 }
 
 int launch_vbcs(const KP &p, cudaStream_t s)
 {
-    DISPATCH(k_vbcs, p.nn, p);
+    if (p.nd == 3) DES_LAUNCH_LIGHT(k_vbcs<3>, p.nn, s, p);
+    else DES_LAUNCH_LIGHT(k_vbcs<2>, p.nn, s, p);
     return 1;
 }
 
@@ -1624,11 +1652,11 @@ int launch_coordinate(const KP &p, cudaStream_t s, bool contract)
 {
     const long long g = (long long)p.nn * p.nd;
     if (contract) {
-        if (p.nd == 3) DES_LAUNCH((k_coordinate<3, true>), g, s, p);
-        else DES_LAUNCH((k_coordinate<2, true>), g, s, p);
+        DES_LAUNCH_LIGHT((k_coordinate<3, true>), g, s, p);
         return 1;
     }
-    DISPATCH(k_coordinate, g, p);
+    if (p.nd == 3) DES_LAUNCH_LIGHT(k_coordinate<3>, g, s, p);
+    else DES_LAUNCH_LIGHT(k_coordinate<2>, g, s, p);
     return 1;
 }
 
@@ -1656,6 +1684,25 @@ int launch_mass_sum(const KP &p, cudaStream_t s)
     if (p.nd == 3 && p.shpdw) DES_NODES((k_mass_sum<3, true, STAGED>), n, s, p);
     else if (p.nd == 3) DES_NODES((k_mass_sum<3, false, STAGED>), n, s, p);
     else DES_NODES((k_mass_sum<2, false, STAGED>), n, s, p);
+    return 1;
+}
+
+int launch_dt_terms(const KP &p, cudaStream_t s)
+{
+    if (p.prm.fixed_dt != 0) return 0;
+    DISPATCH(k_dt_terms, p.ne, p);
+    return 1;
+}
+
+__global__ void __launch_bounds__(256) k_swap_volume(const double *__restrict__ vol, double *__restrict__ vol_old, int n)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < n) vol_old[e] = vol[e];
+}
+
+int launch_swap_volume(const KP &p, cudaStream_t s)
+{
+    DES_LAUNCH_LIGHT(k_swap_volume, p.ne, s, p.vol, p.vol_old, p.ne);
     return 1;
 }
 

@@ -1,6 +1,8 @@
 // des_kernels.cuh -- host-side launchers of the explicit-step kernels.
 #pragma once
 
+#include <algorithm>
+
 #include <cuda_runtime.h>
 
 #include "des_common.cuh"
@@ -51,6 +53,14 @@ inline int grid_blocks(long long n, int most = 256)
             DES_LAUNCH(KERNEL, nw_, s, __VA_ARGS__);                                     \
     } while (0)
 
+// DES_LAUNCH for kernels of a few instructions a value (the per-function motion,
+// boundary condition and temperature updates): starting a block costs them as
+// much as its work.  Blocks of 64 or 128 / 256, us a call: coordinates of
+// 998,400 tets 6.3 / 4.3 in a mixed context, velocity BCs 5.8 / 4.3; below
+// 100,000 tets no difference.
+#define DES_LAUNCH_LIGHT(KERNEL, n, s, ...) \
+    KERNEL<<<(unsigned)std::max(1LL, ((long long)(n) + 255) / 256), 256, 0, (s)>>>(__VA_ARGS__)
+
 // flags of the element geometry pass
 enum GeoFlags : int {
     GEO_COPY_OLD = 1,    // volume_old <- volume        (dynearthsol.cxx:226)
@@ -88,12 +98,15 @@ int launch_force(const KP &p, cudaStream_t s, bool fused_motion);
 int launch_velocity(const KP &p, cudaStream_t s, bool contract = false);
 int launch_vbcs(const KP &p, cudaStream_t s);
 int launch_coordinate(const KP &p, cudaStream_t s, bool contract = false);
+int launch_swap_volume(const KP &p, cudaStream_t s);   // volume_old <- volume
 int launch_geometry(const KP &p, cudaStream_t s, int flags);
 // the chained step's geometry pass, which also does the next step's element
 // pass (k_elem_pass's or k_elem_pass_mixed3's work)
 int launch_geometry_ahead(const KP &p, cudaStream_t s, int flags);
 // compute_mass from the element terms of a GEO_MASS_TERMS geometry pass (same sums, same order)
 int launch_mass_sum(const KP &p, cudaStream_t s);
+// compute_dt's element terms alone (for launch_dt_finalize)
+int launch_dt_terms(const KP &p, cudaStream_t s);
 int launch_dt_finalize(const KP &p, cudaStream_t s, bool only_on_step);
 int launch_quality(const KP &p, cudaStream_t s, unsigned long long *red);
 // red[2], red[3]: bad_mesh_quality's first tiny element and first drifted bottom node

@@ -686,9 +686,6 @@ __global__ void __launch_bounds__(TPB_M) k_strain_rate_mixed3(KP p, int begin_st
     strain_rate_mixed_elem(p, e, sr);
 }
 
-// heat stencil on FP64 temperature differences (sum_j D_ij = 0), FP32
-// products, a compensated FP32 nodal sum of the heat terms; dvoldt in FP64
-// (fields.cxx:99-146, geometry.cxx:111-155)
 // dvoldt (quantity 0) in FP64, the others in compensated FP32 sums
 struct SumNode {
     using Term = double;   // the pairs travel as the FP64 value's two words
@@ -708,56 +705,56 @@ struct SumNode {
     static __device__ __forceinline__ double value(int c, const State &s) { return c == 0 ? s.d : s.w.value(); }
 };
 
+// des_update_temperature's heat sums (fields.cxx:99-146): the stencil on FP64
+// temperature differences (sum_j D_ij = 0), FP32 products, a compensated FP32
+// sum of the terms.  A walk reads its node's temperature once, a staged entry
+// for itself.
+struct SumF32 {
+    using Term = float;
+    using State = dw_sum;
+    static __device__ __forceinline__ void add(int, State &s, Term t) { s.add(t); }
+    static __device__ __forceinline__ double value(int, const State &s) { return s.value(); }
+};
+
 template <bool STAGED>
-__global__ void __launch_bounds__(192) k_heat_dvoldt_mixed3(KP p, int heat, int do_dvoldt)
+__global__ void __launch_bounds__(256) k_heat_gather_mixed3(KP p)
 {
     const bool k_const = (p.mat.nmat == 1) && !p.ef[DES_EF_THERM_COND];
-    double sum[2] = {0, 0};   // dvoldt, tdot
-    const int n = node_sums<SumNode, 2, 3, STAGED>(
-        p.sup_off, 0, p.nn, heat ? 2 : 1,
-        [&](int q, double *t) {
+    double tdot;
+    const int n = node_sums<SumF32, 1, 3, STAGED>(
+        p.sup_off, 0, p.nn, 1,
+        [&](int q, float *t, int node) {
             const int ent = p.sup_ent[q];
             const int e = ent >> 2, i = ent & 3;
-            const double vol = p.vol[e];
-            if (heat) {
-                const double Tn = p.T[conn_at(p, i, e)];
-                const float sxi = shp32_at(p, 0, i, e), syi = shp32_at(p, 1, i, e), szi = shp32_at(p, 2, i, e);
-                float diffusion = 0.0f;
+            const double Tn = p.T[STAGED ? conn_at(p, i, e) : node];
+            const float sxi = shp32_at(p, 0, i, e), syi = shp32_at(p, 1, i, e), szi = shp32_at(p, 2, i, e);
+            float diffusion = 0.0f;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (j == i) continue;
-                    const float D = sxi * shp32_at(p, 0, j, e) + syi * shp32_at(p, 1, j, e)
-                        + szi * shp32_at(p, 2, j, e);
-                    diffusion += D * f32_of(p.T[conn_at(p, j, e)] - Tn);
-                }
-                const float volf = f32_of(vol);
-                const float kv = f32_of(k_const ? p.mat.therm_cond[0] : m_k(p, e)) * volf;
-                const float rh = f32_of(m_hr_over_cp(p, e)) * volf;
-                t[1] = SumNode::pack(dw{kv * diffusion - rh, 0.0f});
+            for (int j = 0; j < 4; ++j) {
+                if (j == i) continue;
+                const float D = sxi * shp32_at(p, 0, j, e) + syi * shp32_at(p, 1, j, e) + szi * shp32_at(p, 2, j, e);
+                diffusion += D * f32_of(p.T[conn_at(p, j, e)] - Tn);
             }
-            t[0] = 0;
-            if (do_dvoldt) {
-                const double dj = p.srate[e] + p.srate[(size_t)p.ne + e] + p.srate[2 * (size_t)p.ne + e];
-                t[0] = dj * vol;
-            }
+            const float volf = f32_of(p.vol[e]);
+            const float kv = f32_of(k_const ? p.mat.therm_cond[0] : m_k(p, e)) * volf;
+            const float rh = f32_of(m_hr_over_cp(p, e)) * volf;
+            *t = kv * diffusion - rh;
         },
-        FromZero<SumNode>(), sum);
-    if (n < 0) return;
-    if (heat) p.tdot[n] = sum[1];
-    if (do_dvoldt) p.ntmp[n] = sum[0] / p.vol_n[n];
+        FromZero<SumF32>(), &tdot);
+    if (n >= 0) p.tdot[n] = tdot;
 }
 
 // ------------------------------------------------------------------
 // Fused step: strain rate, heat, dvoldt and the temperature update as one
 // element pass and one node pass.  The per-pair work of the node-centric
-// gather above (k_heat_dvoldt_mixed3: the stencil row of the node's slot,
+// gather above (k_heat_gather_mixed3: the stencil row of the node's slot,
 // four temperature differences and their FP32 conversions, which issue on
 // the FP64 pipe) is done once per element: the element pass stores the
 // four FP32 heat terms of the element and its dvoldt term, and the node
 // pass sums them over the support list in ascending element order.  Each
 // term is the very value the gather forms for that (node, element) pair,
 // and the sums run in the same order, so the result is bit-identical to
-// k_strain_rate_mixed3 + k_heat_dvoldt_mixed3 + k_temperature_update.
+// k_strain_rate_mixed3 + k_heat_gather_mixed3 + k_dvoldt + k_temperature_update.
 // ------------------------------------------------------------------
 __global__ void __launch_bounds__(TPB_M) k_elem_pass_mixed3(KP p, int heat)
 {
@@ -784,7 +781,7 @@ __global__ void __launch_bounds__(TPB_M) k_elem_pass_mixed3(KP p, int heat)
 // step's clock, which the look-ahead pass could not: the step's dt is final
 // only after k_dt_finalize.
 // The heat terms go into a compensated FP32 sum (des_dw.cuh), as
-// k_heat_dvoldt_mixed3 sums them; the dvoldt terms into an FP64 one: they
+// k_heat_gather_mixed3 sums them; the dvoldt terms into an FP64 one: they
 // cancel between a node's elements, and the 2^-47 of a double-word split of
 // each moved the volumetric rate enough to change the default damping's
 // copysign at some nodes within ten steps.
@@ -855,13 +852,16 @@ int launch_strain_rate_mixed(const KP &p, cudaStream_t s, bool begin_step)
     return 1;
 }
 
-int launch_heat_and_dvoldt_mixed(const KP &p, cudaStream_t s, bool heat, bool dvoldt)
+int launch_heat_gather_mixed(const KP &p, cudaStream_t s)
 {
     // a term here is an element's stencil row: a walk forms a node's 24 rows one
     // after the other, so that staging pays on larger meshes too.  20 loops of
     // the per-function entry points, staged / walk: 73,728 tets 3.38 / 3.87 ms,
-    // 162,624 (30,375 nodes) 4.82 / 5.18, 282,240 (51,984) 6.62 / 6.77
-    DES_NODES_IF(p.nn <= 152 * 256, k_heat_dvoldt_mixed3<STAGED>, p.nn, s, p, (int)heat, (int)dvoldt);
+    // 162,624 (30,375 nodes) 4.82 / 5.18, 282,240 (51,984) 6.62 / 6.77.  The
+    // walk's time is the L1 and L2 hits of its rows: a warp to a block 221 us a
+    // call at 998,400 tets, blocks of 64 248, 128 234, 192 229, 256 231.
+    if (p.nn <= 152 * 256) k_heat_gather_mixed3<true><<<(p.nn + NPB - 1) / NPB, STAGED_THREADS, 0, s>>>(p);
+    else k_heat_gather_mixed3<false><<<(p.nn + 31) / 32, 32, 0, s>>>(p);
     return 1;
 }
 

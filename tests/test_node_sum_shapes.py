@@ -41,5 +41,27 @@ def test_shape_by_size(lib, name, cells, prec, staged, split):
             assert (on > 0, off > 0) == (split, not split)
         if prec == "mixed":   # its heat terms are costlier: staged up to 38,912 nodes
             m.call("update_temperature")
-            assert lib.fake_block_of(b"k_heat_dvoldt_mixed3") == 192
+            assert lib.fake_block_of(b"k_heat_gather_mixed3") == 192
+        m.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_entry_points_launch_their_own_kernels(lib, prec):
+    """A copy and compute_dt's terms are not the geometry pass; the light updates have blocks of 256."""
+    from dynearthsol_gb300 import capi
+    from dynearthsol_gb300.config import initial_state, make_workload
+    from dynearthsol_gb300.solver import DeviceModel
+    wl = make_workload("c1_3d_evp", cells=(32, 32, 12))
+    with fake_runtime.installed(lib):
+        st, cp = initial_state(wl)
+        m = DeviceModel(wl, comp_pressure=cp, precision=capi.PREC_FP64 if prec == "fp64" else capi.PREC_MIXED)
+        m.upload(st, (0.0, 1.0, 0))
+        lib.fake_reset()
+        m.call("swap_volume")
+        m.call("compute_dt")
+        assert lib.fake_block_of(b"k_geometry") == 0
+        for name, kernel in (("update_velocity", b"k_velocity"), ("apply_vbcs", b"k_vbcs"),
+                             ("update_coordinate", b"k_coordinate")):
+            m.call(name)
+            assert lib.fake_block_of(kernel) == 256, kernel
         m.close()
