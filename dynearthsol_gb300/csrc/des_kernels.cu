@@ -1755,19 +1755,19 @@ int launch_shp_join(const KP &p, cudaStream_t s)
 {
     if (!p.shpdw) return 0;
     const long long n = (long long)p.ne * p.npe * p.nd;
-    DES_LAUNCH(k_shp_join, n, s, p.shpdw, p.shp, n);
+    DES_LAUNCH_LIGHT(k_shp_join, n, s, p.shpdw, p.shp, n);
     return 1;
 }
 
 int launch_aos_to_soa(const double *aos, double *soa, int n, int ncomp, cudaStream_t s)
 {
-    DES_LAUNCH(k_aos_to_soa, (long long)n * ncomp, s, aos, soa, n, ncomp);
+    DES_LAUNCH_LIGHT(k_aos_to_soa, (long long)n * ncomp, s, aos, soa, n, ncomp);
     return 1;
 }
 
 int launch_soa_to_aos(const double *soa, double *aos, int n, int ncomp, cudaStream_t s)
 {
-    DES_LAUNCH(k_soa_to_aos, (long long)n * ncomp, s, soa, aos, n, ncomp);
+    DES_LAUNCH_LIGHT(k_soa_to_aos, (long long)n * ncomp, s, soa, aos, n, ncomp);
     return 1;
 }
 

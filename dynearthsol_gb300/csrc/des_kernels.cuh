@@ -53,11 +53,11 @@ inline int grid_blocks(long long n, int most = 256)
             DES_LAUNCH(KERNEL, nw_, s, __VA_ARGS__);                                     \
     } while (0)
 
-// DES_LAUNCH for kernels of a few instructions a value (the per-function motion,
-// boundary condition and temperature updates): starting a block costs them as
-// much as its work.  Blocks of 64 or 128 / 256, us a call: coordinates of
-// 998,400 tets 6.3 / 4.3 in a mixed context, velocity BCs 5.8 / 4.3; below
-// 100,000 tets no difference.
+// DES_LAUNCH for kernels of a few instructions a value (copies, layout
+// conversions, the per-function motion, boundary condition and temperature
+// updates): starting a block costs them as much as its work.  Blocks of 64 or 128 / 256, us a call: coordinates of
+// 998,400 tets 6.3 / 4.3 in a mixed context, velocity BCs 5.8 / 4.3; an upload of
+// 1,200 triangles 152 / 139.
 #define DES_LAUNCH_LIGHT(KERNEL, n, s, ...) \
     KERNEL<<<(unsigned)std::max(1LL, ((long long)(n) + 255) / 256), 256, 0, (s)>>>(__VA_ARGS__)
 

@@ -65,3 +65,16 @@ def test_entry_points_launch_their_own_kernels(lib, prec):
             m.call(name)
             assert lib.fake_block_of(kernel) == 256, kernel
         m.close()
+
+
+def test_layout_conversions_have_blocks_of_256(lib):
+    from dynearthsol_gb300.config import initial_state, make_workload
+    from dynearthsol_gb300.solver import DeviceModel
+    wl = make_workload("c0_2d_ep", cells=(60, 10))
+    with fake_runtime.installed(lib):
+        st, cp = initial_state(wl)
+        m = DeviceModel(wl, comp_pressure=cp)
+        m.upload(st, (0.0, 1.0, 0))
+        m.download()
+        assert lib.fake_block_of(b"k_aos_to_soa") == lib.fake_block_of(b"k_soa_to_aos") == 256
+        m.close()
