@@ -22,11 +22,7 @@
 
 namespace des {
 
-constexpr int TPB_A = 128;
-
-// DES_LAUNCH for kernels of at most TPB_A threads a block
-#define DES_LAUNCH_A(KERNEL, n, s, ...) \
-    KERNEL<<<grid_blocks(n, TPB_A), block_threads(n, TPB_A), 0, (s)>>>(__VA_ARGS__)
+constexpr int TPB_A = BLOCK_MOST;   // the element and facet kernels' largest block
 
 __device__ __forceinline__ double tshp(const TapeStep &t, size_t ne, int k, int i, int e)
 {
@@ -506,7 +502,7 @@ int launch_adj_force(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStrea
 {
     int n = 0;
     if (p.nbf > 0) {
-        DES_LAUNCH_A(k_adj_facets, p.nbf, s, p, a, t);
+        DES_LAUNCH(k_adj_facets, p.nbf, s, p, a, t);
         ++n;
     }
     DES_LAUNCH_W(k_adj_force, p.ne, s, p, a, t);
@@ -1205,7 +1201,7 @@ int launch_adj_gather_vT(const KP &p, const AdjBufs &a, cudaStream_t s)
 
 int launch_adj_start_geometry(const KP &p, const AdjBufs &a, const TapeStep &t, cudaStream_t s)
 {
-    DES_LAUNCH_A(k_adj_start_geometry, p.ne, s, p, a, t);
+    DES_LAUNCH(k_adj_start_geometry, p.ne, s, p, a, t);
     return 1;
 }
 

@@ -1162,7 +1162,7 @@ PERFN(des_update_temperature,
       n += (p.shpdw ? launch_heat_gather_mixed(p, s) + launch_temperature_update(p, s)
                     : launch_update_temperature(p, s)))
 PERFN(des_update_strain_rate,
-      n += (p.shpdw ? launch_strain_rate_mixed(p, s, false) : launch_strain_rate(p, s, false)))
+      n += (p.shpdw ? launch_strain_rate_mixed(p, s) : launch_strain_rate(p, s)))
 PERFN(des_compute_dvoldt, n += launch_dvoldt(p, s))
 PERFN(des_compute_edvoldt, n += launch_edvoldt(p, s))
 PERFN(des_update_stress,
@@ -1308,7 +1308,7 @@ int enqueue_step_chain(des_ctx *c, int part)
     int n = 0;
     const bool thermal = p.prm.has_thermal_diffusion != 0, mixed = use_mixed(c);
     if (part == 0) n += mixed ? launch_elem_pass_mixed(p, s, thermal) : launch_elem_pass(p, s, thermal);
-    n += mixed ? launch_node_pass_mixed(p, s, thermal, part != 0, part != 0)
+    n += mixed ? launch_node_pass_mixed(p, s, thermal, part != 0)
                : launch_node_pass(p, s, thermal, part != 0);
     n += mixed ? launch_update_stress_mixed(p, s, true, part == 2, part != 0) : launch_update_stress(p, s, true);
     n += launch_nmd_gather(p, s, mixed);

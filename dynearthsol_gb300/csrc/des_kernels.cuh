@@ -19,19 +19,17 @@ namespace des {
 // steps 13.5 -> 9.9, 14,400 yielding tets x 100 mixed steps 12.3 -> 10.0,
 // 118,326 tets x 10 loops of the per-function entry points 5.24 -> 4.67,
 // 998,400 tets x 20 FP64 steps 39.5 -> 39.0 (128 and 64 alike), 998,400 tets
-// x 50 mixed steps 28.3 -> 27.6 (128); blocks of 32 are slower than 64 at
-// every size (launch and scheduling of blocks).
+// x 50 mixed steps 28.3 -> 27.6 (128).  Blocks of 32 for all of them are slower
+// than 64 at every size (launch and scheduling of blocks); for the few kernels
+// of DES_LAUNCH_W they are not.
 inline bool one_wave(long long n) { return n <= 152LL * 2048; }
 
-inline int block_threads(long long n, int most = 256)
-{
-    const int t = one_wave(n) ? 64 : 128;
-    return t < most ? t : most;
-}
+constexpr int BLOCK_MOST = 128;   // of DES_LAUNCH
+inline int block_threads(long long n) { return one_wave(n) ? 64 : BLOCK_MOST; }
 
-inline int grid_blocks(long long n, int most = 256)
+inline int grid_blocks(long long n)
 {
-    const long long t = block_threads(n, most), b = (n + t - 1) / t;
+    const long long t = block_threads(n), b = (n + t - 1) / t;
     return (int)(b < 1 ? 1 : b);
 }
 
@@ -42,8 +40,11 @@ inline int grid_blocks(long long n, int most = 256)
 // DES_LAUNCH for the 3D FP64 geometry and reverse element kernels, which a
 // small mesh's warps share an SM's FP64 pipe for: up to one wave a warp to a
 // block, so that no SM has more of them than it must.  Measured (blocks of 64
-// / 32 threads): a window of 50 steps of 14,400 tets and its reverse 12.36 /
-// 12.08 ms.  The other kernels, and 2D, take the same time or 0.3% more.
+// / 32 threads), windows of 20 steps and their reverse: 14,400 tets 4.03 / 3.94
+// ms, 49,152 6.85 / 6.69, 105,600 11.90 / 11.89, 193,536 18.3 / 18.2, 301,056
+// 23.1 / 23.1; 50 FP64 steps of 49,152 tets 6.66 / 6.53, of 105,600 12.14 /
+// 12.17: nothing to choose from a third of a wave on.  The other kernels, and
+// 2D, take the same time or 0.3% more.
 #define DES_LAUNCH_W(KERNEL, n, s, ...)                                                  \
     do {                                                                                 \
         const long long nw_ = (n);                                                       \
@@ -55,9 +56,9 @@ inline int grid_blocks(long long n, int most = 256)
 
 // DES_LAUNCH for kernels of a few instructions a value (copies, layout
 // conversions, the per-function motion, boundary condition and temperature
-// updates): starting a block costs them as much as its work.  Blocks of 64 or 128 / 256, us a call: coordinates of
-// 998,400 tets 6.3 / 4.3 in a mixed context, velocity BCs 5.8 / 4.3; an upload of
-// 1,200 triangles 152 / 139.
+// updates): starting a block costs them as much as its work.  Blocks of 64 or
+// 128 / 256, us a call: coordinates of 998,400 tets 6.3 / 4.3 in a mixed
+// context, velocity BCs 5.8 / 4.3; an upload of 1,200 triangles 152 / 139.
 #define DES_LAUNCH_LIGHT(KERNEL, n, s, ...) \
     KERNEL<<<(unsigned)std::max(1LL, ((long long)(n) + 255) / 256), 256, 0, (s)>>>(__VA_ARGS__)
 
@@ -74,7 +75,7 @@ enum GeoFlags : int {
 };
 
 // Each launcher returns the number of kernels it launched.
-int launch_strain_rate(const KP &p, cudaStream_t s, bool begin_step);
+int launch_strain_rate(const KP &p, cudaStream_t s);
 int launch_update_temperature(const KP &p, cudaStream_t s);       // tdot -> p.tdot, T (FP64 contexts)
 int launch_temperature_update(const KP &p, cudaStream_t s);       // T from p.tdot
 int launch_dvoldt(const KP &p, cudaStream_t s);                   // -> ntmp

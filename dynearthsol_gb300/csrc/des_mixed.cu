@@ -515,8 +515,7 @@ static __device__ __noinline__ void evp_rest(const KP &p, int e, int rest, bool 
 // 998,400 tets: 177 us with the FP64 branches in place, 121 us with the list,
 // 111 us with the shear strain rates as floats (ahead), the density's
 // buoyancy formed where the forces are, and the quarterings, clamps and
-// softening bounds taken as integer operations.  14,400 tets with a yielding
-// band: the list 9.4 ms a pass of 100 steps, in place 8.3 ms.
+// softening bounds taken as integer operations.
 template <bool LIST>
 __global__ void __launch_bounds__(LIST ? 128 : 64, LIST ? 8 : 4) k_update_stress_evp3(KP p, int fused, int outputs,
                                                                                        int ahead)
@@ -674,13 +673,9 @@ __device__ __forceinline__ void strain_rate_mixed_elem(const KP &p, int e, doubl
     for (int c = 0; c < 6; ++c) p.srate[c * ne + e] = out[c];
 }
 
-__global__ void __launch_bounds__(TPB_M) k_strain_rate_mixed3(KP p, int begin_step)
+__global__ void __launch_bounds__(TPB_M) k_strain_rate_mixed3(KP p)
 {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (begin_step && e == 0) {
-        p.clk->steps += 1;
-        p.clk->time += p.clk->dt;
-    }
     if (e >= p.ne) return;
     double sr[6];
     strain_rate_mixed_elem(p, e, sr);
@@ -774,21 +769,20 @@ __global__ void __launch_bounds__(TPB_M) k_elem_pass_mixed3(KP p, int heat)
     elem_terms_mixed(p, e, sr, p.vol[e], s32, heat);
 }
 
-// The node pass: heat and dvoldt sums, the temperature update.  In the
-// chained step (mass_sums) it also forms the previous step's compute_mass
-// sums (volume_n, mass, tmass) from the element records that the look-ahead
-// geometry pass wrote (KP::ndpk), as k_mass_sum forms them, and (begin_step) starts the
-// step's clock, which the look-ahead pass could not: the step's dt is final
-// only after k_dt_finalize.
+// The node pass: heat and dvoldt sums, the temperature update.  MASS (a chained
+// step): it also forms the previous step's compute_mass sums (volume_n, mass,
+// tmass) from the element records that the look-ahead geometry pass wrote
+// (KP::ndpk), as k_mass_sum forms them, and starts the step's clock, which the
+// look-ahead pass could not: its last block forms dt.
 // The heat terms go into a compensated FP32 sum (des_dw.cuh), as
 // k_heat_gather_mixed3 sums them; the dvoldt terms into an FP64 one: they
 // cancel between a node's elements, and the 2^-47 of a double-word split of
 // each moved the volumetric rate enough to change the default damping's
 // copysign at some nodes within ten steps.
 template <bool MASS, bool STAGED>
-__global__ void __launch_bounds__(192) k_node_pass_mixed3(KP p, int heat, int begin_step)
+__global__ void __launch_bounds__(192) k_node_pass_mixed3(KP p, int heat)
 {
-    if (begin_step && blockIdx.x == 0 && threadIdx.x == 0) {   // dynearthsol.cxx:325-326
+    if (MASS && blockIdx.x == 0 && threadIdx.x == 0) {   // dynearthsol.cxx:325-326
         p.clk->steps += 1;
         p.clk->time += p.clk->dt;
     }
@@ -839,6 +833,11 @@ int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused, bool out
     const int n = p.e_hi - p.e_lo, out = outputs || !fused;
     if (p.mat.rheol_type != DES_RH_EVP)
         DES_LAUNCH(k_update_stress_mixed3, n, s, p, (int)fused, (int)ahead);
+    // The line is the one between blocks of 64 and of 128, whose registers the two
+    // forms have.  100 steps, list / in place: 14,400 tets with a yielding band
+    // 9.0 / 8.1 ms, 49,152 10.9 / 10.5, 105,600 14.8 / 15.7, 193,536 21.1 / 25.0,
+    // 301,056 26.7 / 31.7; without yielding 4.7 / 4.6, 5.74 / 5.69, 9.0 / 9.6,
+    // 14.4 / 14.7, 16.8 / 17.7: the list would already pay from ~80,000 on.
     else if (one_wave(n))
         DES_LAUNCH(k_update_stress_evp3<false>, n, s, p, (int)fused, out, (int)ahead);
     else
@@ -846,9 +845,9 @@ int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused, bool out
     return 1;
 }
 
-int launch_strain_rate_mixed(const KP &p, cudaStream_t s, bool begin_step)
+int launch_strain_rate_mixed(const KP &p, cudaStream_t s)
 {
-    DES_LAUNCH(k_strain_rate_mixed3, p.ne, s, p, (int)begin_step);
+    DES_LAUNCH(k_strain_rate_mixed3, p.ne, s, p);
     return 1;
 }
 
@@ -871,11 +870,11 @@ int launch_elem_pass_mixed(const KP &p, cudaStream_t s, bool heat)
     return 1;
 }
 
-int launch_node_pass_mixed(const KP &p, cudaStream_t s, bool heat, bool mass_sums, bool begin_step)
+int launch_node_pass_mixed(const KP &p, cudaStream_t s, bool heat, bool mass_sums)
 {
     const int n = p.n_hi - p.n_lo;
-    if (mass_sums) DES_NODES((k_node_pass_mixed3<true, STAGED>), n, s, p, (int)heat, (int)begin_step);
-    else DES_NODES((k_node_pass_mixed3<false, STAGED>), n, s, p, (int)heat, (int)begin_step);
+    if (mass_sums) DES_NODES((k_node_pass_mixed3<true, STAGED>), n, s, p, (int)heat);
+    else DES_NODES((k_node_pass_mixed3<false, STAGED>), n, s, p, (int)heat);
     return 1;
 }
 

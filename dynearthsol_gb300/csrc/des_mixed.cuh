@@ -11,12 +11,12 @@ namespace des {
 // in the step that follows reads them); ahead: the strain rate is the
 // look-ahead geometry pass's (its shear components in KP::sh32)
 int launch_update_stress_mixed(const KP &p, cudaStream_t s, bool fused, bool outputs = true, bool ahead = false);
-int launch_strain_rate_mixed(const KP &p, cudaStream_t s, bool begin_step);
+int launch_strain_rate_mixed(const KP &p, cudaStream_t s);
 int launch_heat_gather_mixed(const KP &p, cudaStream_t s);   // heat sums -> p.tdot
 // fused step: strain rate + heat terms + dvoldt terms, then the nodal sums and the temperature update
 int launch_elem_pass_mixed(const KP &p, cudaStream_t s, bool heat);
 // mass_sums: first the compute_mass sums of the look-ahead geometry pass's
-// element terms (k_mass_sum's); begin_step: advance the clock (steps, time)
-int launch_node_pass_mixed(const KP &p, cudaStream_t s, bool heat, bool mass_sums = false, bool begin_step = false);
+// element terms (k_mass_sum's), and the clock advance
+int launch_node_pass_mixed(const KP &p, cudaStream_t s, bool heat, bool mass_sums = false);
 
 }  // namespace des
